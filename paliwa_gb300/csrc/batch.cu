@@ -841,9 +841,18 @@ struct paliwa_gb_ct {
   CtSubspace *subspaces_dev = nullptr;
   int *lists_dev = nullptr;
   CtGrid *grids_dev = nullptr;
-  int *heavy_dev = nullptr;
-  long long *heavy_first_dev = nullptr;
   int *block_sub_dev = nullptr;
+  CtBlock *blocks_dev = nullptr;
+  int *order_dev = nullptr;
+  int *unit_grid_dev = nullptr;
+  long long *unit_first_dev = nullptr;
+  long long *families_dev = nullptr;
+  long long *family_first_dev = nullptr;
+  // FP32 grids: the sparse values as floats during a restrict.
+  float *values_dev = nullptr;
+  long long ncombine = 0;   // combine CTAs
+  long long nrestrict = 0;  // restrict CTAs
+  bool big = false;         // a grid of 2^31 points or more
   CtParams params{};
 };
 
@@ -854,6 +863,151 @@ uint64_t level_key(int const *s, int ndim) {
   uint64_t k = 0;
   for (int d = 0; d < ndim; ++d) k = (k << 5) | static_cast<uint64_t>(s[d]);
   return k;
+}
+
+template <typename T>
+void upload(T **dst, std::vector<T> const &v, char const *what) {
+  if (v.empty()) return;
+  size_t const bytes = v.size() * sizeof(T);
+  cuda_check(cudaMalloc(reinterpret_cast<void **>(dst), bytes), what);
+  cuda_check(cudaMemcpy(*dst, v.data(), bytes, cudaMemcpyHostToDevice), what);
+}
+
+// log2 of a subspace's points.
+int subspace_log2(CtSubspace const &ss, int ndim) {
+  int n = 0;
+  for (int d = 0; d < ndim; ++d) n += std::max(0, ss.level[d] - 1);
+  return n;
+}
+
+// The combine's CTAs: subspaces of fewer than kCtBlock points grouped by
+// size, longest grid lists first (the lists of one CTA are then about
+// equally long, and the longest chains of updates start first), then the
+// larger subspaces cut into kCtBlock points in storage order (neighbouring
+// CTAs share sectors of the grids).
+void plan_combine(paliwa_gb_ct &ct, std::vector<CtSubspace> const &subs) {
+  int const nsubs = static_cast<int>(subs.size());
+  constexpr int log2block = Log2<kCtBlock>::value;
+  std::vector<int> order(nsubs), log2p(nsubs);
+  auto const length = [&](int i) {
+    return subs[i].grid_end - subs[i].grid_begin;
+  };
+  for (int i = 0; i < nsubs; ++i) {
+    order[i] = i;
+    log2p[i] = std::min(subspace_log2(subs[i], ct.ndim), log2block);
+  }
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    if (log2p[a] != log2p[b]) return log2p[a] < log2p[b];
+    return log2p[a] < log2block && length(a) > length(b);
+  });
+  std::vector<CtBlock> blocks;
+  for (int i = 0; i < nsubs;) {
+    int const lp = log2p[order[i]];
+    CtBlock blk{};
+    blk.order_first = i;
+    blk.log2p = lp;
+    blk.longest = length(order[i]);
+    if (lp < log2block) {
+      int const most = std::min(ct_max_subs(lp), kCtBlock >> lp);
+      while (blk.nsub < most && i + blk.nsub < nsubs &&
+             log2p[order[i + blk.nsub]] == lp)
+        ++blk.nsub;
+      blocks.push_back(blk);
+      i += blk.nsub;
+      continue;
+    }
+    blk.nsub = 1;
+    long long const size = 1LL << subspace_log2(subs[order[i]], ct.ndim);
+    for (blk.local = 0; blk.local < size; blk.local += kCtBlock)
+      blocks.push_back(blk);
+    ++i;
+  }
+  // The lists of the small subspaces' CTAs, longest first over all sizes.
+  std::stable_sort(blocks.begin(), blocks.end(),
+                   [&](CtBlock const &a, CtBlock const &b) {
+                     int const la = a.log2p < log2block ? a.longest : -1;
+                     int const lb = b.log2p < log2block ? b.longest : -1;
+                     return la > lb;
+                   });
+  ct.ncombine = static_cast<long long>(blocks.size());
+  upload(&ct.blocks_dev, blocks, "upload combine blocks");
+  upload(&ct.order_dev, order, "upload subspace order");
+  ct.params.blocks = ct.blocks_dev;
+  ct.params.order = ct.order_dev;
+}
+
+// The restrict's units of kCtUnit points (the grid of each) and every grid's
+// table of families: for the leading levels (s_1 .. s_{d-1}), 0 <= s <= l,
+// last dimension fastest, the first sparse point of (s_1 .. s_{d-1}, 0) and
+// the highest kept last level of the grid (a subspace's lower neighbours are
+// in every grid that holds it, so the kept levels are 0 .. top).
+void plan_restrict(paliwa_gb_ct &ct, std::vector<CtSubspace> const &subs,
+                   int64_t const *levels) {
+  int const nd = ct.ndim;
+  // Leading levels -> {first sparse point, highest kept last level}: the
+  // subspaces of a family are consecutive and start at last level 0.
+  std::unordered_map<uint64_t, std::pair<long long, int>> family;
+  std::vector<int> s(nd);
+  for (auto const &ss : subs) {
+    for (int d = 0; d < nd; ++d) s[d] = ss.level[d];
+    auto const it =
+        family.emplace(level_key(s.data(), nd - 1),
+                       std::make_pair(ss.offset, -1)).first;
+    it->second.second = std::max(it->second.second, s[nd - 1]);
+  }
+  std::vector<int> unit_grid;
+  std::vector<long long> unit_first(ct.ngrids), first(ct.ngrids), table;
+  for (int g = 0; g < ct.ngrids; ++g) {
+    int64_t const *lv = levels + static_cast<size_t>(g) * nd;
+    int64_t total = 0;
+    for (int d = 0; d < nd; ++d) total += lv[d];
+    unit_first[g] = static_cast<long long>(unit_grid.size());
+    unit_grid.insert(unit_grid.end(),
+                     ((1LL << total) + kCtUnit - 1) / kCtUnit, g);
+    first[g] = static_cast<long long>(table.size());
+    std::fill(s.begin(), s.end(), 0);
+    while (true) {
+      auto const it = family.find(level_key(s.data(), nd - 1));
+      long long e = 0;
+      if (it != family.end()) {
+        int const top =
+            std::min<int>(it->second.second, static_cast<int>(lv[nd - 1]));
+        e = it->second.first |
+            (static_cast<long long>(top + 1) << kCtFamilyShift);
+      }
+      table.push_back(e);
+      int d = nd - 2;
+      while (d >= 0 && s[d] == lv[d]) s[d--] = 0;
+      if (d < 0) break;
+      ++s[d];
+    }
+  }
+  ct.nrestrict = static_cast<long long>(unit_grid.size());
+  upload(&ct.unit_grid_dev, unit_grid, "upload restrict units");
+  upload(&ct.unit_first_dev, unit_first, "upload restrict unit offsets");
+  upload(&ct.families_dev, table, "upload families");
+  upload(&ct.family_first_dev, first, "upload family offsets");
+  ct.params.unit_grid = ct.unit_grid_dev;
+  ct.params.unit_first = ct.unit_first_dev;
+  ct.params.families = ct.families_dev;
+  ct.params.family_first = ct.family_first_dev;
+  if (ct.dtype != PALIWA_GB_F64 && ct.npoints > 0)
+    cuda_check(cudaMalloc(&ct.values_dev, ct.npoints * sizeof(float)),
+               "cudaMalloc(restrict values)");
+}
+
+void free_ct(paliwa_gb_ct &ct) {
+  cudaFree(ct.subspaces_dev);
+  cudaFree(ct.lists_dev);
+  cudaFree(ct.grids_dev);
+  cudaFree(ct.block_sub_dev);
+  cudaFree(ct.blocks_dev);
+  cudaFree(ct.order_dev);
+  cudaFree(ct.unit_grid_dev);
+  cudaFree(ct.unit_first_dev);
+  cudaFree(ct.families_dev);
+  cudaFree(ct.family_first_dev);
+  cudaFree(ct.values_dev);
 }
 
 void build_ct(paliwa_gb_ct &ct, int64_t const *levels,
@@ -923,33 +1077,17 @@ void build_ct(paliwa_gb_ct &ct, int64_t const *levels,
     std::memset(&grids[g], 0, sizeof(CtGrid));
     grids[g].base = reinterpret_cast<unsigned long long>(grid_ptrs[g]);
     grids[g].coefficient = coefficients[g];
-    for (int d = 0; d < nd; ++d)
-      grids[g].level[d] =
-          static_cast<signed char>(levels[static_cast<size_t>(g) * nd + d]);
-  }
-  auto upload = [](auto **dst, auto const &v, char const *what) {
-    if (v.empty()) return;
-    size_t const bytes = v.size() * sizeof(v[0]);
-    cuda_check(cudaMalloc(reinterpret_cast<void **>(dst), bytes), what);
-    cuda_check(cudaMemcpy(*dst, v.data(), bytes, cudaMemcpyHostToDevice),
-               what);
-  };
-  std::vector<int> heavy;
-  std::vector<long long> heavy_first;
-  long long nheavy_points = 0;
-  for (size_t i = 0; i < subs.size(); ++i) {
-    if (subs[i].grid_end - subs[i].grid_begin <= kCtHeavy) continue;
-    heavy.push_back(static_cast<int>(i));
-    heavy_first.push_back(nheavy_points);
-    long long const next =
-        i + 1 < subs.size() ? subs[i + 1].offset : off;
-    nheavy_points += next - subs[i].offset;
+    int step = 0;
+    for (int d = nd - 1; d >= 0; --d) {
+      int const l = static_cast<int>(levels[static_cast<size_t>(g) * nd + d]);
+      grids[g].level[d] = static_cast<signed char>(l);
+      step += l;
+      grids[g].step[d / 4] |= static_cast<unsigned>(step) << (8 * (d % 4));
+    }
   }
   upload(&ct.subspaces_dev, subs, "upload subspaces");
   upload(&ct.lists_dev, lists, "upload grid lists");
   upload(&ct.grids_dev, grids, "upload grids");
-  upload(&ct.heavy_dev, heavy, "upload heavy subspaces");
-  upload(&ct.heavy_first_dev, heavy_first, "upload heavy offsets");
   // First subspace of every CTA's 256 points (the subspace holding point
   // 256 b), so that no CTA searches the whole subspace list.
   std::vector<int> block_sub((off + kCtBlock - 1) / kCtBlock);
@@ -971,11 +1109,9 @@ void build_ct(paliwa_gb_ct &ct, int64_t const *levels,
   ct.params.npoints = ct.npoints;
   for (int d = 0; d < nd && d < kMaxDims; ++d)
     ct.params.max_level[d] = static_cast<signed char>(lmax[d]);
-  ct.params.heavy = ct.heavy_dev;
-  ct.params.heavy_first = ct.heavy_first_dev;
   ct.params.block_sub = ct.block_sub_dev;
-  ct.params.nheavy = static_cast<int>(heavy.size());
-  ct.params.nheavy_points = nheavy_points;
+  plan_combine(ct, subs);
+  plan_restrict(ct, subs, levels);
   // Products c * v are exact in FP64 when c has at most 53 - 24 = 29
   // significant bits and v is a float (whose magnitude lies in
   // [2^-149, 2^128]), provided |c| stays within [2^-500, 2^500] so that the
@@ -1006,35 +1142,91 @@ void build_ct(paliwa_gb_ct &ct, int64_t const *levels,
   ct.params.exact_products = exact ? 1 : 0;
 }
 
-template <int OP>
-void ct_launch(paliwa_gb_ct const &ct, double *sparse, double *full,
-               cudaStream_t s) {
+// Dimensions padded to 4, 8 or 12 (a padded dimension has one point).
+template <typename S, bool Fused>
+void launch_combine(paliwa_gb_ct const &ct, CtParams const &p,
+                    cudaStream_t s) {
+  unsigned const blocks = static_cast<unsigned>(ct.ncombine);
+  if (ct.big)
+    ct_combine_kernel<S, kMaxDims, Fused, true><<<blocks, kCtBlock, 0, s>>>(p);
+  else if (ct.ndim <= 4)
+    ct_combine_kernel<S, 4, Fused, false><<<blocks, kCtBlock, 0, s>>>(p);
+  else if (ct.ndim <= 8)
+    ct_combine_kernel<S, 8, Fused, false><<<blocks, kCtBlock, 0, s>>>(p);
+  else
+    ct_combine_kernel<S, kMaxDims, Fused, false><<<blocks, kCtBlock, 0, s>>>(
+        p);
+  cuda_check(cudaGetLastError(), "ct_combine_kernel launch");
+}
+
+void ct_combine(paliwa_gb_ct const &ct, double *sparse, cudaStream_t s) {
   if (ct.npoints == 0) return;
   CtParams p = ct.params;
   p.sparse = sparse;
+  if (ct.dtype == PALIWA_GB_F64)
+    return p.exact_products ? launch_combine<double, true>(ct, p, s)
+                            : launch_combine<double, false>(ct, p, s);
+  p.exact_products ? launch_combine<float, true>(ct, p, s)
+                   : launch_combine<float, false>(ct, p, s);
+}
+
+// Two to six dimensions have kernels of their own while 32-bit indices hold
+// every grid and the sparse grid (with a unit to spare past a grid's end);
+// anything else takes the general one.
+template <typename S>
+void launch_restrict(paliwa_gb_ct const &ct, CtParams const &p,
+                     cudaStream_t s) {
+  unsigned const blocks = static_cast<unsigned>(ct.nrestrict);
+  bool const small = !ct.big && ct.npoints < (1LL << 31);
+  switch (small ? ct.ndim : 0) {
+  case 2:
+    ct_restrict_kernel<S, 2, unsigned><<<blocks, kCtBlock, 0, s>>>(p);
+    break;
+  case 3:
+    ct_restrict_kernel<S, 3, unsigned><<<blocks, kCtBlock, 0, s>>>(p);
+    break;
+  case 4:
+    ct_restrict_kernel<S, 4, unsigned><<<blocks, kCtBlock, 0, s>>>(p);
+    break;
+  case 5:
+    ct_restrict_kernel<S, 5, unsigned><<<blocks, kCtBlock, 0, s>>>(p);
+    break;
+  case 6:
+    ct_restrict_kernel<S, 6, unsigned><<<blocks, kCtBlock, 0, s>>>(p);
+    break;
+  default:
+    ct_restrict_kernel<S, kMaxDims, unsigned long long>
+        <<<blocks, kCtBlock, 0, s>>>(p);
+  }
+  cuda_check(cudaGetLastError(), "ct_restrict_kernel launch");
+}
+
+void ct_restrict(paliwa_gb_ct const &ct, double const *sparse,
+                 cudaStream_t s) {
+  if (ct.npoints == 0) return;
+  CtParams p = ct.params;
+  if (ct.dtype == PALIWA_GB_F64) {
+    p.values = sparse;
+    launch_restrict<double>(ct, p, s);
+  } else {
+    long long const nb = (ct.npoints + kCtBlock - 1) / kCtBlock;
+    ct_narrow_kernel<<<static_cast<unsigned>(std::min(nb, 16LL * 152)),
+                       kCtBlock, 0, s>>>(sparse, ct.values_dev, ct.npoints);
+    p.values = ct.values_dev;
+    launch_restrict<float>(ct, p, s);
+  }
+}
+
+void ct_scatter(paliwa_gb_ct const &ct, double const *sparse, double *full,
+                cudaStream_t s) {
+  if (ct.npoints == 0) return;
+  CtParams p = ct.params;
+  p.sparse = const_cast<double *>(sparse);
   p.full = full;
-  unsigned const blocks =
-      static_cast<unsigned>((ct.npoints + kCtBlock - 1) / kCtBlock);
-  switch (ct.dtype) {
-  case PALIWA_GB_F64:
-    ct_kernel<double, OP><<<blocks, kCtBlock, 0, s>>>(p);
-    break;
-  case PALIWA_GB_F32:
-  case PALIWA_GB_F32C:
-    ct_kernel<float, OP><<<blocks, kCtBlock, 0, s>>>(p);
-    break;
-  default: throw StatusError(PALIWA_GB_INVALID_ARGUMENT, "unknown dtype");
-  }
-  cuda_check(cudaGetLastError(), "ct_kernel launch");
-  if (OP == kRestrict && p.nheavy_points > 0) {
-    unsigned const hblocks =
-        static_cast<unsigned>((p.nheavy_points * 32 + 255) / 256);
-    if (ct.dtype == PALIWA_GB_F64)
-      ct_heavy_restrict_kernel<double><<<hblocks, 256, 0, s>>>(p);
-    else
-      ct_heavy_restrict_kernel<float><<<hblocks, 256, 0, s>>>(p);
-    cuda_check(cudaGetLastError(), "ct_heavy_restrict_kernel launch");
-  }
+  ct_scatter_kernel<<<static_cast<unsigned>((ct.npoints + kCtBlock - 1) /
+                                            kCtBlock),
+                      kCtBlock, 0, s>>>(p);
+  cuda_check(cudaGetLastError(), "ct_scatter_kernel launch");
 }
 
 } // namespace
@@ -1407,15 +1599,15 @@ int paliwa_gb_ct_create(int ndim, int ngrids, const int64_t *levels,
     ct->ndim = ndim;
     ct->ngrids = ngrids;
     ct->dtype = dtype;
+    for (int g = 0; g < ngrids; ++g) {
+      int64_t total = 0;
+      for (int d = 0; d < ndim; ++d) total += levels[g * ndim + d];
+      ct->big |= total >= 31;
+    }
     try {
       build_ct(*ct, levels, coefficients, maximum_level, grid_ptrs, keep_all);
     } catch (...) {
-      cudaFree(ct->subspaces_dev);
-      cudaFree(ct->lists_dev);
-      cudaFree(ct->grids_dev);
-      cudaFree(ct->heavy_dev);
-      cudaFree(ct->heavy_first_dev);
-      cudaFree(ct->block_sub_dev);
+      free_ct(*ct);
       throw;
     }
     *out = ct.release();
@@ -1449,8 +1641,7 @@ int paliwa_gb_ct_combine(paliwa_gb_ct *ct, double *sparse, void *stream) {
   return guarded([&] {
     if (ct == nullptr || sparse == nullptr)
       throw StatusError(PALIWA_GB_INVALID_ARGUMENT, "null argument");
-    ct_launch<kCombine>(*ct, sparse, nullptr,
-                        static_cast<cudaStream_t>(stream));
+    ct_combine(*ct, sparse, static_cast<cudaStream_t>(stream));
   });
 }
 
@@ -1459,8 +1650,7 @@ int paliwa_gb_ct_restrict(paliwa_gb_ct *ct, const double *sparse,
   return guarded([&] {
     if (ct == nullptr || sparse == nullptr)
       throw StatusError(PALIWA_GB_INVALID_ARGUMENT, "null argument");
-    ct_launch<kRestrict>(*ct, const_cast<double *>(sparse), nullptr,
-                         static_cast<cudaStream_t>(stream));
+    ct_restrict(*ct, sparse, static_cast<cudaStream_t>(stream));
   });
 }
 
@@ -1478,19 +1668,13 @@ int paliwa_gb_ct_scatter(paliwa_gb_ct *ct, const double *sparse, double *full,
     cuda_check(cudaMemsetAsync(full, 0, sizeof(double) << total,
                                static_cast<cudaStream_t>(stream)),
                "cudaMemsetAsync");
-    ct_launch<kScatter>(*ct, const_cast<double *>(sparse), full,
-                        static_cast<cudaStream_t>(stream));
+    ct_scatter(*ct, sparse, full, static_cast<cudaStream_t>(stream));
   });
 }
 
 void paliwa_gb_ct_destroy(paliwa_gb_ct *ct) {
   if (ct == nullptr) return;
-  cudaFree(ct->subspaces_dev);
-  cudaFree(ct->lists_dev);
-  cudaFree(ct->grids_dev);
-  cudaFree(ct->heavy_dev);
-  cudaFree(ct->heavy_first_dev);
-  cudaFree(ct->block_sub_dev);
+  free_ct(*ct);
   delete ct;
 }
 

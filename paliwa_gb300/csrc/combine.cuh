@@ -13,6 +13,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 namespace pgb {
@@ -26,10 +27,24 @@ struct CtSubspace {
   signed char level[kMaxDims];
 };
 
-struct CtGrid {
+struct __align__(16) CtGrid {
   unsigned long long base;  // byte address of the grid
   double coefficient;
   signed char level[kMaxDims];
+  // log2 of level 0's element step along each dimension (the dimension's
+  // extent times its stride), one byte each: level s steps step - s.
+  unsigned step[kMaxDims / 4];
+};
+
+// Work of one combine CTA: nsub subspaces of 2^log2p points each (their ids
+// at CtParams::order + order_first; all points of each), or, for a subspace
+// of more than kCtBlock points, kCtBlock of its points from `local` on.
+struct CtBlock {
+  long long local;
+  int order_first;
+  int nsub;
+  int log2p;    // points of each subspace held by the CTA
+  int longest;  // longest grid list among its subspaces
 };
 
 struct CtParams {
@@ -46,44 +61,69 @@ struct CtParams {
   // of at most 29 significant bits and moderate magnitude on FP32 grids,
   // +-1 on FP64 grids): the combine then fuses multiply and add.
   int exact_products;
-  // Subspaces contained in more than kCtHeavy grids are restricted one warp
-  // per point (ct_heavy_restrict_kernel): heavy[i] is the subspace index,
-  // heavy_first[i] the first of its points in the heavy numbering (prefix
-  // sums of the sizes).
-  int const *heavy;
-  long long const *heavy_first;
-  int nheavy;
-  long long nheavy_points;
   // block_sub[b]: the subspace holding point kCtBlock * b (the first point
-  // of CTA b), planned on the host.
+  // of scatter's CTA b), planned on the host.
   int const *block_sub;
+  // Combine: its CTAs and the subspace ids they refer to.
+  CtBlock const *blocks;
+  int const *order;
+  // Restrict: the grid of every unit of kCtUnit points, each grid's first
+  // unit, and its families (see ct_restrict_kernel): families[
+  // family_first[g] + index of (s_1 .. s_{d-1})].
+  int const *unit_grid;
+  long long const *unit_first;
+  long long const *families;
+  long long const *family_first;
+  void const *values;  // the sparse values in the grids' type
 };
 
-// Points (threads) per CTA of ct_kernel.
+// Points (threads) per CTA of the combine and scatter kernels.
 constexpr int kCtBlock = 256;
+// Grid descriptors staged per batch of a combine CTA.
+constexpr int kCtStage = 256;
+// Grid values a combine thread loads before it adds them, and the kernel's
+// CTAs per SM (48 registers). Measured, 4D |l|_1 = 19 - q and 6D 16 - q, us:
+// 8 values and 5 CTAs 1567 and 997, 4 and 5 1575 and 1090, 8 and 4 1776 and
+// 1008, 4 and 6 1774 and 1147, 8 and 3 1975 and 1127.
+constexpr int kCtAhead = 8;
+constexpr int kCtCtas = 5;
+// Subspaces of up to 2^kCtLog2Few points have the longest grid lists (those of
+// one point every grid): their values are loaded by every thread of the CTA,
+// since one thread with kCtAhead loads in flight took 2.0 ms for 7,798 grids.
+constexpr int kCtLog2Few = 3;
+// Subspaces of one combine CTA, at most, by their points: the fewer, the more
+// grids a batch holds.
+inline int ct_max_subs(int log2p) {
+  return log2p <= 1 ? 2 : log2p <= kCtLog2Few ? 4 : 8;
+}
+// Grid points per restrict CTA: kCtGroups groups of 4 per thread.
+constexpr int kCtGroups = 4;
+constexpr int kCtUnit = 4 * kCtGroups * kCtBlock;
 
-// Grid count above which restrict writes a subspace's points one warp per
-// point (lanes over grids) instead of one thread per point: a thread would
-// walk thousands of grids (the coarsest subspaces are in every grid) while
-// the rest of the launch has finished. Measured on GB300 (FP32 grids):
-// 6D scheme |l|_1 = 16 - q, restrict 5.3 -> 2.8 ms; 4D |l|_1 = 20 - q
-// unchanged (8.1 -> 8.3 ms). Combine keeps one thread per point for every
-// subspace: the warp form made the 4D combine slower (9.0 -> 11.3 ms).
-constexpr int kCtHeavy = 1024;
+// A family is the subspaces (s_1 .. s_{d-1}, 0 .. top) of one leading level
+// vector; they lie one after another in the sparse grid. Packed as the first
+// sparse point in the low 56 bits and top + 1 above (0: none kept).
+constexpr int kCtFamilyShift = 56;
 
 // float -> double without the conversion instruction, which on GB300 runs
-// on the FP64 pipe: for normal numbers the double is the float's sign,
-// exponent rebiased by 1023 - 127 and fraction shifted by 29 bits (the
-// exact value); zeros, subnormals, infinities and NaNs take the conversion.
+// on the FP64 pipe: the double is the float's sign, exponent rebiased by
+// 1023 - 127 and fraction shifted by 29 bits (the exact value). Subnormals are
+// scaled by 2^24 first, zeros, infinities and NaNs keep their own exponent
+// field. No branch holds a conversion: the compiler runs a short one for
+// every value under a predicate, and one conversion per value doubled the
+// combine's FP64 work.
 __device__ __forceinline__ double widen(float x) {
-  unsigned const u = __float_as_uint(x);
-  unsigned const e = (u >> 23) & 0xffu;
-  if (e == 0u || e == 0xffu) return static_cast<double>(x);
-  unsigned long long const bits =
-      (static_cast<unsigned long long>(u >> 31) << 63) |
-      (static_cast<unsigned long long>(e + (1023 - 127)) << 52) |
-      (static_cast<unsigned long long>(u & 0x7fffffu) << 29);
-  return __longlong_as_double(static_cast<long long>(bits));
+  unsigned u = __float_as_uint(x);
+  unsigned const a = u & 0x7fffffffu;
+  unsigned bias = (1023u - 127u) << 20;
+  if (a < 0x00800000u) {
+    u = __float_as_uint(__fmul_rn(x, 16777216.0f));
+    bias -= a == 0u ? bias : 24u << 20;
+  }
+  unsigned hi = ((u & 0x7fffffffu) >> 3) + bias;
+  if (a >= 0x7f800000u) hi |= 0x7ff00000u;
+  return __hiloint2double(static_cast<int>(hi | (u & 0x80000000u)),
+                          static_cast<int>(u << 29));
 }
 __device__ __forceinline__ double widen(double x) { return x; }
 
@@ -108,44 +148,336 @@ __device__ __forceinline__ long long ct_offset(long long p,
   return off;
 }
 
-// Combined value of one sparse point: sum over the containing grids, in
-// grid order, of coefficient * value. One grid per iteration: loading
-// several grids ahead (8 per batch: 64 registers) measured slower on the 4D
-// scheme (10.6 against 9.0 ms), as the loop is limited by the scattered
-// loads, not by their latency.
-template <typename S, bool Fused>
-__device__ __forceinline__ double ct_combine_point(CtParams const &p,
-                                                   CtSubspace const &ss,
-                                                   long long local) {
-  double acc = 0.0;
-  for (int gi = ss.grid_begin; gi < ss.grid_end; ++gi) {
-    CtGrid const &g = p.grids[p.grid_lists[gi]];
-    long long const off = ct_offset(local, ss.level, g.level, p.ndim);
-    double const v = widen(reinterpret_cast<S const *>(g.base)[off]);
-    if constexpr (Fused)
-      acc = __fma_rn(g.coefficient, v, acc);
-    else
-      acc = __dadd_rn(acc, __dmul_rn(g.coefficient, v));
+// Combine: sparse[p] = sum over the containing grids, in grid order, of
+// coefficient * value in FP64 (with exact products fma(c, v, acc) rounds
+// like the reference driver's separate multiply and add, and issues one FP64
+// instruction instead of two).
+//
+// The floor is one FP64 update per contained grid value: about two lane
+// operations per clock and SM, 0.45 ms for the 273 M values of 4D |l|_1 =
+// 18 - q, behind one scattered load each. A CTA takes points of subspaces of
+// one size (a few subspaces, so that small ones fill its warps) and walks
+// their grid lists in batches: every thread stages one descriptor (address,
+// coefficient and the element step of each dimension) in shared memory, then
+// each point's thread forms its addresses with one multiply-add per dimension
+// and keeps kCtAhead loads in flight. Measured (FP32 grids), against a thread
+// that walked list entry -> grid -> value by itself and converted each value
+// on the FP64 pipe: 4D |l|_1 = 19 - q 3.60 -> 1.57 ms, 20 - q 8.5 -> 3.7, 6D
+// 16 - q 7.5 -> 1.0.
+template <typename S, int ND, bool Fused, bool Big>
+__global__ void __launch_bounds__(kCtBlock, kCtCtas)
+    ct_combine_kernel(CtParams const p) {
+  using Mult = typename std::conditional<Big, unsigned long long,
+                                         unsigned>::type;
+  // One descriptor: 16-byte reads, one wavefront each (the lanes of a warp
+  // read the same one, or a few).
+  struct __align__(16) Desc {
+    unsigned long long base;
+    double coef;
+    Mult mult[ND];
+  };
+  __shared__ Desc s_desc[kCtStage];
+  __shared__ S s_value[1 << kCtLog2Few][kCtStage];
+  int const t = threadIdx.x;
+  CtBlock const blk = p.blocks[blockIdx.x];
+  int const pi = t & ((1 << blk.log2p) - 1);
+  int const si = t >> blk.log2p;
+  bool const active = si < blk.nsub;
+  // Batch: kCtStage / (subspaces rounded up to a power of two) grids each.
+  int const log2subs = blk.nsub <= 1 ? 0 : 32 - __clz(blk.nsub - 1);
+  int const log2k = 31 - __clz(kCtStage) - log2subs;
+  int const K = 1 << log2k;
+  // This thread's point, as odd multiples m_d of each dimension's step.
+  int len = 0;
+  long long point = 0;
+  unsigned m[ND];
+#pragma unroll
+  for (int d = 0; d < ND; ++d) m[d] = 0;
+  if (active) {
+    CtSubspace const &ss = p.subspaces[p.order[blk.order_first + si]];
+    len = ss.grid_end - ss.grid_begin;
+    long long r = blk.local + pi;
+    point = ss.offset + r;
+#pragma unroll
+    for (int d = ND - 1; d >= 0; --d) {
+      int const sd = d < p.ndim ? ss.level[d] : 0;
+      if (sd == 0) continue;
+      m[d] = 2 * static_cast<unsigned>(r & ((1LL << (sd - 1)) - 1)) + 1;
+      r >>= sd - 1;
+    }
   }
-  return acc;
+  // The subspace whose grids this thread stages.
+  int const st = t >> log2k;
+  int st_begin = 0, st_end = 0;
+  unsigned st_level[ND / 4];  // its levels, 4 dimensions per word
+#pragma unroll
+  for (int w = 0; w < ND / 4; ++w) st_level[w] = 0;
+  if (st < blk.nsub) {
+    CtSubspace const &ss = p.subspaces[p.order[blk.order_first + st]];
+    st_begin = ss.grid_begin + (t & (K - 1));
+    st_end = ss.grid_end;
+#pragma unroll
+    for (int w = 0; w < ND / 4; ++w)
+      st_level[w] = reinterpret_cast<unsigned const *>(ss.level)[w];
+  }
+  double acc = 0.0;
+  bool const staged = blk.log2p <= kCtLog2Few;
+  for (int k0 = 0; k0 < blk.longest; k0 += K) {
+    if (k0 > 0) __syncthreads();  // the last batch is done with
+    if (st_begin + k0 < st_end) {
+      CtGrid const &g = p.grids[p.grid_lists[st_begin + k0]];
+      Desc desc;
+      desc.base = g.base;
+      desc.coef = g.coefficient;
+      unsigned step[ND / 4];  // 4 dimensions' step bytes per word
+#pragma unroll
+      for (int w = 0; w < ND / 4; ++w) step[w] = g.step[w];
+#pragma unroll
+      for (int d = 0; d < ND; ++d)
+        desc.mult[d] = static_cast<Mult>(1)
+                       << (((step[d / 4] - st_level[d / 4]) >> (8 * (d % 4))) &
+                           63u);
+      s_desc[t] = desc;
+      if (staged) {
+        S const *const from = reinterpret_cast<S const *>(desc.base);
+        S x[1 << kCtLog2Few];
+#pragma unroll
+        for (int i = 0; i < (1 << kCtLog2Few); ++i) {
+          if (i >> blk.log2p) break;
+          unsigned long long off = 0;
+          unsigned r = static_cast<unsigned>(i);
+#pragma unroll
+          for (int d = ND - 1; d >= 0; --d) {
+            unsigned const sd = (st_level[d / 4] >> (8 * (d % 4))) & 63u;
+            if (sd == 0) continue;
+            off += static_cast<unsigned long long>(
+                       2 * (r & ((1u << (sd - 1)) - 1)) + 1) * desc.mult[d];
+            r >>= sd - 1;
+          }
+          x[i] = from[off];
+        }
+#pragma unroll
+        for (int i = 0; i < (1 << kCtLog2Few); ++i)
+          if (!(i >> blk.log2p)) s_value[i][t] = x[i];
+      }
+    }
+    __syncthreads();
+    int const n = min(K, len - k0);
+    int const e0 = si << log2k;
+    auto add = [&](double coef, S x) {
+      double const v = widen(x);
+      if constexpr (Fused)
+        acc = __fma_rn(coef, v, acc);
+      else
+        acc = __dadd_rn(acc, __dmul_rn(coef, v));
+    };
+    if (staged) {
+      for (int k = 0; k < n; ++k)
+        add(s_desc[e0 + k].coef, s_value[pi][e0 + k]);
+      continue;
+    }
+    auto value = [&](int e, double &coef) {
+      Desc const desc = s_desc[e];
+      unsigned long long off = 0;
+#pragma unroll
+      for (int d = 0; d < ND; ++d)
+        off += static_cast<unsigned long long>(m[d]) * desc.mult[d];
+      coef = desc.coef;
+      return reinterpret_cast<S const *>(desc.base)[off];
+    };
+    int k = 0;
+    for (; k + kCtAhead <= n; k += kCtAhead) {
+      S x[kCtAhead];
+      double c[kCtAhead];
+#pragma unroll
+      for (int i = 0; i < kCtAhead; ++i) x[i] = value(e0 + k + i, c[i]);
+#pragma unroll
+      for (int i = 0; i < kCtAhead; ++i) add(c[i], x[i]);
+    }
+    for (; k < n; ++k) {
+      double c;
+      S const x = value(e0 + k, c);
+      add(c, x);
+    }
+  }
+  if (active) p.sparse[point] = acc;
 }
 
-// Which of the three operations a launch performs.
-enum CtOp { kCombine = 0, kRestrict = 1, kScatter = 2 };
+// The sparse values in the grids' type, converted once per point: a
+// conversion per grid value would take the FP64 pipe as long as the combine.
+__global__ void __launch_bounds__(kCtBlock)
+    ct_narrow_kernel(double const *in, float *out, long long n) {
+  long long const step = static_cast<long long>(gridDim.x) * kCtBlock;
+  for (long long i = static_cast<long long>(blockIdx.x) * kCtBlock +
+                     threadIdx.x;
+       i < n; i += step)
+    out[i] = static_cast<float>(in[i]);
+}
 
-template <typename S, int OP>
-__global__ void __launch_bounds__(kCtBlock) ct_kernel(CtParams const p) {
+// Restrict: every grid point whose subspace is kept takes its combined value.
+//
+// Bound by memory: each grid is written once, in storage order, and the
+// sparse values are gathered. (Written from the sparse side, one thread per
+// sparse point over its grids, every store touched a 32-byte sector for 4
+// bytes: 4D |l|_1 = 19 - q 3.17 -> 1.11 ms, 20 - q 7.7 -> 2.6, 6D 16 - q
+// 2.65 -> 0.66.) Thread = 4 consecutive points 4 a .. 4 a + 3 of a last-axis row:
+// levels l, l - 1, l and, for 4 a, whatever its trailing zeros say, so a warp
+// gathers a few contiguous runs. The leading indices name the row's family,
+// whose first point and kept levels come from a table per grid. ND: the
+// dimensions (kMaxDims: any number); I: the type of point indices (32 bits
+// where the grid and the sparse grid allow it: the index arithmetic issues on
+// 80 % of the cycles otherwise).
+template <int ND, typename I> struct CtRows {
+  int lv[ND];     // levels of the leading dimensions and the last
+  int radix[ND];  // of the family index
+  long long const *families;
+  int nd;
+
+  __device__ __forceinline__ CtRows(CtParams const &p, int g) {
+    nd = ND < kMaxDims ? ND : p.ndim;
+    families = p.families + p.family_first[g];
+    int r = 1;
+#pragma unroll
+    for (int d = ND - 1; d >= 0; --d) {
+      lv[d] = d < nd ? p.grids[g].level[d] : 0;
+      radix[d] = r;
+      if (d < nd - 1) r *= lv[d] + 1;
+    }
+  }
+  __device__ __forceinline__ int last() const {
+    int l = lv[0];
+#pragma unroll
+    for (int d = 1; d < ND; ++d)
+      if (d == nd - 1) l = lv[d];
+    return l;
+  }
+};
+
+// A row of the grid along its last axis.
+template <typename I> struct CtRow {
+  I base;   // first sparse point of its family
+  I fam;    // points of the family at its coarsest level
+  I pos;    // the row among them
+  int top;  // highest kept level of the last axis (-1: none)
+
+  template <int ND>
+  __device__ __forceinline__ CtRow(CtRows<ND, I> const &rows, I row) {
+    int fi = 0, log2fam = 0;
+    pos = 0;
+#pragma unroll
+    for (int d = ND - 1; d >= 0; --d) {
+      if (d >= rows.nd - 1) continue;
+      int const l = rows.lv[d];
+      unsigned const k = static_cast<unsigned>(row) & ((1u << l) - 1);
+      row >>= l;
+      int const tz = __ffs(k | (1u << l)) - 1;
+      int const s = l - tz;  // k = 0: tz = l, level 0
+      fi += s * rows.radix[d];
+      pos += static_cast<I>((k >> tz) >> 1) << log2fam;
+      log2fam += max(s - 1, 0);
+    }
+    long long const e = rows.families[fi];
+    base = static_cast<I>(e & ((1LL << kCtFamilyShift) - 1));
+    top = static_cast<int>(e >> kCtFamilyShift) - 1;
+    fam = static_cast<I>(1) << log2fam;
+  }
+  // Sparse point j of level s >= 1 of the row.
+  __device__ __forceinline__ I at(int s, unsigned j) const {
+    return base + ((fam + pos) << (s - 1)) + j;
+  }
+  // Sparse point of last-axis index k (its level in s).
+  __device__ __forceinline__ I of(unsigned k, int l, int &s) const {
+    int const tz = __ffs(k | (1u << l)) - 1;
+    s = l - tz;
+    return s == 0 ? base + pos : at(s, (k >> tz) >> 1);
+  }
+};
+
+template <typename S, int ND, typename I>
+__global__ void __launch_bounds__(kCtBlock)
+    ct_restrict_kernel(CtParams const p) {
+  int const g = p.unit_grid[blockIdx.x];
+  CtRows<ND, I> const rows(p, g);
+  unsigned long long const base = p.grids[g].base;
+  S *const out = reinterpret_cast<S *>(base);
+  S const *const val = reinterpret_cast<S const *>(p.values);
+  int total = 0;
+#pragma unroll
+  for (int d = 0; d < ND; ++d) total += rows.lv[d];
+  I const n = static_cast<I>(1) << total;
+  int const l = rows.last();
+  I const first =
+      static_cast<I>(blockIdx.x - p.unit_first[g]) * kCtUnit + 4 * threadIdx.x;
+  if (l >= 2) {
+    bool const vec = (base & 15) == 0;
+    S v[kCtGroups][4];
+    unsigned keep[kCtGroups];
+#pragma unroll
+    for (int q = 0; q < kCtGroups; ++q) {
+      I const f = first + q * 4 * kCtBlock;
+      keep[q] = 0;
+      if (f >= n) continue;
+      CtRow<I> const r(rows, f >> l);
+      unsigned const k = static_cast<unsigned>(f) & ((1u << l) - 1);
+      int s;
+      I const at0 = r.of(k, l, s);
+      if (s <= r.top) {
+        v[q][0] = val[at0];
+        keep[q] = 1;
+      }
+      if (l - 1 <= r.top) {
+        v[q][2] = val[r.at(l - 1, k >> 2)];
+        keep[q] |= 4;
+      }
+      if (l <= r.top) {
+        I const at1 = r.at(l, k >> 1);
+        v[q][1] = val[at1];
+        v[q][3] = val[at1 + 1];
+        keep[q] |= 10;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kCtGroups; ++q) {
+      S *const to = out + first + q * 4 * kCtBlock;
+      if (keep[q] == 15u && vec) {
+        constexpr int PER = 16 / sizeof(S);
+#pragma unroll
+        for (int i = 0; i < 4; i += PER) {
+          uint4 u;
+          memcpy(&u, &v[q][i], 16);
+          *reinterpret_cast<uint4 *>(to + i) = u;
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if ((keep[q] >> i) & 1u) to[i] = v[q][i];
+      }
+    }
+    return;
+  }
+  // Rows of one or two points: each point has a row of its own.
+  for (int q = 0; q < kCtGroups; ++q)
+    for (int i = 0; i < 4; ++i) {
+      I const f = first + q * 4 * kCtBlock + i;
+      if (f >= n) continue;
+      CtRow<I> const r(rows, f >> l);
+      int s;
+      I const at = r.of(static_cast<unsigned>(f) & ((1u << l) - 1), l, s);
+      if (s <= r.top) out[f] = val[at];
+    }
+}
+
+// Scatter: full[p] += sparse[p] on the full grid at the maximum level.
+__global__ void __launch_bounds__(kCtBlock) ct_scatter_kernel(
+    CtParams const p) {
   long long const first = static_cast<long long>(blockIdx.x) * kCtBlock;
   long long const point = first + threadIdx.x;
   if (point >= p.npoints) return;
-  // The CTA's first subspace comes from the host's table (a search of the
-  // whole list per CTA, behind a barrier, measured as the combine's second
-  // stall reason).
+  // The CTA's first subspace comes from the host's table. Most CTAs lie
+  // inside one subspace: one load settles that. Otherwise the CTA's 256
+  // points span at most 256 subspaces (each has at least one point): a
+  // binary search over those.
   int const sub0 = p.block_sub[blockIdx.x];
-  // Most CTAs lie inside one subspace: one load settles that. Otherwise
-  // the CTA's 256 points span at most 256 subspaces (each has at least one
-  // point): a binary search over those, instead of a walk that is as long
-  // as the number of small subspaces before the point.
   int sub = sub0;
   if (sub0 + 1 < p.nsubspaces && p.subspaces[sub0 + 1].offset <= point) {
     int lo = sub0 + 1;
@@ -160,55 +492,9 @@ __global__ void __launch_bounds__(kCtBlock) ct_kernel(CtParams const p) {
     sub = lo;
   }
   CtSubspace const &ss = p.subspaces[sub];
-  long long const local = point - ss.offset;
-  if (OP == kRestrict && ss.grid_end - ss.grid_begin > kCtHeavy) return;
-  if constexpr (OP == kScatter) {
-    long long const off = ct_offset(local, ss.level, p.max_level, p.ndim);
-    p.full[off] = __dadd_rn(p.full[off], p.sparse[point]);
-    return;
-  } else if constexpr (OP == kCombine) {
-    // acc = acc + c * v in grid order, rounded like the reference driver.
-    // With exact products fma(c, v, acc) rounds identically and issues one
-    // FP64 instruction instead of two; the choice is made once per thread,
-    // outside the loop, so that no thread evaluates both forms.
-    p.sparse[point] = p.exact_products != 0
-                          ? ct_combine_point<S, true>(p, ss, local)
-                          : ct_combine_point<S, false>(p, ss, local);
-  } else {
-    S const v = static_cast<S>(p.sparse[point]);
-    for (int gi = ss.grid_begin; gi < ss.grid_end; ++gi) {
-      CtGrid const &g = p.grids[p.grid_lists[gi]];
-      long long const off = ct_offset(local, ss.level, g.level, p.ndim);
-      reinterpret_cast<S *>(g.base)[off] = v;
-    }
-  }
-}
-
-// Restrict of the points of heavy subspaces, one warp per point: the lanes
-// write the point's value into 32 of its grids at a time.
-template <typename S>
-__global__ void __launch_bounds__(256) ct_heavy_restrict_kernel(
-    CtParams const p) {
-  long long const w =
-      (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  int const lane = threadIdx.x & 31;
-  if (w >= p.nheavy_points) return;
-  int lo = 0, hi = p.nheavy - 1;
-  while (lo < hi) {
-    int const mid = (lo + hi + 1) >> 1;
-    if (p.heavy_first[mid] <= w)
-      lo = mid;
-    else
-      hi = mid - 1;
-  }
-  CtSubspace const &ss = p.subspaces[p.heavy[lo]];
-  long long const local = w - p.heavy_first[lo];
-  S const v = static_cast<S>(p.sparse[ss.offset + local]);
-  for (int gi = ss.grid_begin + lane; gi < ss.grid_end; gi += 32) {
-    CtGrid const &g = p.grids[p.grid_lists[gi]];
-    long long const off = ct_offset(local, ss.level, g.level, p.ndim);
-    reinterpret_cast<S *>(g.base)[off] = v;
-  }
+  long long const off =
+      ct_offset(point - ss.offset, ss.level, p.max_level, p.ndim);
+  p.full[off] = __dadd_rn(p.full[off], p.sparse[point]);
 }
 
 } // namespace pgb
