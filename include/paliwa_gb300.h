@@ -67,7 +67,9 @@ const char *paliwa_gb_last_error(void);
 int paliwa_gb_version(void);
 
 /* Waits for the work queued on `stream` (the fence() of an execution-space
- * instance, paliwa/paliwa_utils.hpp:27-32). */
+ * instance, paliwa/paliwa_utils.hpp:27-32). PALIWA_GB_TIMEOUT if a bounded
+ * wait of a single-grid transform's tile copies gave up since the last
+ * report (the next transform call reports it too). */
 int paliwa_gb_synchronize(void *stream);
 
 /* Wavelet name -> id. Unknown names return PALIWA_GB_OUT_OF_RANGE, as
@@ -255,18 +257,17 @@ int paliwa_gb_batch_set_groups(paliwa_gb_batch *batch, int ngroups);
  * directions after synchronizing the device. No counterpart in the
  * reference. */
 int paliwa_gb_batch_use_slabs(paliwa_gb_batch *batch, int enable);
-/* enable != 0 (default): FP32-compensated stages of strided pencils of up
- * to 2048 points (up to 128 chunks; inner extent of 4 or more columns, or
- * of 2 with the pencil pairs one after another) and of the last axis'
- * pencils of up to 4096 points, in 16-byte aligned grids,
- * may run on the TMA wide kernel: the wide kernel's register transform,
- * with each tile moved between HBM and shared memory by bulk tensor copies
- * over a tensor map of the grid's axis (bounded waits, reported by
- * paliwa_gb_batch_status). It is the planner's default for them except the
- * strided 4-point chunks, which stay an autotuner choice. 0 keeps every
- * such stage on the wide, tile or staged kernel's per-thread copies.
- * Results are the same bits either way. Re-plans both directions after
- * synchronizing the device. No counterpart in the reference. */
+/* enable != 0 (default): stages of 16-byte aligned grids may run on the TMA
+ * wide kernel: the wide kernel's register transform, with each tile moved
+ * between HBM and shared memory by bulk tensor copies over a tensor map of
+ * the grid's axis (bounded waits, reported by paliwa_gb_batch_status). It
+ * applies to float pencils of up to 2048 points (strided: inner extent of 4
+ * or more columns, or of 2 with the pencil pairs one after another) and of up
+ * to 4096 along the last axis, and to double pencils of up to 1024 points,
+ * and is the planner's default for those it runs faster. 0 keeps every stage
+ * on the per-thread-copy kernels. Results are the same bits either way.
+ * Re-plans both directions after synchronizing the device. No counterpart in
+ * the reference. */
 int paliwa_gb_batch_use_tma(paliwa_gb_batch *batch, int enable);
 /* ctas > 0 caps every launch of the batch at that many CTAs per SM (the
  * kernels are persistent: by default a launch takes every slot that fits),
@@ -295,7 +296,9 @@ int paliwa_gb_batch_info(const paliwa_gb_batch *batch, int64_t *points,
  * trailing axes in one pass; its bytes count one read and one write of each
  * point), 2048 + R the TMA wide kernel (+ 32: pencils of 8 to 32 chunks,
  * + 64: more, + 96: the last axis, + 160: its pencils of more than 32
- * chunks, + 128: inner extent 2); `kernels` may be null. Call with
+ * chunks, + 128: inner extent 2; chunks of 32 doubles: 2048 + 224 with up to
+ * 4 of them per pencil, + 225 with more, + 226 along the last axis);
+ * `kernels` may be null. Call with
  * capacity 0 to get *nlaunches first. */
 int paliwa_gb_batch_profile(paliwa_gb_batch *batch, int forward, void *stream,
                             int capacity, int *nlaunches, float *ms,

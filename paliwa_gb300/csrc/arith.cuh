@@ -335,4 +335,41 @@ struct RowF64 {
   }
 };
 
+// Rows of 8 bytes, for the TMA wide kernel (twide.cuh): RowF32C above, two
+// columns of Plain<float, true> as one f32x2 pair, or one column of
+// Plain<double, true>.
+struct RowF32x2 {
+  using V = f2;
+  using Store = uint2;
+  static constexpr bool kPacked = false;
+  static __device__ __forceinline__ V load(Store u) {
+    return f2_bits(u.x, u.y);
+  }
+  static __device__ __forceinline__ Store store(V v) {
+    return {f2_lo(v), f2_hi(v)};
+  }
+  template <bool C1>
+  static __device__ __forceinline__ V update(Coeffs const &c, V lo, V me,
+                                             V up) {
+    return RowF32::template pair<C1>(c, lo, me, up);
+  }
+};
+struct ColF64 {
+  using V = double;
+  using Store = uint2;
+  static constexpr bool kPacked = false;
+  static __device__ __forceinline__ V load(Store u) {
+    return __hiloint2double(static_cast<int>(u.y), static_cast<int>(u.x));
+  }
+  static __device__ __forceinline__ Store store(V v) {
+    return {static_cast<unsigned>(__double2loint(v)),
+            static_cast<unsigned>(__double2hiint(v))};
+  }
+  template <bool C1>
+  static __device__ __forceinline__ V update(Coeffs const &c, V lo, V me,
+                                             V up) {
+    return Plain<double, true>::template update<C1>(c, lo, me, up);
+  }
+};
+
 } // namespace pgb

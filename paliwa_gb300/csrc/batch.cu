@@ -21,20 +21,16 @@
 #include <unordered_map>
 #include <vector>
 
-#include <cudaTypedefs.h>
-
 #include "combine.cuh"
 #include "paliwa_gb300.h"
 #include "plan.hpp"
 #include "slab.cuh"
-#include "twide.cuh"
+#include "twide_plan.hpp"
 
 namespace pgb {
 void launch_slab_f64(int sched, SlabParams const &p, cudaStream_t s);
 void launch_slab_f32(int sched, SlabParams const &p, cudaStream_t s);
 void launch_slab_f32c(int sched, SlabParams const &p, cudaStream_t s);
-void launch_twide_f32c(int sched, int R, TWideParams const &p,
-                       cudaStream_t s);
 } // namespace pgb
 
 using namespace pgb;
@@ -46,10 +42,9 @@ namespace {
 // group, 26.1 with two, 25.7 with three, 25.6 with four.
 constexpr int kBatchGroups = 4;
 
-// Kernel code of a slab launch (slab.cuh) and, plus the chunk size, of a
-// TMA wide launch (twide.cuh); the others are plan.hpp's.
+// Kernel code of a slab launch (slab.cuh); the others are plan.hpp's and
+// twide_plan.hpp's.
 constexpr int kSlab = 1024;
-constexpr int kTWide = 2048;
 
 struct Launch {
   int group = 0;
@@ -162,7 +157,7 @@ struct paliwa_gb_batch {
   // Slab launches (slab.cuh): the tensor map over the grids' memory as
   // 128-byte rows from slab_base, and the error word of their bounded waits.
   bool use_slabs = true;
-  // TMA wide launches for strided wide stages of FP32c grids.
+  // TMA wide launches for the stages planned on them.
   bool use_tma = true;
   bool slab_map_ok = false;
   unsigned long long slab_base = 0;
@@ -246,17 +241,8 @@ SlabJob slab_job(paliwa_gb_batch const &b, int g, int m,
 // (8 rows), 128-byte swizzle.
 bool encode_slab_map(CUtensorMap *map, unsigned long long base,
                      unsigned long long rows, size_t es) {
-  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-  if (encode == nullptr) {
-    cudaDriverEntryPointQueryResult q{};
-    void *fn = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000,
-                                         cudaEnableDefault,
-                                         &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || fn == nullptr)
-      return false;
-    encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-  }
+  auto const encode = tensor_map_encoder();
+  if (encode == nullptr) return false;
   if (rows == 0 || rows > (1ULL << 31)) return false;
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(128 / es), rows};
   cuuint64_t strides[1] = {128};
@@ -269,172 +255,6 @@ bool encode_slab_map(CUtensorMap *map, unsigned long long base,
       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
-}
-
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-  if (encode == nullptr) {
-    cudaDriverEntryPointQueryResult q{};
-    void *fn = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000,
-                                         cudaEnableDefault,
-                                         &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || fn == nullptr)
-      return nullptr;
-    encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-  }
-  return encode;
-}
-
-// Chunk size of the TMA wide launch that may take a stage (the stage's own
-// kernel otherwise): strided wide stages (chunks of 2-16 points, up to 4 per
-// pencil), and tile or staged stages of pencils of 128 to 2048 points (8 to
-// 128 chunks of 16 points); 0 for the rest.
-int twide_chunk(Stage const &st) {
-  int const R = st.R;
-  if (R == kWide + 2 || R == kWide + 4 || R == kWide + 8 || R == kWide + 16)
-    return R - kWide;
-  if (R == kWideContig + 4 || R == kWideContig + 8 || R == kWideContig + 16)
-    return R - kWideContig;
-  bool const last = st.job.log2_inner == 0 && st.job.log2_kstride == 0;
-  if ((R == kTile + 16 || R == kTileLong + 16 || R == 16 || R == 32) &&
-      st.job.log2_n >= 7 && st.job.log2_n <= (last ? 12 : 11))
-    return 16;
-  return 0;
-}
-
-// The TMA wide job and tensor map of a strided stage (FP32c, float storage)
-// with chunks of r points, covering tiles of Ct = 2 NT / G columns. Up to 4
-// chunks per pencil: the 3D view [outer][n][inner] of the stage's pencils
-// with the axis' strides and boxes {Bx, n, Sx}. 8 to 128 chunks of 16
-// points (the chunked layout): the 5D view [outer][inner / 4][row of
-// chunk][chunk][4 columns] and one box per tile, so that shared memory holds
-// the tile as [column quad][row of chunk][chunk][4 columns]. False when the
-// stage does not qualify (alignment, inner extent under 4 columns, more than
-// 128 chunks, 2^30 tiles or more, or the encoder refuses the map).
-bool twide_job(Stage const &st, int r, TWideJob &job, CUtensorMap &map,
-               long long &tiles) {
-  auto encode = tensor_map_encoder();
-  LiftJob const &lj = st.job;
-  int const log2r = 31 - __builtin_clz(static_cast<unsigned>(r));
-  int const log2G = lj.log2_n - log2r;
-  if (encode == nullptr || lj.periodic != 1 || lj.base % 16 != 0)
-    return false;
-  bool const last = lj.log2_inner == 0 && lj.log2_kstride == 0;
-  bool const pairs = lj.log2_inner == 1 && lj.log2_kstride == 1 &&
-                     lj.log2_astride == lj.log2_n + 1;
-  if (last || pairs) {
-    // The last axis (contiguous layout), or a strided axis of inner extent
-    // 2 whose pencil pairs lie one after another (pairs layout): the
-    // stage's points as rows of 32 floats (128 bytes), boxes of the unit's
-    // 16 r rows, 128-byte swizzle; units of 512 r floats (whole pencils).
-    if (r < 4 || log2G < 0 || log2G > (pairs ? 2 : 5 + 3 * (r == 16)))
-      return false;
-    long long const points = lj.columns << lj.log2_n;
-    int const log2unit = 9 + log2r;
-    int const log2u = r >= 8 ? 0 : 3 - log2r;  // units per tile
-    if (points % 32 != 0 || (points >> (log2unit + log2u)) >= (1LL << 30))
-      return false;
-    tiles = (points + (1LL << (log2unit + log2u)) - 1) >> (log2unit + log2u);
-    std::memset(&job, 0, sizeof(job));
-    job.log2_n = lj.log2_n;
-    job.nlevels = lj.nlevels;
-    job.chunked = pairs ? 3 : 2;
-    job.nxb = 1;
-    job.log2_bx = log2unit - lj.log2_n;  // box bytes = the unit
-    job.log2_sx = 0;
-    cuuint64_t dims[2] = {32, static_cast<cuuint64_t>(points / 32)};
-    cuuint64_t strides[1] = {128};
-    cuuint32_t box[2] = {32, static_cast<cuuint32_t>(16 * r)};
-    cuuint32_t elem[2] = {1, 1};
-    CUresult const res = encode(
-        &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
-        reinterpret_cast<void *>(lj.base), dims, strides, box, elem,
-        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return res == CUDA_SUCCESS;
-  }
-  if (lj.log2_inner < 2 || log2G < 0 || log2G > 7 || lj.log2_n > 11 ||
-      (log2G > 2 && r != 16))
-    return false;
-  int const log2ct = Log2<kTWideThreads>::value + 1 - log2G;
-  // Units per tile: TWideShape<R>::kUnits (16 KB tiles for chunks of up to
-  // 8 points).
-  int const log2u = r >= 8 ? 0 : 3 - log2r;
-  std::memset(&job, 0, sizeof(job));
-  job.log2_n = lj.log2_n;
-  job.log2_inner = lj.log2_inner;
-  job.nlevels = lj.nlevels;
-  job.log2_bx = std::min(std::min(lj.log2_inner, log2ct), 8);
-  job.log2_sx = std::max(0, log2ct - lj.log2_inner);
-  job.nxb = 1 << (log2ct - job.log2_bx - job.log2_sx);
-  job.log2_rs = job.log2_bx;
-  tiles = (lj.columns + (1LL << (log2ct + log2u)) - 1) >> (log2ct + log2u);
-  if (tiles >= (1LL << 30)) return false;
-  long long const outer = lj.columns >> lj.log2_inner;
-  if (log2G >= 3) {
-    job.chunked = 1;
-    job.nxb = 1;
-    job.log2_bx = std::min(lj.log2_inner, log2ct);  // Bx >= 4: log2ct <= 6
-    job.log2_sx = log2ct - job.log2_bx;
-    // Groups of 8 columns (32-byte box rows) where the tile and the inner
-    // extent hold them, else 4 (16 bytes, the least a box row may be):
-    // wider rows halve the rows the tensor memory accelerator moves (the
-    // chunked form: 3.91 against 3.5 TB/s on the 4D batch). Not for more
-    // than 32 chunks, whose warps would read 8-way conflicting banks (the
-    // long form measured slower with them).
-    int const xlo = log2ct >= 3 && lj.log2_inner >= 3 && log2G <= 5 ? 3 : 2;
-    job.log2_xlo = xlo;
-    job.log2_rs = log2G + xlo;
-    cuuint64_t dims[5] = {1u << xlo, static_cast<cuuint64_t>(1) << log2G,
-                          static_cast<cuuint64_t>(r),
-                          static_cast<cuuint64_t>(1) << (lj.log2_inner - xlo),
-                          static_cast<cuuint64_t>(outer)};
-    cuuint64_t strides[4] = {
-        static_cast<cuuint64_t>(4 * r) << lj.log2_kstride,
-        static_cast<cuuint64_t>(4) << lj.log2_kstride,
-        static_cast<cuuint64_t>(4) << xlo,
-        static_cast<cuuint64_t>(4) << lj.log2_astride};
-    cuuint32_t box[5] = {1u << xlo, 1u << log2G, static_cast<cuuint32_t>(r),
-                         1u << (job.log2_bx - xlo), 1u << job.log2_sx};
-    cuuint32_t elem[5] = {1, 1, 1, 1, 1};
-    CUresult const res = encode(
-        &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5,
-        reinterpret_cast<void *>(lj.base), dims, strides, box, elem,
-        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return res == CUDA_SUCCESS;
-  }
-  cuuint64_t dims[3] = {static_cast<cuuint64_t>(1) << lj.log2_inner,
-                        static_cast<cuuint64_t>(1) << lj.log2_n,
-                        static_cast<cuuint64_t>(outer)};
-  cuuint64_t strides[2] = {static_cast<cuuint64_t>(4) << lj.log2_kstride,
-                           static_cast<cuuint64_t>(4) << lj.log2_astride};
-  cuuint32_t box[3] = {1u << job.log2_bx, 1u << lj.log2_n,
-                       1u << job.log2_sx};
-  // An outer index's n rows of `inner` columns are one contiguous block
-  // when the pencil stride is the inner extent (no sub-lattice). When a
-  // tile holds whole blocks (inner < Ct) and a block fits one box
-  // dimension, the map takes the block as its rows: box rows of n inner
-  // floats instead of inner (fewer, longer rows for the tensor memory
-  // accelerator), the same bytes in the same shared-memory order, the same
-  // box coordinates (x = y = 0).
-  if (lj.log2_kstride == lj.log2_inner && lj.log2_inner < log2ct &&
-      lj.log2_n + lj.log2_inner <= 8) {
-    int const log2blk = lj.log2_n + lj.log2_inner;
-    dims[0] = static_cast<cuuint64_t>(1) << log2blk;
-    dims[1] = 1;
-    strides[0] = static_cast<cuuint64_t>(4) << log2blk;
-    box[0] = 1u << log2blk;
-    box[1] = 1;
-  }
-  cuuint32_t elem[3] = {1, 1, 1};
-  CUresult const res = encode(
-      &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
-      reinterpret_cast<void *>(lj.base), dims, strides, box, elem,
-      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return res == CUDA_SUCCESS;
 }
 
 // The tensor map over every grid of the batch (rows of 128 bytes from the
@@ -470,8 +290,8 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
   std::vector<CUtensorMap> maps;
   size_t const es = dtype_size(b.dtype);
   int const ws = wavelet_schedule(filters);
-  bool const tma = b.use_tma && dr.tma && b.dtype == PALIWA_GB_F32C &&
-                   ws >= 0 && tensor_map_encoder() != nullptr;
+  bool const tma =
+      b.use_tma && dr.tma && ws >= 0 && tensor_map_encoder() != nullptr;
   // First axis of every grid's slab group (ndim: none).
   std::vector<int> slab_from(b.ngrids, b.ndim);
   if (b.use_slabs && dr.slabs && b.slab_map_ok && ws >= 0)
@@ -524,17 +344,9 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
           if (k < stages[i].size()) {
             Stage const &st = stages[i][k];
             int code = st.R;
-            int const r = twide_chunk(st);
-            if (tma && st.tma && r > 0 &&
-                canonical_shifts(st.job, (ws & 1) != 0)) {
-              int const log2G = st.job.log2_n - (31 - __builtin_clz(r));
-              bool const last =
-                  st.job.log2_inner == 0 && st.job.log2_kstride == 0;
-              code = kTWide + r +
-                     (last ? (log2G > 5 ? kTWideLongContig : kTWideContig)
-                      : st.job.log2_inner == 1 ? kTWidePairs
-                      : log2G > 5 ? kTWideLong
-                      : log2G >= 3 ? kTWideChunked : 0);
+            if (tma && canonical_shifts(st.job, (ws & 1) != 0)) {
+              int const form = twide_code(st, b.dtype);
+              if (form != 0) code = kTWide + form;
             }
             by_r[code].push_back(&st);
           }
@@ -546,14 +358,22 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
             L.sched = ws;
             L.job_first = all_twide.size();
             L.tile_first = twide_tiles.size();
-            // Stages that do not qualify, by their own kernel.
+            // Stages that do not qualify, by their own kernel; all of them
+            // when they are too few points together.
             std::map<int, std::vector<Stage const *>> rest;
+            long long points = 0;
+            bool tuned = false;
+            for (Stage const *st : list) {
+              points += stage_points(*st);
+              tuned |= st->tuned;
+            }
+            bool const enough =
+                tuned || twide_enough(R - kTWide, b.dtype, points);
             for (Stage const *st : list) {
               TWideJob job;
               CUtensorMap map;
               long long tiles = 0;
-              if (!twide_job(*st, (R - kTWide) % kTWideChunked, job, map,
-                             tiles)) {
+              if (!enough || !twide_job(*st, b.dtype, job, map, tiles)) {
                 rest[st->R].push_back(st);
                 continue;
               }
@@ -678,7 +498,7 @@ void launch_one(paliwa_gb_batch &b, Direction &dr, Launch const &L,
     p.total_tiles = L.tiles;
     p.error = b.slab_error;
     p.ctas_per_sm = b.ctas_per_sm;
-    launch_twide_f32c(L.sched, L.R - kTWide, p, s);
+    launch_twide(b.dtype, L.sched, L.R - kTWide, p, s);
     return;
   }
   if (L.R != kSlab) {

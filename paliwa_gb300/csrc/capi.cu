@@ -7,6 +7,7 @@
 
 #include "paliwa_gb300.h"
 #include "launch.cuh"
+#include "twide_plan.hpp"
 
 namespace pgb {
 
@@ -205,27 +206,23 @@ KernelSet periodic_kernels(AxisView const &v, bool canon) {
       v.log2_inner + v.log2_es >=
           tile_piece_log2(log2G, v.log2_row + v.log2_es))
     k.mask |= 1 << kChooseTile;
-  // The TMA wide kernel: FP32c strided stages, 16-byte aligned, inner
-  // extents of 4 or more columns; wide stages of up to 4 chunks, and
-  // pencils of 8 to 128 chunks of 16 points (128 to 2048 points).
-  if (!last && v.wide_last && v.log2_inner >= 2 && v.base % 16 == 0 &&
-      v.columns < (1LL << 30) &&
-      ((k.has(kChooseWide) &&
-        v.log2_n - (31 - __builtin_clz(static_cast<unsigned>(
-                             wide_chunk(v.log2_n)))) <= 2) ||
-       (R == 16 && log2G >= 3 && log2G <= 7)))
-    k.mask |= 1 << kChooseTmaWide;
-  // ... and the last axis' wide stages of chunks of 4 to 16 points and its
-  // pencils of 64 to 256 chunks of 16 points (1024 to 4096 points), and the
-  // wide stages of strided axes of inner extent 2 whose pencil pairs lie
-  // one after another.
-  if (last && v.wide_last && v.base % 16 == 0 &&
-      ((k.has(kChooseWide) && R >= 4) ||
-       (R == 16 && log2G >= 6 && log2G <= 8)))
-    k.mask |= 1 << kChooseTmaWide;
-  if (!last && v.wide_last && k.has(kChooseWide) && v.log2_inner == 1 &&
-      v.log2_kstride == 1 && v.log2_astride == v.log2_n + 1 &&
-      wide_chunk(v.log2_n) >= 4 && v.base % 16 == 0)
+  // The TMA wide kernel: 16-byte aligned grids under a wavelet schedule.
+  // Floats: strided pencils of up to 2048 points whose inner extent is 4 or
+  // more columns, or 2 with the pencil pairs one after another (up to 64
+  // points); the last axis' pencils of 4 to 4096 points. Doubles: pencils of
+  // up to 1024 points, strided ones of 2 or more columns (a box row is at
+  // least 16 bytes).
+  bool const pairs = !last && v.log2_inner == 1 && v.log2_kstride == 1 &&
+                     v.log2_astride == v.log2_n + 1;
+  bool tma = false;
+  if (v.log2_es == 3)
+    tma = last ? v.log2_n >= 2 && v.log2_n <= 10
+               : v.log2_inner >= 1 && v.log2_n <= 10;
+  else
+    tma = last ? v.log2_n >= 2 && v.log2_n <= 12
+               : (v.log2_inner >= 2 && v.log2_n <= 11) ||
+                     (pairs && v.log2_n >= 2 && v.log2_n <= 6);
+  if (tma && canon && v.base % 16 == 0 && v.columns < (1LL << 29))
     k.mask |= 1 << kChooseTmaWide;
   // Default: the wide kernel for strided pencils (and FP32c last-axis
   // pencils: measured on 2^26-point grids, 3.0-4.5 TB/s against 2.8-4.1 on
@@ -245,26 +242,35 @@ KernelSet periodic_kernels(AxisView const &v, bool canon) {
   else
     k.dflt = staged_chunk(v) == 32 ? kChooseStaged32 : kChooseStaged;
   k.fallback = k.dflt;
-  // (The TMA wide kernel is the default for strided wide chunks of 8 and
-  // 16 points, for strided pencils of 8 to 128 chunks and for the last
-  // axis' wide stages, measured on the 4D CT batch: per launch 4.73 against
-  // 4.01 TB/s at 8 points, 4.73 against 3.16 at 16, about 3.7 against 2.29
-  // on the tile kernel's pencils of 128 and 256 points, 0.46 against 0.71
-  // ms on the staged kernel's pencils of 512; on pencils of 1024 and 2048
-  // points, whose chunks exchange through shared memory, as fast as the
-  // staged kernel per launch (0.92 ms each) and the step 21.59 against
-  // 22.02 ms with it; on the last axis 4.86 against 3.60 TB/s at 16 points,
-  // 4.97 against 4.42 at 8 and 4.96 against 4.79 at 4 (the step 20.37
-  // against 21.20 ms), and on its pencils of 1024-4096 points 0.39 against
-  // 0.41 ms on the staged kernel (19.71 against 19.81 ms); on strided axes
-  // of inner extent 2, 3.3-3.5 against 1.4-2.0 TB/s (20.15 against 20.30
-  // ms). On strided 4-point chunks of
-  // wider inner extents the wide kernel is faster, 5.26 against 4.39-4.55
-  // TB/s.)
-  if (k.has(kChooseTmaWide) &&
-      (last || v.log2_inner == 1 || wide_chunk(v.log2_n) >= 8 ||
-       !k.has(kChooseWide)))
-    k.dflt = kChooseTmaWide;
+  // The TMA wide kernel is the default where it was measured faster
+  // (forward CDF (2,2) along one axis of 2^26-point grids, GB/s against the
+  // default above; several inner extents):
+  //  * the last axis and inner extent 2: every length (FP32 n = 512 5800
+  //    against 5170, n = 2048 6020 against 3740; FP32c n = 512 3690 against
+  //    3000, inner extent 2 n = 8 5950 against 3240; FP64 n = 512 1830
+  //    against 1510);
+  //  * strided FP64 pencils of 8 points and more (equal at 8, n = 512 1830
+  //    against 1360);
+  //  * strided float pencils of 8 points and more (FP32c n = 128 4670 against
+  //    2920, n = 2048 3430 against 2380; FP32 n = 512 5530 against 4850), but
+  //    FP32 up to 512 only (n = 1024, 16 columns: 3610 against 4650 on the
+  //    tile kernel). On 4-point chunks the two are within 1 % for single
+  //    grids, and the wide kernel is faster in batches (5.26 against
+  //    4.39-4.55 TB/s).
+  // Not where 32 or more chunks lie on more than 16 pages of 2 MB (pencils of
+  // 64 MB and more): a box visits the chunks row by row, so every box row
+  // then waits for its page, 8 clocks each (FP32c n = 512, 256 KB rows: 1240
+  // against 2600 GB/s, 64 KB rows 3720 against 2620; n = 1024 from 64 KB rows
+  // on 1650 against 2590; FP64 n = 1024 1250 against 1520).
+  if (k.has(kChooseTmaWide)) {
+    int const longest = v.log2_es == 3 ? 10 : v.wide_last ? 11 : 9;
+    int const log2chunks = v.log2_n - (v.log2_es == 3 ? 5 : 4);
+    bool const pages = log2chunks >= 5 &&
+                       v.log2_n + v.log2_kstride + v.log2_es >= 26;
+    if (last || pairs ||
+        (v.log2_n >= 3 && v.log2_n <= longest && !pages))
+      k.dflt = kChooseTmaWide;
+  }
   return k;
 }
 
@@ -305,8 +311,10 @@ void plan_periodic(AxisView const &v, std::vector<int> const &shifts, int ws,
     int choice = ks.dflt;
     if (tuning != nullptr) {
       auto const it = tuning->choice.find(tuning_class(v));
-      if (it != tuning->choice.end() && ks.has(it->second))
+      if (it != tuning->choice.end() && ks.has(it->second)) {
         choice = it->second;
+        st.tuned = true;
+      }
     }
     auto tile_stage = [&] {
       st.R = (log2G <= 5 ? kTile : kTileLong) + 16;
@@ -314,8 +322,8 @@ void plan_periodic(AxisView const &v, std::vector<int> const &shifts, int ws,
           ceil_div(v.columns >> v.log2_row, kThreads >> log2G);
     };
     if (choice == kChooseTmaWide) {
-      // Marked for the TMA wide kernel (batches); elsewhere, and for the
-      // grids that do not qualify, planned for the kernel it stands in for.
+      // Marked for the TMA wide kernel, and planned for the kernel it stands
+      // in for, which runs the stages that do not qualify.
       st.tma = true;
       choice = ks.fallback;
     }
@@ -562,13 +570,8 @@ void transform_axis(void *grid, int dtype, int ndim, int64_t const *level,
     bool const exact = exact_scalers(filters);
     bool const sym = symmetric_filters(filters);
     int const ws = wavelet_schedule(filters);
-    for (auto const &st : stages) {
-      LiftParams p = params;
-      p.job = st.job;
-      int const sched =
-          ws >= 0 && canonical_shifts(st.job, (ws & 1) != 0) ? ws : -1;
-      launch_lift(dtype, exact, sym, sched, st.R, p, nullptr, 1, st.tiles, s);
-    }
+    for (auto const &st : stages)
+      launch_stage(dtype, exact, sym, ws, params, st, s);
   } catch (...) {
     if (shadow) cudaFreeAsync(shadow, s);
     throw;
@@ -614,6 +617,7 @@ int paliwa_gb_synchronize(void *stream) {
   return guarded([&] {
     cuda_check(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)),
                "cudaStreamSynchronize");
+    check_stage_errors();
   });
 }
 

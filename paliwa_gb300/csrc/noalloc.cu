@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "launch.cuh"
+#include "twide_plan.hpp"
 #include "paliwa_gb300.h"
 
 namespace {
@@ -113,13 +114,7 @@ extern "C" int paliwa_gb_transform_noalloc(void *grid, int dtype, int ndim,
       plan_axis(view, shifts, filters, plans[d]);
     }
     for (auto const &stages : plans)
-      for (auto const &st : stages) {
-        LiftParams p = params;
-        p.job = st.job;
-        int const sched =
-            ws >= 0 && canonical_shifts(st.job, (ws & 1) != 0) ? ws : -1;
-        launch_lift(dtype, exact, sym, sched, st.R, p, nullptr, 1, st.tiles,
-                    s);
-      }
+      for (auto const &st : stages)
+        launch_stage(dtype, exact, sym, ws, params, st, s);
   });
 }

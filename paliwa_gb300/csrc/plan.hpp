@@ -83,8 +83,10 @@ struct Stage {
   int tclass = 0;
   unsigned kernels = 0;
   int dflt = 0;
-  // A wide stage that a batch runs on the TMA wide kernel.
+  // A stage planned on the TMA wide kernel, and whether a tuning chose it
+  // (otherwise launches of few points keep the stage's own kernel).
   bool tma = false;
+  bool tuned = false;
 };
 
 constexpr int kWindowLog2 = 12;   // points per column per CTA round (4096)

@@ -56,8 +56,12 @@
 
 namespace pgb {
 
-constexpr int kTWideThreads = 256;               // transform threads
-constexpr int kTWideBlock = kTWideThreads + 32;  // + the producer warp
+constexpr int kTWideThreads = 256;  // transform threads
+// Chunks of 32 points (FP64) take 128, for tiles of the same 32 KB; the
+// producer warp comes on top.
+__host__ __device__ constexpr int twide_threads(int r) {
+  return r >= 32 ? kTWideThreads / 2 : kTWideThreads;
+}
 // Added to the chunk size of a launch whose pencils have 8 to 32 chunks
 // (chunked form), more than 32 chunks (long form), lie along the last axis
 // (contiguous form; more than 32 chunks: long contiguous form) or along a
@@ -67,6 +71,11 @@ constexpr int kTWideLong = 64;
 constexpr int kTWideContig = 96;
 constexpr int kTWidePairs = 128;
 constexpr int kTWideLongContig = 160;
+// Launch codes of the forms with 32-point chunks (FP64): dense, chunked and
+// pairs.
+constexpr int kTWide32Dense = 224;
+constexpr int kTWide32Chunked = 225;
+constexpr int kTWide32Pairs = 226;
 
 struct TWideJob {
   long long tile_begin;  // first tile of this job in the launch
@@ -92,6 +101,9 @@ struct TWideParams {
   long long total_tiles;
   unsigned *error;          // set to 1 when a bounded wait gives up
   int ctas_per_sm;          // cap on the launch's CTAs per SM (0: none)
+  // jobs == nullptr: the launch's only job and its map.
+  TWideJob job;
+  CUtensorMap map;
 };
 
 __device__ __forceinline__ void tma_load_3d(void *dst, void const *map, int x,
@@ -134,7 +146,7 @@ __device__ __forceinline__ void fence_tensormap(void const *map) {
 // dominated 8 KB ones); kStages tile buffers per CTA.
 template <int R> struct TWideShape {
   static constexpr int kUnits = R >= 8 ? 1 : 8 / R;
-  static constexpr int kUnitBytes = 8 * kTWideThreads * R;
+  static constexpr int kUnitBytes = 8 * twide_threads(R) * R;
   static constexpr int kTileBytes = kUnits * kUnitBytes;
   static constexpr int kStages = R >= 16 ? 3 : 4;
   static constexpr size_t kSmemBytes =
@@ -208,7 +220,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar,
 // kernel for several forms kept more registers live and spilled.) Longer
 // pencils (form 2 and 5 of the launch codes): twide_long_kernel below.
 template <class A, int R, class Sched, int FORM>
-__global__ void __launch_bounds__(kTWideBlock, R >= 16 ? 2 : 3)
+__global__ void __launch_bounds__(twide_threads(R) + 32, R >= 16 ? 2 : 3)
     twide_kernel(__grid_constant__ const TWideParams p) {
   constexpr bool CHUNKED = FORM == 1;
   constexpr bool PAIRS = FORM == 4;
@@ -216,7 +228,7 @@ __global__ void __launch_bounds__(kTWideBlock, R >= 16 ? 2 : 3)
   using V = typename A::V;
   using W = typename A::Store;
   static_assert(sizeof(W) == 8, "rows of two float columns");
-  constexpr int NT = kTWideThreads;
+  constexpr int NT = twide_threads(R);
   constexpr int S = TWideShape<R>::kStages;
   constexpr int TILE = TWideShape<R>::kTileBytes;
   constexpr int U = TWideShape<R>::kUnits;
@@ -273,19 +285,23 @@ __global__ void __launch_bounds__(kTWideBlock, R >= 16 ? 2 : 3)
     return 4 << (job.log2_bx + job.log2_n + job.log2_sx);
   };
   // Contiguous layout: the first 128-byte row of unit u of `tile` (a unit
-  // is 16 R rows).
+  // is 2 NT R / 32 rows).
   auto contig_row = [](TWideJob const &job, long long tile, int u) {
-    return static_cast<int>(((tile - job.tile_begin) * U + u) << (LOG2R + 4));
+    return static_cast<int>(((tile - job.tile_begin) * U + u)
+                            << (LOG2R + LOG2NT - 4));
   };
 
   // The producer lane issues every copy; it keeps the last map it fenced.
-  int fenced = -1;
+  // A single job's map (0) lies in the parameters and needs no fence.
+  TWideJob const *const jobs = p.jobs != nullptr ? p.jobs : &p.job;
+  CUtensorMap const *const maps = p.jobs != nullptr ? p.maps : &p.map;
+  int fenced = p.jobs != nullptr ? -1 : 0;
   auto issue_load = [&](long long k) {
     int const b = static_cast<int>(k % S);
     long long const tile = first + k * step;
-    sjob[b] = p.jobs[p.tile_job[tile]];
+    sjob[b] = jobs[p.tile_job != nullptr ? p.tile_job[tile] : 0];
     TWideJob const &job = sjob[b];
-    void const *const map = p.maps + job.map;
+    void const *const map = maps + job.map;
     if (job.map != fenced) {
       fence_tensormap(map);
       fenced = job.map;
@@ -316,7 +332,7 @@ __global__ void __launch_bounds__(kTWideBlock, R >= 16 ? 2 : 3)
     int const b = static_cast<int>(k % S);
     long long const tile = first + k * step;
     TWideJob const &job = sjob[b];
-    void const *const map = p.maps + job.map;
+    void const *const map = maps + job.map;
     int const bb = box_bytes(job);
     for (int u = 0; u < U; ++u) {
       int x0, z0;
@@ -392,14 +408,15 @@ __global__ void __launch_bounds__(kTWideBlock, R >= 16 ? 2 : 3)
     // more than 32 chunks would take exchange paths that need a barrier).
     bool const valid =
         CONTIG ? R >= 4 && job.chunked == (PAIRS ? 3 : 2) &&
-                     static_cast<unsigned>(log2G) <= (PAIRS ? 2u : 5u)
-               : (CHUNKED ? R == 16 && job.chunked == 1 && log2G >= 3 &&
-                                log2G <= 5
+                     static_cast<unsigned>(log2G) <=
+                         (PAIRS && R < 32 ? 2u : 5u)
+               : (CHUNKED ? R >= 16 && job.chunked == 1 &&
+                                log2G >= 3 && log2G <= 5
                           : !job.chunked &&
                                 static_cast<unsigned>(log2G) <= 2u) &&
                      job.log2_rs ==
                          (CHUNKED ? log2G + job.log2_xlo : job.log2_bx) &&
-                     (!CHUNKED || (job.log2_xlo >= 2 && job.log2_xlo <= 3));
+                     (!CHUNKED || (job.log2_xlo >= 2 && job.log2_xlo <= 4));
     if constexpr (CONTIG) {
       if (valid) {
         // Thread = (chunk c, column pair g): the G chunks of a pencil pair
@@ -576,7 +593,10 @@ __global__ void __launch_bounds__(kTWideThreads, 2)
 
   // Thread 0's copies (one box per tile: 5D, or 2D of 16 R rows of 128
   // bytes); it keeps the last map it fenced.
-  int fenced = -1;
+  // A single job's map (0) lies in the parameters and needs no fence.
+  TWideJob const *const jobs = p.jobs != nullptr ? p.jobs : &p.job;
+  CUtensorMap const *const maps = p.jobs != nullptr ? p.maps : &p.map;
+  int fenced = p.jobs != nullptr ? -1 : 0;
   auto origin = [](TWideJob const &job, long long tile, int &q0, int &z0) {
     int const log2ct = LOG2NT + 1 - (job.log2_n - LOG2R);
     long long const col0 = (tile - job.tile_begin) << log2ct;
@@ -587,9 +607,9 @@ __global__ void __launch_bounds__(kTWideThreads, 2)
   auto issue_load = [&](long long k) {
     int const b = static_cast<int>(k % S);
     long long const tile = first + k * step;
-    sjob[b] = p.jobs[p.tile_job[tile]];
+    sjob[b] = jobs[p.tile_job != nullptr ? p.tile_job[tile] : 0];
     TWideJob const &job = sjob[b];
-    void const *const map = p.maps + job.map;
+    void const *const map = maps + job.map;
     if (job.map != fenced) {
       fence_tensormap(map);
       fenced = job.map;
@@ -610,13 +630,13 @@ __global__ void __launch_bounds__(kTWideThreads, 2)
     long long const tile = first + k * step;
     TWideJob const &job = sjob[b];
     if constexpr (CONTIG) {
-      tma_store_2d(reinterpret_cast<CUtensorMap const *>(p.maps + job.map), 0,
+      tma_store_2d(reinterpret_cast<CUtensorMap const *>(maps + job.map), 0,
                    static_cast<int>((tile - job.tile_begin) << (LOG2R + 4)),
                    tiles + b * TILE);
     } else {
       int q0, z0;
       origin(job, tile, q0, z0);
-      tma_store_5d(p.maps + job.map, q0, z0, tiles + b * TILE);
+      tma_store_5d(maps + job.map, q0, z0, tiles + b * TILE);
     }
     bulk_commit();
   };

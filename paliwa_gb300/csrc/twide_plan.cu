@@ -1,0 +1,298 @@
+// Host side of the TMA wide kernel: stages, jobs, tensor maps and launches
+// of single grids.
+#include <algorithm>
+#include <atomic>
+#include <cstring>
+#include <mutex>
+
+#include "paliwa_gb300.h"
+#include "twide_plan.hpp"
+
+namespace pgb {
+
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+  static PFN_cuTensorMapEncodeTiled_v12000 const encode = [] {
+    cudaDriverEntryPointQueryResult q{};
+    void *fn = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000,
+                                         cudaEnableDefault,
+                                         &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+  }();
+  return encode;
+}
+
+namespace {
+
+// Points per thread of the TMA wide kernel (0: it does not take the stage).
+// Floats: whole pencils of up to 16 points, chunks of n / 4 points up to 64
+// (a strided axis) and of 16 points beyond. Doubles: whole pencils of up to
+// 32 points and chunks of 32 beyond: the FP64 pipe runs a coarse step of one
+// head per chunk as a whole warp instruction, so half the chunks are half
+// that waste (512 points: 140 instead of 160 DFMAs for every 128 needed).
+int twide_chunk(LiftJob const &job, int dtype) {
+  int const n = job.log2_n;
+  bool const last = job.log2_inner == 0 && job.log2_kstride == 0;
+  if (dtype == PALIWA_GB_F64) return n < 1 || n > 10 ? 0 : 1 << std::min(n, 5);
+  if (n < 1 || n > (last ? 12 : 11)) return 0;
+  if (n <= 4) return 1 << n;
+  if (n <= 6 && !last) return 1 << (n - 2);
+  return 16;
+}
+
+} // namespace
+
+int twide_code(Stage const &st, int dtype) {
+  int const r = st.tma ? twide_chunk(st.job, dtype) : 0;
+  if (r == 0) return 0;
+  int const log2G = st.job.log2_n - (31 - __builtin_clz(r));
+  // Inner extent in floats (see twide_job).
+  int const inner = st.job.log2_inner + (dtype == PALIWA_GB_F64 ? 1 : 0);
+  if (r == 32)
+    return inner == 1 ? kTWide32Pairs
+           : log2G >= 3 ? kTWide32Chunked : kTWide32Dense;
+  bool const last = inner == 0 && st.job.log2_kstride == 0;
+  return r + (last         ? (log2G > 5 ? kTWideLongContig : kTWideContig)
+              : inner == 1 ? kTWidePairs
+              : log2G > 5  ? kTWideLong
+              : log2G >= 3 ? kTWideChunked : 0);
+}
+
+// Measured per launch, replayed from a graph (us, against the stage's own
+// kernel): FP32 n = 16 at 2^12 points 3.6 against 3.1, at 2^14 3.8 against
+// 4.1; FP32c 4.6 against 3.4 and 4.8 against 6.1; FP64 at 2^10 7.5 against
+// 6.5, at 2^12 7.9 against 7.6 and at 2^14 7.8 against 22.4 (few threads of
+// the FP64 pipe); chunked and long forms win from their smallest launches
+// (FP32 n = 128 at 2^12 4.1 against 6.7).
+bool twide_enough(int code, int dtype, long long points) {
+  bool const longer =
+      code == kTWide32Chunked || code == kTWideChunked + 16 ||
+      code == kTWideLong + 16 || code == kTWideLongContig + 16;
+  return longer || points >= (dtype == PALIWA_GB_F64 ? 1LL << 12 : 1LL << 13);
+}
+
+// Up to 4 chunks per pencil (dense): the 3D view [outer][n][inner] of the
+// stage's pencils with the axis' strides and boxes {Bx, n, Sx}. 8 chunks and
+// more (chunk-interleaved): the 5D view [outer][inner / X][row of chunk]
+// [chunk][X columns] and one box per tile, so that shared memory holds the
+// tile as [column group][row of chunk][chunk][X columns]. The last axis and
+// inner extents of 2 floats: rows of 128 bytes.
+bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap &map,
+               long long &tiles) {
+  auto encode = tensor_map_encoder();
+  LiftJob lj = st.job;
+  int const r = twide_chunk(lj, dtype);
+  if (encode == nullptr || r == 0 || lj.periodic != 1 || lj.base % 16 != 0)
+    return false;
+  // A double column is two float columns: the grid is viewed as floats with
+  // twice the inner extent (every copy moves 4-byte words).
+  if (dtype == PALIWA_GB_F64) {
+    ++lj.log2_inner;
+    ++lj.log2_kstride;
+    ++lj.log2_astride;
+    lj.columns *= 2;
+  }
+  int const log2r = 31 - __builtin_clz(static_cast<unsigned>(r));
+  int const log2G = lj.log2_n - log2r;
+  int const threads = twide_threads(r);
+  int const log2nt = 31 - __builtin_clz(static_cast<unsigned>(threads));
+  bool const last = lj.log2_inner == 0 && lj.log2_kstride == 0;
+  bool const pairs = lj.log2_inner == 1 && lj.log2_kstride == 1 &&
+                     lj.log2_astride == lj.log2_n + 1;
+  if (last || pairs) {
+    // The last axis (contiguous layout), or a strided axis of inner extent
+    // 2 whose pencil pairs lie one after another (pairs layout): the
+    // stage's points as rows of 32 floats (128 bytes), boxes of the unit's
+    // rows, 128-byte swizzle; units of 2 threads r floats (whole pencils).
+    if (r < 4 || log2G < 0 ||
+        log2G > (pairs ? (r == 32 ? 5 : 2) : 5 + 3 * (r == 16)))
+      return false;
+    long long const points = lj.columns << lj.log2_n;
+    int const log2unit = 1 + log2nt + log2r;
+    int const log2u = r >= 8 ? 0 : 3 - log2r;  // units per tile
+    if (points % 32 != 0 || (points >> (log2unit + log2u)) >= (1LL << 30))
+      return false;
+    tiles = (points + (1LL << (log2unit + log2u)) - 1) >> (log2unit + log2u);
+    std::memset(&job, 0, sizeof(job));
+    job.log2_n = lj.log2_n;
+    job.nlevels = lj.nlevels;
+    job.chunked = pairs ? 3 : 2;
+    job.nxb = 1;
+    job.log2_bx = log2unit - lj.log2_n;  // box bytes = the unit
+    job.log2_sx = 0;
+    cuuint64_t dims[2] = {32, static_cast<cuuint64_t>(points / 32)};
+    cuuint64_t strides[1] = {128};
+    cuuint32_t box[2] = {32, 1u << (log2unit - 5)};
+    cuuint32_t elem[2] = {1, 1};
+    CUresult const res = encode(
+        &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+        reinterpret_cast<void *>(lj.base), dims, strides, box, elem,
+        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return res == CUDA_SUCCESS;
+  }
+  if (lj.log2_inner < 2 || log2G < 0 || log2G > 7 || lj.log2_n > 11 ||
+      (log2G > 2 && r < 16) || (r == 32 && log2G > 5))
+    return false;
+  int const log2ct = log2nt + 1 - log2G;
+  // Units per tile: TWideShape<R>::kUnits (16 KB tiles for chunks of up to
+  // 8 points).
+  int const log2u = r >= 8 ? 0 : 3 - log2r;
+  std::memset(&job, 0, sizeof(job));
+  job.log2_n = lj.log2_n;
+  job.log2_inner = lj.log2_inner;
+  job.nlevels = lj.nlevels;
+  job.log2_bx = std::min(std::min(lj.log2_inner, log2ct), 8);
+  job.log2_sx = std::max(0, log2ct - lj.log2_inner);
+  job.nxb = 1 << (log2ct - job.log2_bx - job.log2_sx);
+  job.log2_rs = job.log2_bx;
+  tiles = (lj.columns + (1LL << (log2ct + log2u)) - 1) >> (log2ct + log2u);
+  if (tiles >= (1LL << 30)) return false;
+  long long const outer = lj.columns >> lj.log2_inner;
+  if (log2G >= 3) {
+    job.chunked = 1;
+    job.nxb = 1;
+    job.log2_bx = std::min(lj.log2_inner, log2ct);  // Bx >= 4: log2ct <= 6
+    job.log2_sx = log2ct - job.log2_bx;
+    // Groups of X columns: 4 (16 bytes, the least a box row may be), 8 or 16
+    // where the tile and the inner extent hold them. Wider rows are fewer for
+    // the tensor memory accelerator, but the chunks a warp reads together lie
+    // X columns apart, on fewer banks. 8 for up to 32 chunks (the chunked
+    // form 3.9 against 3.5 TB/s on the 4D batch; the long form is slower with
+    // them); 16 for up to 16 chunks of plain floats, whose arithmetic is cheap
+    // (n = 128 6.0 against 5.5 TB/s, n = 256 6.1 against 5.5), and for FP32c
+    // where the pencils span 256 MB or more: every box row is then a page of
+    // its own, at 8 clocks each (n = 128 4.75 against 3.25, n = 256 3.97
+    // against 3.53 and less; below that span 4.77 against 4.84 and 3.97
+    // against 4.45).
+    bool const spread =
+        lj.log2_n + lj.log2_kstride + 2 >= 28 || dtype == PALIWA_GB_F32;
+    int const xmax = log2G > 5 ? 2 : log2G <= 4 && r == 16 && spread ? 4 : 3;
+    int const xlo = std::max(2, std::min({xmax, log2ct, lj.log2_inner}));
+    job.log2_xlo = xlo;
+    job.log2_rs = log2G + xlo;
+    cuuint64_t dims[5] = {1u << xlo, static_cast<cuuint64_t>(1) << log2G,
+                          static_cast<cuuint64_t>(r),
+                          static_cast<cuuint64_t>(1) << (lj.log2_inner - xlo),
+                          static_cast<cuuint64_t>(outer)};
+    cuuint64_t strides[4] = {
+        static_cast<cuuint64_t>(4 * r) << lj.log2_kstride,
+        static_cast<cuuint64_t>(4) << lj.log2_kstride,
+        static_cast<cuuint64_t>(4) << xlo,
+        static_cast<cuuint64_t>(4) << lj.log2_astride};
+    cuuint32_t box[5] = {1u << xlo, 1u << log2G, static_cast<cuuint32_t>(r),
+                         1u << (job.log2_bx - xlo), 1u << job.log2_sx};
+    cuuint32_t elem[5] = {1, 1, 1, 1, 1};
+    CUresult const res = encode(
+        &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5,
+        reinterpret_cast<void *>(lj.base), dims, strides, box, elem,
+        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return res == CUDA_SUCCESS;
+  }
+  cuuint64_t dims[3] = {static_cast<cuuint64_t>(1) << lj.log2_inner,
+                        static_cast<cuuint64_t>(1) << lj.log2_n,
+                        static_cast<cuuint64_t>(outer)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(4) << lj.log2_kstride,
+                           static_cast<cuuint64_t>(4) << lj.log2_astride};
+  cuuint32_t box[3] = {1u << job.log2_bx, 1u << lj.log2_n,
+                       1u << job.log2_sx};
+  // An outer index's n rows of `inner` columns are one contiguous block
+  // when the pencil stride is the inner extent (no sub-lattice). When a
+  // tile holds whole blocks (inner < Ct) and a block fits one box
+  // dimension, the map takes the block as its rows: box rows of n inner
+  // floats instead of inner (fewer, longer rows for the tensor memory
+  // accelerator), the same bytes in the same shared-memory order, the same
+  // box coordinates (x = y = 0).
+  if (lj.log2_kstride == lj.log2_inner && lj.log2_inner < log2ct &&
+      lj.log2_n + lj.log2_inner <= 8) {
+    int const log2blk = lj.log2_n + lj.log2_inner;
+    dims[0] = static_cast<cuuint64_t>(1) << log2blk;
+    dims[1] = 1;
+    strides[0] = static_cast<cuuint64_t>(4) << log2blk;
+    box[0] = 1u << log2blk;
+    box[1] = 1;
+  }
+  cuuint32_t elem[3] = {1, 1, 1};
+  CUresult const res = encode(
+      &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
+      reinterpret_cast<void *>(lj.base), dims, strides, box, elem,
+      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return res == CUDA_SUCCESS;
+}
+
+void launch_twide(int dtype, int sched, int code, TWideParams const &p,
+                  cudaStream_t s) {
+  switch (dtype) {
+  case PALIWA_GB_F64: return launch_twide_f64(sched, code, p, s);
+  case PALIWA_GB_F32: return launch_twide_f32(sched, code, p, s);
+  case PALIWA_GB_F32C: return launch_twide_f32c(sched, code, p, s);
+  }
+  throw StatusError(PALIWA_GB_INVALID_ARGUMENT, "unknown dtype");
+}
+
+namespace {
+
+// The error word of the single-grid launches' bounded waits: one mapped,
+// portable host word, so that the host reads it without a copy and every
+// device can set it. Allocated by the first such launch (also inside a
+// stream capture: the allocation is not part of the captured work).
+std::atomic<unsigned *> g_error_word{nullptr};
+
+unsigned *stage_error_word() {
+  unsigned *word = g_error_word.load(std::memory_order_acquire);
+  if (word != nullptr) return word;
+  static std::mutex mutex;
+  std::lock_guard<std::mutex> lock(mutex);
+  word = g_error_word.load(std::memory_order_acquire);
+  if (word != nullptr) return word;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cuda_check(cudaThreadExchangeStreamCaptureMode(&mode),
+             "cudaThreadExchangeStreamCaptureMode");
+  void *p = nullptr;
+  cudaError_t const e = cudaHostAlloc(
+      &p, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  cuda_check(e, "cudaHostAlloc(error word)");
+  word = static_cast<unsigned *>(p);
+  *static_cast<unsigned volatile *>(word) = 0;
+  g_error_word.store(word, std::memory_order_release);
+  return word;
+}
+
+} // namespace
+
+void check_stage_errors() {
+  unsigned volatile *const word = g_error_word.load(std::memory_order_acquire);
+  if (word == nullptr || *word == 0) return;
+  *word = 0;
+  throw StatusError(PALIWA_GB_TIMEOUT,
+                    "a bounded wait of an earlier transform's tile copies "
+                    "gave up");
+}
+
+void launch_stage(int dtype, bool exact, bool symmetric, int ws,
+                  LiftParams const &params, Stage const &st, cudaStream_t s) {
+  int const sched =
+      ws >= 0 && canonical_shifts(st.job, (ws & 1) != 0) ? ws : -1;
+  if (st.tma && sched >= 0) {
+    TWideParams p;
+    std::memset(&p, 0, sizeof(p));
+    int const code = twide_code(st, dtype);
+    if (code != 0 && twide_enough(code, dtype, stage_points(st)) &&
+        twide_job(st, dtype, p.job, p.map, p.total_tiles)) {
+      check_stage_errors();
+      p.error = stage_error_word();
+      return launch_twide(dtype, sched, code, p, s);
+    }
+  }
+  LiftParams p = params;
+  p.job = st.job;
+  launch_lift(dtype, exact, symmetric, sched, st.R, p, nullptr, 1, st.tiles,
+              s);
+}
+
+} // namespace pgb

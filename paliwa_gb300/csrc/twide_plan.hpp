@@ -1,0 +1,54 @@
+// Host side of the TMA wide kernel (twide.cuh): which stages it takes, their
+// jobs and tensor maps, and its launches.
+#pragma once
+
+#include <cudaTypedefs.h>
+
+#include "plan.hpp"
+#include "twide.cuh"
+
+namespace pgb {
+
+// Launch codes kTWide + a form code (twide_code).
+constexpr int kTWide = 2048;
+
+// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
+// against libcuda); nullptr where the driver lacks it.
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
+
+// The form code of the TMA wide launch that takes a stage planned on it
+// (Stage::tma): the chunk size plus the form's offset, or kTWide32*; 0 for
+// the other stages.
+int twide_code(Stage const &st, int dtype);
+
+// The stage's job, tensor map and tiles. False when it does not qualify
+// (alignment, 2^30 tiles or more, or the encoder refuses the map); the stage
+// then runs on its own kernel (Stage::R).
+bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap &map,
+               long long &tiles);
+
+// Whether a launch of form `code` over `points` points in all is worth its
+// start-up (mbarriers, the tensor map's first fetch).
+bool twide_enough(int code, int dtype, long long points);
+
+// sched = 2 * wavelet + (forward ? 1 : 0); code as from twide_code.
+void launch_twide(int dtype, int sched, int code, TWideParams const &p,
+                  cudaStream_t s);
+void launch_twide_f32(int sched, int code, TWideParams const &p,
+                      cudaStream_t s);
+void launch_twide_f32c(int sched, int code, TWideParams const &p,
+                       cudaStream_t s);
+void launch_twide_f64(int sched, int code, TWideParams const &p,
+                      cudaStream_t s);
+
+// Launches one stage of a single grid: on the TMA wide kernel when it is
+// planned on it and qualifies, else on its own kernel. ws is the filters'
+// wavelet schedule (or -1).
+void launch_stage(int dtype, bool exact, bool symmetric, int ws,
+                  LiftParams const &params, Stage const &st, cudaStream_t s);
+
+// Throws PALIWA_GB_TIMEOUT (and clears the flag) when a bounded wait of a
+// single-grid launch gave up since the last call.
+void check_stage_errors();
+
+} // namespace pgb

@@ -79,10 +79,15 @@ TWIDE_LONG = 64
 TWIDE_CONTIG = 96
 TWIDE_PAIRS = 128
 TWIDE_LONG_CONTIG = 160
+# Chunks of 32 points (FP64): their own codes per form.
+TWIDE_32 = {224: "twide_kernel R=32", 225: "twide_kernel chunked R=32",
+            226: "twide_kernel inner 2 R=32"}
 
 
 def kernel_name(code):
     """Name of the lifting kernel behind a launch code of Batch.profile."""
+    if code - TWIDE_KERNEL in TWIDE_32:
+        return TWIDE_32[code - TWIDE_KERNEL]
     if code > TWIDE_KERNEL + TWIDE_LONG_CONTIG:
         return ("twide_kernel long last axis "
                 f"R={code - TWIDE_KERNEL - TWIDE_LONG_CONTIG}")
@@ -171,10 +176,9 @@ class Batch:
         _lib.check(self._lib.paliwa_gb_batch_use_slabs(self._h, int(enable)))
 
     def use_tma(self, enable):
-        """Run FP32c strided stages of up to 16 chunks per pencil on the TMA
-        wide kernel where the plan chose it (default), or on the wide and
-        tile kernels' per-thread copies (the same bits). Synchronizes the
-        device."""
+        """Run stages on the TMA wide kernel where the plan chose it
+        (default), or on the per-thread-copy kernels (the same bits).
+        Synchronizes the device."""
         _lib.check(self._lib.paliwa_gb_batch_use_tma(self._h, int(enable)))
 
     def set_ctas_per_sm(self, ctas):

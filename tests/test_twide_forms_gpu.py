@@ -1,0 +1,69 @@
+"""Single grids on the TMA wide kernel at the edges of its forms, bit for bit
+against the oracle (FP64, FP32) and the compensated model: every pencil length
+it takes along strided axes of several inner extents and the last axis, fewer
+columns than a tile holds, partial last tiles, and grids that start on no
+16-byte boundary (which keep the per-thread-copy kernels)."""
+import numpy as np
+import pytest
+
+import paliwa_gb300 as pg
+
+pytestmark = pytest.mark.gpu
+
+WAVELETS = ["hat", "biorthogonal", "fullweighting"]
+
+
+def want(x, level, lmin, wavelet, forward, mode):
+    import oracle as O
+    from compensated import hierarchize as model
+    if mode == "f32c":
+        return model(x, level, lmin, wavelet, forward)
+    f = O.hierarchize if forward else O.dehierarchize
+    return f(x.copy(), level, lmin, level, wavelet)
+
+
+@pytest.mark.parametrize("mode", ["f64", "f32", "f32c"])
+@pytest.mark.parametrize("log2_n", range(1, 13))
+def test_every_pencil_length_and_inner_extent(mode, log2_n):
+    import torch
+    rng = np.random.default_rng(log2_n)
+    dtype = np.float64 if mode == "f64" else np.float32
+    wavelet = WAVELETS[log2_n % 3]
+    for inner in (0, 1, 2, 3, 4, 6, 9):
+        for outer in (0, 1, 3, 5):
+            if outer + inner + log2_n > 18 or (outer > 3 and inner > 4):
+                continue
+            level, lmin = (outer, log2_n, inner), (outer, 0, inner)
+            n = 1 << sum(level)
+            x = rng.uniform(-1, 1, [1 << l for l in level]).astype(dtype)
+            for offset in (0, 1) if inner in (0, 2) else (0,):
+                buf = torch.empty(n + 1, device="cuda",
+                                  dtype=getattr(torch, x.dtype.name))
+                g = buf[offset:offset + n]
+                for forward in (True, False):
+                    g.copy_(torch.from_numpy(x.reshape(-1)))
+                    f = pg.hierarchize if forward else pg.dehierarchize
+                    f(g, level, lmin, level, wavelet,
+                      compensated=mode == "f32c")
+                    torch.cuda.synchronize()
+                    got = g.cpu().numpy().reshape(x.shape)
+                    exp = want(x, level, lmin, wavelet, forward, mode)
+                    assert np.array_equal(got, exp), (level, offset, forward)
+
+
+@pytest.mark.parametrize("mode", ["f64", "f32", "f32c"])
+def test_more_tiles_than_resident_ctas(mode):
+    """Enough tiles that every CTA's buffers cycle several times."""
+    import torch
+    rng = np.random.default_rng(3)
+    dtype = np.float64 if mode == "f64" else np.float32
+    for level in ((9, 5, 10), (12, 6, 5), (13, 10), (4, 10, 10)):
+        dim = 1
+        lmin = tuple(0 if d == dim else l for d, l in enumerate(level))
+        x = rng.uniform(-1, 1, [1 << l for l in level]).astype(dtype)
+        g = torch.from_numpy(x).cuda()
+        pg.hierarchize(g, level, lmin, level, "biorthogonal",
+                       compensated=mode == "f32c")
+        torch.cuda.synchronize()
+        exp = want(x, level, lmin, "biorthogonal", True, mode)
+        assert np.array_equal(g.cpu().numpy(), exp), level
