@@ -249,11 +249,12 @@ int paliwa_gb_batch_use_graphs(paliwa_gb_batch *batch, int enable);
  * reference (its CT driver spreads grids over execution-space instances,
  * test/test_paliwa_combination_technique.cpp:164-174). */
 int paliwa_gb_batch_set_groups(paliwa_gb_batch *batch, int ngroups);
-/* enable != 0 (default): grids whose trailing axes span blocks ("slabs") of
- * at most 32 KB, with levels to transform along two or more of those axes,
- * transform all of them in one launch of the slab kernel (one HBM pass over
- * the grid, tiles moved by the tensor memory accelerator); 0 plans every
- * axis on its own. Results are the same bits either way. Re-plans both
+/* enable != 0: grids whose trailing axes span blocks ("slabs") of at most
+ * 32 KB, with levels to transform along two or more of those axes, transform
+ * all of them in one launch of the slab kernel (one HBM pass over the grid,
+ * tiles moved by the tensor memory accelerator); 0 plans every axis on its
+ * own. A new batch takes the faster way for its type and size (slabs for FP32
+ * and for small batches). Results are the same bits either way. Re-plans both
  * directions after synchronizing the device. No counterpart in the
  * reference. */
 int paliwa_gb_batch_use_slabs(paliwa_gb_batch *batch, int enable);

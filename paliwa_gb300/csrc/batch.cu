@@ -71,8 +71,8 @@ struct Direction {
   CUtensorMap *maps_dev = nullptr;
   cudaGraphExec_t graph = nullptr;
   Tuning tuning;  // kernel forced per class (autotuner)
-  // Slab launches where they apply (the batch's setting); the autotuner
-  // clears it when the direction runs faster axis by axis.
+  // Slab launches where they apply (default_slabs, or the batch's setting);
+  // the autotuner takes the other choice when the direction runs faster so.
   bool slabs = true;
   // TMA wide launches for the stages planned on them (the batch's setting).
   bool tma = true;
@@ -168,6 +168,24 @@ struct paliwa_gb_batch {
 };
 
 namespace {
+
+// Whether a new batch plans slabs. They save launches, which is what small
+// batches spend their time on (FP32c 6D |l|_1 = 12 - q, 2.6 M points: 134
+// against 247 us there and back; FP64 165 against 300), but their axes are
+// bound by barriers and latencies at about half the TMA wide kernel's rate
+// for double and double-float arithmetic: FP32c from about 2^25 points on
+// (6D 14 - q, 30 M points: 592 against 744 us; 4D 16 - q, 48 M: 1059 against
+// 1068; 5D 16 - q, 139 M: 2288 against 2051; 4D 20 - q: 23.1 against 19.9 ms)
+// and FP64 from about 2^22 (4D 14 - q, 7.4 M: 602 against 518) are faster
+// axis by axis. Plain FP32 is bound by memory either way and takes slabs
+// throughout (5D 16 - q 1532 against 1685; 4D 18 - q 3105 against 3102).
+bool default_slabs(int dtype, long long points) {
+  switch (dtype) {
+  case PALIWA_GB_F64: return points <= 1LL << 22;
+  case PALIWA_GB_F32C: return points <= 1LL << 25;
+  }
+  return true;
+}
 
 // The slab group of grid g: its trailing axes whose slab (the product of
 // their extents) fits one tile, when that group holds at least two axes
@@ -1083,6 +1101,7 @@ int paliwa_gb_batch_create(int ndim, int ngrids, const int64_t *levels,
       for (int d = 0; d < ndim; ++d) total += levels[g * ndim + d];
       b->points += 1LL << total;
     }
+    for (Direction &dr : b->dir) dr.slabs = default_slabs(dtype, b->points);
     try {
       cuda_check(cudaMalloc(&b->slab_error, sizeof(unsigned)),
                  "cudaMalloc(error word)");
@@ -1142,6 +1161,7 @@ int paliwa_gb_batch_use_slabs(paliwa_gb_batch *batch, int enable) {
       throw StatusError(PALIWA_GB_INVALID_ARGUMENT, "null batch");
     cuda_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
     batch->use_slabs = enable != 0;
+    for (Direction &dr : batch->dir) dr.slabs = batch->use_slabs;
     setup_groups(*batch, batch->ngroups);
   });
 }

@@ -171,8 +171,9 @@ class Batch:
 
     def use_slabs(self, enable):
         """Plan the trailing axes of grids whose slabs fit a tile as one
-        slab launch (default), or every axis on its own (the same bits).
-        Synchronizes the device."""
+        slab launch, or every axis on its own (the same bits; a new batch
+        takes the faster way for its type and size). Synchronizes the
+        device."""
         _lib.check(self._lib.paliwa_gb_batch_use_slabs(self._h, int(enable)))
 
     def use_tma(self, enable):
