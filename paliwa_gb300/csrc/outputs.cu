@@ -18,9 +18,11 @@
 // front 0 and 2^level points; a window may wrap around the period, so one
 // buffer holds a slab and the periodic halo it needs (what the reference
 // keeps in separate local and remote storage).
+#include <algorithm>
 #include <cstdint>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "arith.cuh"
@@ -90,6 +92,118 @@ __global__ void __launch_bounds__(kOutThreads) out_pass_kernel(OutPass const p) 
   }
 }
 
+// The whole pass list in one launch. A CTA holds the touched stretch of the
+// axis (extent points from buffer index k0 on) of 2^log2cols columns in shared
+// memory, runs every pass there and writes the written points back, so each
+// point is read and written once instead of once per pass, and the passes are
+// separated by CTA barriers instead of launches. (The launches were the cost:
+// a slab of 160 x 256 x 128 doubles, 8 passes, 71 us with one launch each.)
+struct OutList {
+  static constexpr int kMaxPass = 48;
+  static constexpr int kMaxFilters = 8;
+  // Uids (the period is at most 2^30): 32 bits hold them and their sums.
+  struct Run {
+    unsigned first, step, s;  // written uids, neighbour distance
+    int count;
+    int filter;
+  };
+  int npasses;
+  int k0, extent;
+  int log2cols;
+  int pitch;           // columns apart (along the axis), or rows apart
+  long long columns;   // columns in all
+  unsigned c1_one_mask;  // filters whose middle coefficient is 1
+  Run run[kMaxPass];
+  Coeffs c[kMaxFilters];
+};
+
+// Element (k, w) of the tile: rows of columns, or, where the axis is the
+// contiguous one (Along), a pencil per column at an odd pitch; threads walk
+// the columns first in every pass (distinct banks either way).
+template <typename T, bool Exact, bool Along>
+__global__ void __launch_bounds__(kOutThreads)
+    out_list_kernel(__grid_constant__ const OutPass p,
+                    __grid_constant__ const OutList q) {
+  using A = Plain<T, Exact>;
+  extern __shared__ __align__(16) unsigned char smem[];
+  T *const tile = reinterpret_cast<T *>(smem);
+  int const cols = 1 << q.log2cols;
+  long long *const coloff = reinterpret_cast<long long *>(
+      smem + ((size_t(q.pitch) * (Along ? cols : q.extent) * sizeof(T) + 15) &
+              ~size_t(15)));
+  unsigned char *const written =
+      reinterpret_cast<unsigned char *>(coloff + cols);
+  int const t = threadIdx.x;
+  T *const g = reinterpret_cast<T *>(p.base);
+  long long const es = p.elem[p.dim];
+  long long const first = static_cast<long long>(blockIdx.x) << q.log2cols;
+  int const ncols = static_cast<int>(
+      q.columns - first < cols ? q.columns - first : cols);
+  for (int w = t; w < ncols; w += kOutThreads) {
+    unsigned long long r = static_cast<unsigned long long>(first + w);
+    long long off = 0;
+    for (int d = p.ndim - 1; d >= 0; --d) {
+      if (d == p.dim) continue;
+      unsigned long long const e = static_cast<unsigned long long>(p.oext[d]);
+      off += (p.obase[d] + static_cast<long long>(r % e) * p.ostep[d]) *
+             p.elem[d];
+      r /= e;
+    }
+    coloff[w] = off;
+  }
+  for (int k = t; k < q.extent; k += kOutThreads) written[k] = 0;
+  __syncthreads();
+  auto at = [&](int k, int w) -> T & {
+    return tile[Along ? w * q.pitch + k : k * q.pitch + w];
+  };
+  // Lanes along the columns, or along the contiguous axis.
+  auto each = [&](auto f) {
+    if (Along) {
+      for (int w = t >> 5; w < ncols; w += kOutThreads / 32)
+        for (int k = t & 31; k < q.extent; k += 32) f(k, w);
+    } else {
+      int const w = t & (cols - 1);
+      if (w < ncols)
+        for (int k = t >> q.log2cols; k < q.extent;
+             k += kOutThreads >> q.log2cols)
+          f(k, w);
+    }
+  };
+  each([&](int k, int w) { at(k, w) = g[coloff[w] + (q.k0 + k) * es]; });
+  __syncthreads();
+  unsigned const m = static_cast<unsigned>(p.period - 1);
+  unsigned const front = static_cast<unsigned>(p.wfront);
+  int const w = t & (cols - 1);
+  auto pass = [&](OutList::Run const &run, auto c1one) {
+    Coeffs const &c = q.c[run.filter];
+    for (int j = t >> q.log2cols; j < run.count;
+         j += kOutThreads >> q.log2cols) {
+      unsigned const x = run.first + j * run.step - front;
+      auto index = [&](unsigned u) {
+        return static_cast<int>((u & m) >> p.log2_spacing) - q.k0;
+      };
+      int const ix = index(x);
+      at(ix, w) = A::template update<decltype(c1one)::value>(
+          c, at(index(x - run.s), w), at(ix, w), at(index(x + run.s), w));
+      if (w == 0) written[ix] = 1;
+    }
+  };
+  for (int i = 0; i < q.npasses; ++i) {
+    OutList::Run const &run = q.run[i];
+    // A product by 1 is exact: leaving it out changes no bits.
+    if (w < ncols) {
+      if ((q.c1_one_mask >> run.filter) & 1u)
+        pass(run, std::true_type{});
+      else
+        pass(run, std::false_type{});
+    }
+    __syncthreads();
+  }
+  each([&](int k, int w) {
+    if (written[k]) g[coloff[w] + (q.k0 + k) * es] = at(k, w);
+  });
+}
+
 int device_sm_count() {
   int dev = 0, sms = 0;
   cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
@@ -124,6 +238,112 @@ void launch_out_pass(int dtype, bool exact, OutPass const &p, cudaStream_t s) {
       out_pass_kernel<float, false><<<blocks, kOutThreads, 0, s>>>(p);
   }
   cuda_check(cudaGetLastError(), "out_pass_kernel launch");
+}
+
+// Shared memory an out_list_kernel CTA may take (two fit an SM).
+constexpr size_t kOutSmem = 100 << 10;
+
+// The passes of one call in their order (the written run of each in p.first,
+// p.step, p.count, p.s and p.c).
+struct OutCall {
+  std::vector<OutPass> passes;
+  std::vector<int> filter;  // the filter of each
+
+  void add(OutPass const &p, int f) {
+    passes.push_back(p);
+    filter.push_back(f);
+  }
+};
+
+template <typename T, bool Exact, bool Along>
+void launch_out_list(OutPass const &p, OutList const &q, size_t smem,
+                     cudaStream_t s) {
+  auto const kernel = out_list_kernel<T, Exact, Along>;
+  cuda_check(cudaFuncSetAttribute(kernel,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(kOutSmem)),
+             "cudaFuncSetAttribute(out list)");
+  unsigned const blocks = static_cast<unsigned>(
+      (q.columns + (1LL << q.log2cols) - 1) >> q.log2cols);
+  kernel<<<blocks, kOutThreads, smem, s>>>(p, q);
+  cuda_check(cudaGetLastError(), "out_list_kernel launch");
+}
+
+// One launch for the whole list when the touched stretch of the axis fits
+// shared memory with 4 columns or more (up to 32: whole 128-byte lines of
+// floats; fewer when that leaves under two CTAs per SM), else one launch per
+// pass.
+void launch_out_call(int dtype, bool exact, OutCall const &call,
+                     long long columns, long long window_extent,
+                     cudaStream_t s) {
+  if (call.passes.empty()) return;
+  auto one_by_one = [&] {
+    for (auto const &p : call.passes) launch_out_pass(dtype, exact, p, s);
+  };
+  size_t const n = call.passes.size();
+  int const nf = *std::max_element(call.filter.begin(), call.filter.end()) + 1;
+  if (n == 1 || n > OutList::kMaxPass || nf > OutList::kMaxFilters)
+    return one_by_one();
+  OutPass const &p = call.passes[0];
+  OutList q{};
+  q.npasses = static_cast<int>(n);
+  q.columns = columns;
+  // The touched buffer indices: the written run and its outer neighbours
+  // where they follow each other in the buffer, else the whole window.
+  auto index = [&](long long u) {
+    return ((u - p.wfront) & (p.period - 1)) >> p.log2_spacing;
+  };
+  long long lo = window_extent, hi = -1;
+  for (size_t i = 0; i < n; ++i) {
+    OutPass const &r = call.passes[i];
+    long long const last = r.first + (r.count - 1) * r.step;
+    long long const a = index(r.first - r.s), b = index(r.first);
+    long long const c = index(last), d = index(last + r.s);
+    if (a < b && c < d && c - b == (last - r.first) >> p.log2_spacing) {
+      lo = std::min(lo, a);
+      hi = std::max(hi, d);
+    } else {
+      lo = 0;
+      hi = window_extent - 1;
+    }
+    if (r.count > 0x7fffffff) return one_by_one();
+    q.run[i] = {static_cast<unsigned>(r.first), static_cast<unsigned>(r.step),
+                static_cast<unsigned>(r.s), static_cast<int>(r.count),
+                call.filter[i]};
+    q.c[call.filter[i]] = r.c;
+    if (r.c.c1 == 1.0) q.c1_one_mask |= 1u << call.filter[i];
+  }
+  long long const extent = hi - lo + 1;
+  bool const along = p.elem[p.dim] == 1;
+  size_t const es = dtype_size(dtype);
+  int log2cols = 5;
+  auto smem_of = [&](int lc) {
+    size_t const pitch = along ? (extent | 1) : (1LL << lc);
+    return ((pitch * (along ? (1LL << lc) : extent) * es + 15) & ~size_t(15)) +
+           (size_t(8) << lc) + extent;
+  };
+  if (extent > (1 << 20) || columns > (1LL << 32)) return one_by_one();
+  while (log2cols > 2 && (smem_of(log2cols) > kOutSmem ||
+                          (columns >> log2cols) < 2 * 152))
+    --log2cols;
+  if (smem_of(log2cols) > kOutSmem) return one_by_one();
+  q.k0 = static_cast<int>(lo);
+  q.extent = static_cast<int>(extent);
+  q.log2cols = log2cols;
+  q.pitch = along ? static_cast<int>(extent | 1) : 1 << log2cols;
+  size_t const smem = smem_of(log2cols);
+  auto go = [&](auto value, auto ex) {
+    using T = decltype(value);
+    constexpr bool E = decltype(ex)::value;
+    if (along)
+      launch_out_list<T, E, true>(p, q, smem, s);
+    else
+      launch_out_list<T, E, false>(p, q, smem, s);
+  };
+  if (dtype == PALIWA_GB_F64)
+    exact ? go(double{}, std::true_type{}) : go(double{}, std::false_type{});
+  else
+    exact ? go(float{}, std::true_type{}) : go(float{}, std::false_type{});
 }
 
 long long floor_mod(long long x, long long m) {
@@ -334,6 +554,7 @@ int paliwa_gb_transform_outputs(
       return v;
     }());
     cudaStream_t const s = static_cast<cudaStream_t>(stream);
+    OutCall call;
     // Execute forwards (:310-329): per level and pass, the parity lattice
     // of that level restricted to the planned bounds, cut at the period.
     for (size_t i = 0; i < lv.size(); ++i) {
@@ -360,7 +581,7 @@ int paliwa_gb_transform_outputs(
           p.count = (upper - begin) / (2 * st) + 1;
           p.oext[dim] = p.count;
           p.total = p.count * others;
-          launch_out_pass(dtype, exact, p, s);
+          call.add(p, static_cast<int>(q));
         };
         if (w.min <= w.max) {
           run(w.min, w.max);
@@ -370,6 +591,7 @@ int paliwa_gb_transform_outputs(
         }
       }
     }
+    launch_out_call(dtype, exact, call, others, wext, s);
   });
 }
 
@@ -463,11 +685,13 @@ extern "C" int paliwa_gb_transform_in_window(
     // uid 0 (lower neighbour period - d) and uid period - d (upper
     // neighbour 0) when the window holds their wrapped neighbours; both sit
     // at the ends of that range, so every pass writes one run.
+    OutCall call;
     for (long l : lv) {
       long long const d = 1LL << (L - l);
       long long const step = 2 * d;
       p.s = d;
-      for (auto const &f : filters) {
+      for (size_t q = 0; q < filters.size(); ++q) {
+        auto const &f = filters[q];
         long long const off = f.first * d;  // the lattice {off + k step}
         auto up_to = [&](long long x) {      // largest lattice point <= x
           return x - floor_mod(x - off, step);
@@ -491,8 +715,9 @@ extern "C" int paliwa_gb_transform_in_window(
         double const *c = f.second.data();
         p.c = Coeffs{c[0], c[1], c[2], static_cast<float>(c[0]),
                      static_cast<float>(c[1]), static_cast<float>(c[2])};
-        launch_out_pass(dtype, exact, p, s);
+        call.add(p, static_cast<int>(q));
       }
     }
+    launch_out_call(dtype, exact, call, others, window_extents[dim], s);
   });
 }
