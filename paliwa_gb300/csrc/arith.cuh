@@ -336,9 +336,9 @@ struct RowF64 {
 };
 
 // Rows of 8 bytes, for the TMA wide kernel (twide.cuh): RowF32C above, two
-// columns of Plain<float, true> as one f32x2 pair, or one column of
-// Plain<double, true>.
-struct RowF32x2 {
+// columns of Plain<float, Exact> as one f32x2 pair, or one column of
+// Plain<double, Exact>.
+template <bool Exact> struct RowF32x2 {
   using V = f2;
   using Store = uint2;
   static constexpr bool kPacked = false;
@@ -351,10 +351,24 @@ struct RowF32x2 {
   template <bool C1>
   static __device__ __forceinline__ V update(Coeffs const &c, V lo, V me,
                                              V up) {
-    return RowF32::template pair<C1>(c, lo, me, up);
+    if constexpr (Exact) {
+      return RowF32::template pair<C1>(c, lo, me, up);
+    } else {
+      V const m = C1 ? me : product(c.f1, me);
+      V const t = f2_add(product(c.f0, lo), m);
+      return f2_add(t, product(c.f2, up));
+    }
+  }
+
+ private:
+  // c * x rounded by itself, as two scalar multiplies: a packed multiply (or
+  // a packed fma with -0) whose product feeds a packed add came out contracted
+  // into one fma.
+  static __device__ __forceinline__ f2 product(float c, f2 x) {
+    return f2_pack(__fmul_rn(c, f2_x(x)), __fmul_rn(c, f2_y(x)));
   }
 };
-struct ColF64 {
+template <bool Exact> struct ColF64 {
   using V = double;
   using Store = uint2;
   static constexpr bool kPacked = false;
@@ -368,7 +382,7 @@ struct ColF64 {
   template <bool C1>
   static __device__ __forceinline__ V update(Coeffs const &c, V lo, V me,
                                              V up) {
-    return Plain<double, true>::template update<C1>(c, lo, me, up);
+    return Plain<double, Exact>::template update<C1>(c, lo, me, up);
   }
 };
 

@@ -516,7 +516,7 @@ void launch_one(paliwa_gb_batch &b, Direction &dr, Launch const &L,
     p.total_tiles = L.tiles;
     p.error = b.slab_error;
     p.ctas_per_sm = b.ctas_per_sm;
-    launch_twide(b.dtype, L.sched, L.R - kTWide, p, s);
+    launch_twide(b.dtype, dr.exact, L.sched, L.R - kTWide, p, s);
     return;
   }
   if (L.R != kSlab) {

@@ -187,7 +187,7 @@ LiftJob make_job(AxisView const &v, std::vector<int> const &sh, size_t first,
 // pieces; the direct kernel pencils that one thread holds whole and
 // last-axis pencils of up to 32 chunks; the staged kernel everything with
 // chunks of 16 points.
-KernelSet periodic_kernels(AxisView const &v, bool canon) {
+KernelSet periodic_kernels(AxisView const &v, bool canon, bool ordered) {
   int const R = chunk_for(v.log2_n);
   int const log2G = v.log2_n - (31 - __builtin_clz(R));
   bool const aligned = canon && v.log2_row > 0;
@@ -206,7 +206,7 @@ KernelSet periodic_kernels(AxisView const &v, bool canon) {
       v.log2_inner + v.log2_es >=
           tile_piece_log2(log2G, v.log2_row + v.log2_es))
     k.mask |= 1 << kChooseTile;
-  // The TMA wide kernel: 16-byte aligned grids under a wavelet schedule.
+  // The TMA wide kernel: 16-byte aligned grids, levels in order.
   // Floats: strided pencils of up to 2048 points whose inner extent is 4 or
   // more columns, or 2 with the pencil pairs one after another (up to 64
   // points); the last axis' pencils of 4 to 4096 points. Doubles: pencils of
@@ -222,7 +222,9 @@ KernelSet periodic_kernels(AxisView const &v, bool canon) {
     tma = last ? v.log2_n >= 2 && v.log2_n <= 12
                : (v.log2_inner >= 2 && v.log2_n <= 11) ||
                      (pairs && v.log2_n >= 2 && v.log2_n <= 6);
-  if (tma && canon && v.base % 16 == 0 && v.columns < (1LL << 29))
+  // (FP32c takes the wavelet schedules only.)
+  if (tma && (canon || (ordered && !v.wide_last)) && v.base % 16 == 0 &&
+      v.columns < (1LL << 29))
     k.mask |= 1 << kChooseTmaWide;
   // Default: the wide kernel for strided pencils (and FP32c last-axis
   // pencils: measured on 2^26-point grids, 3.0-4.5 TB/s against 2.8-4.1 on
@@ -270,6 +272,10 @@ KernelSet periodic_kernels(AxisView const &v, bool canon) {
     if (last || pairs ||
         (v.log2_n >= 3 && v.log2_n <= longest && !pages))
       k.dflt = kChooseTmaWide;
+    // A caller's filters otherwise run on the staged or direct kernel, which
+    // read every step's distance, parity and coefficients (FP32 n = 512,
+    // 256 columns, four passes of CDF 9/7: 2830 against 1620 GB/s).
+    if (!canon && !pages) k.dflt = kChooseTmaWide;
   }
   return k;
 }
@@ -304,7 +310,9 @@ void plan_periodic(AxisView const &v, std::vector<int> const &shifts, int ws,
     st.job.periodic = 1;
     st.job.log2_window = v.log2_n;
     bool const canon = ws >= 0 && canonical_shifts(st.job, (ws & 1) != 0);
-    KernelSet const ks = periodic_kernels(v, canon);
+    bool const ordered = canonical_shifts(st.job, true) ||
+                         canonical_shifts(st.job, false);
+    KernelSet const ks = periodic_kernels(v, canon, ordered);
     st.tclass = tuning_class(v);
     st.kernels = ks.mask;
     st.dflt = ks.dflt;

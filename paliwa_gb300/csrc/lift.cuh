@@ -363,6 +363,76 @@ template <> struct WaveletPasses<2, false> {
   using type = PassList<Pass<1, 2, 4, 2, 4>, Pass<0, -2, 8, -2, 4>>;
 };
 
+// A caller's filters (transform_in), read per pass.
+struct FilterTable {
+  int npasses;
+  unsigned c1_one_mask;
+  int offsets[kMaxPasses];
+  Coeffs coeffs[kMaxPasses];
+};
+
+// Any filters over the contiguous level range of hierarchize_in (FWD) or
+// dehierarchize_in: the levels are unrolled with compile-time distances, as in
+// WaveletSched, and each pass takes its parity and coefficients from the
+// table (one uniform branch per pass).
+template <bool FWD> struct TableSched {
+  static constexpr bool kTable = true;
+
+  template <class A, int R, int K, class Ctx>
+  static __device__ __forceinline__ void fine_level(typename A::V (&v)[R],
+                                                    Ctx &ctx,
+                                                    FilterTable const &f) {
+    constexpr int S = 1 << K;
+    for (int ps = 0; ps < f.npasses; ++ps) {
+      int const o = f.offsets[ps];
+      typename A::V const pub = o == 1 ? v[0] : v[R - S];
+      typename A::V const nb = ctx.fine_neighbor(o, pub);
+      if ((f.c1_one_mask >> ps) & 1u)
+        fine_step<A, R, S, true>(v, o, nb, f.coeffs[ps]);
+      else
+        fine_step<A, R, S, false>(v, o, nb, f.coeffs[ps]);
+      ctx.fine_wrote_heads(o);
+    }
+  }
+  template <class A, int R, int K, class Ctx>
+  static __device__ __forceinline__ void fine(typename A::V (&v)[R], Ctx &ctx,
+                                              int L, FilterTable const &f) {
+    if constexpr (K >= 0 && (1 << K) < R) {
+      if (K < L) fine_level<A, R, K>(v, ctx, f);
+      fine<A, R, FWD ? K + 1 : K - 1>(v, ctx, L, f);
+    }
+  }
+  template <class A, int R, class Ctx>
+  static __device__ __forceinline__ void coarse(typename A::V (&v)[R],
+                                                Ctx &ctx, int L,
+                                                FilterTable const &f) {
+    constexpr int LOG2R = Log2<R>::value;
+    for (int i = LOG2R; i < L; ++i) {
+      int const sh = FWD ? i : LOG2R + L - 1 - i;
+      for (int ps = 0; ps < f.npasses; ++ps) {
+        Coeffs const &cf = f.coeffs[ps];
+        bool const c1one = (f.c1_one_mask >> ps) & 1u;
+        ctx.coarse(v[0], f.offsets[ps], 1 << (sh - LOG2R),
+                   [&](typename A::V lo, typename A::V me, typename A::V up) {
+                     return coarse_update<A>(cf, c1one, lo, me, up);
+                   });
+      }
+    }
+  }
+  template <class A, int R, int NT, class Ctx>
+  static __device__ __forceinline__ void run_levels(typename A::V (&v)[R],
+                                                    Ctx &ctx, int L,
+                                                    FilterTable const &f) {
+    if constexpr (FWD) {
+      fine<A, R, 0>(v, ctx, L, f);
+      coarse<A, R>(v, ctx, L, f);
+    } else {
+      coarse<A, R>(v, ctx, L, f);
+      fine<A, R, Log2<R>::value - 1>(v, ctx, L, f);
+    }
+  }
+};
+
 // Schedule of hierarchize (FWD: levels fine to coarse, distances 1, 2, 4, ...)
 // and dehierarchize (coarse to fine) with a compile-time wavelet: the fine
 // levels are unrolled with compile-time distance, parity and coefficients.
@@ -370,6 +440,7 @@ template <> struct WaveletPasses<2, false> {
 template <int W, bool FWD> struct WaveletSched {
   using Passes = typename WaveletPasses<W, FWD>::type;
   static constexpr bool kForward = FWD;
+  static constexpr bool kTable = false;
   static constexpr bool kSplit = true;  // fine_only / coarse_only below
 
   template <class A, int R, int NT, int K, class P, class Ctx>

@@ -122,7 +122,9 @@ struct KernelSet {
 struct Tuning {
   std::map<int, int> choice;  // tuning_class -> KernelChoice
 };
-KernelSet periodic_kernels(AxisView const &v, bool canonical);
+// canonical: a wavelet schedule's levels; ordered: the level range of
+// hierarchize_in or dehierarchize_in, with any filters.
+KernelSet periodic_kernels(AxisView const &v, bool canonical, bool ordered);
 int tuning_class(AxisView const &v);
 
 void plan_axis(AxisView const &view, std::vector<int> const &shifts,

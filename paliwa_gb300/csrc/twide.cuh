@@ -104,7 +104,19 @@ struct TWideParams {
   // jobs == nullptr: the launch's only job and its map.
   TWideJob job;
   CUtensorMap map;
+  FilterTable filters;  // read by TableSched launches
 };
+
+// The levels of one chunk under the launch's schedule.
+template <class Sched, class A, int R, int NT, class Ctx>
+__device__ __forceinline__ void twide_levels(typename A::V (&v)[R], Ctx &ctx,
+                                             int nlevels,
+                                             TWideParams const &p) {
+  if constexpr (Sched::kTable)
+    Sched::template run_levels<A, R, NT>(v, ctx, nlevels, p.filters);
+  else
+    Sched::template run_levels<A, R, NT>(v, ctx, nlevels);
+}
 
 __device__ __forceinline__ void tma_load_3d(void *dst, void const *map, int x,
                                             int y, int z, uint64_t *bar) {
@@ -444,7 +456,7 @@ __global__ void __launch_bounds__(twide_threads(R) + 32, R >= 16 ? 2 : 3)
             }
             RoundCtx<A, NT, true> ctx(t, c, 1 << log2G, log2G, lane, 1,
                                       nullptr, nullptr);
-            Sched::template run_levels<A, R, NT>(v, ctx, job.nlevels);
+            twide_levels<Sched, A, R, NT>(v, ctx, job.nlevels, p);
 #pragma unroll
             for (int i = 0; i < R / 2; ++i) {
               W const r0 = A::store(v[2 * i]);
@@ -475,7 +487,7 @@ __global__ void __launch_bounds__(twide_threads(R) + 32, R >= 16 ? 2 : 3)
           }
           RoundCtx<A, NT, true> ctx(t, c, 1 << log2G, log2G, lane, 1,
                                     nullptr, nullptr);
-          Sched::template run_levels<A, R, NT>(v, ctx, job.nlevels);
+          twide_levels<Sched, A, R, NT>(v, ctx, job.nlevels, p);
 #pragma unroll
           for (int i = 0; i < R / 4; ++i) {
             W const r0 = A::store(v[4 * i]);
@@ -528,7 +540,7 @@ __global__ void __launch_bounds__(twide_threads(R) + 32, R >= 16 ? 2 : 3)
               *reinterpret_cast<W const *>(tf + idx0 + (j << job.log2_rs)));
         RoundCtx<A, NT, true> ctx(t, c, G, log2G, lane, 1, nullptr, nullptr,
                                   log2ls);
-        Sched::template run_levels<A, R, NT>(v, ctx, job.nlevels);
+        twide_levels<Sched, A, R, NT>(v, ctx, job.nlevels, p);
 #pragma unroll
         for (int j = 0; j < R; ++j)
           *reinterpret_cast<W *>(tf + idx0 + (j << job.log2_rs)) =
@@ -689,7 +701,7 @@ __global__ void __launch_bounds__(kTWideThreads, 2)
           v[4 * i + 3] = A::load(W{f0.w, f1.w});
         }
         RoundCtx<A, NT, false, 256> ctx(t, c, G, log2G, lane, 1, heads, xch);
-        Sched::template run_levels<A, R, NT>(v, ctx, job.nlevels);
+        twide_levels<Sched, A, R, NT>(v, ctx, job.nlevels, p);
 #pragma unroll
         for (int i = 0; i < R / 4; ++i) {
           W const r0 = A::store(v[4 * i]);
@@ -720,7 +732,7 @@ __global__ void __launch_bounds__(kTWideThreads, 2)
         v[j] = A::load(
             *reinterpret_cast<W const *>(tf + idx0 + (j << job.log2_rs)));
       RoundCtx<A, NT, false, 128> ctx(t, c, G, log2G, lane, 1, heads, xch);
-      Sched::template run_levels<A, R, NT>(v, ctx, job.nlevels);
+      twide_levels<Sched, A, R, NT>(v, ctx, job.nlevels, p);
 #pragma unroll
       for (int j = 0; j < R; ++j)
         *reinterpret_cast<W *>(tf + idx0 + (j << job.log2_rs)) =

@@ -95,4 +95,11 @@ template <class F> void with_wavelet_sched(int sched, F &&f) {
   throw StatusError(2, "twide kernel planned without a wavelet schedule");
 }
 
+// Calls f with the schedule of a caller's filters.
+template <class F> void with_table_sched(int sched, F &&f) {
+  if (sched == kTableSched) return f(TableSched<false>{});
+  if (sched == kTableSched + 1) return f(TableSched<true>{});
+  throw StatusError(2, "bad table schedule");
+}
+
 } // namespace pgb

@@ -224,11 +224,16 @@ bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap &map,
   return res == CUDA_SUCCESS;
 }
 
-void launch_twide(int dtype, int sched, int code, TWideParams const &p,
-                  cudaStream_t s) {
+void launch_twide(int dtype, bool exact, int sched, int code,
+                  TWideParams const &p, cudaStream_t s) {
+  bool const table = sched >= kTableSched;
   switch (dtype) {
-  case PALIWA_GB_F64: return launch_twide_f64(sched, code, p, s);
-  case PALIWA_GB_F32: return launch_twide_f32(sched, code, p, s);
+  case PALIWA_GB_F64:
+    return table ? launch_twide_table_f64(exact, sched, code, p, s)
+                 : launch_twide_f64(sched, code, p, s);
+  case PALIWA_GB_F32:
+    return table ? launch_twide_table_f32(exact, sched, code, p, s)
+                 : launch_twide_f32(sched, code, p, s);
   case PALIWA_GB_F32C: return launch_twide_f32c(sched, code, p, s);
   }
   throw StatusError(PALIWA_GB_INVALID_ARGUMENT, "unknown dtype");
@@ -278,15 +283,23 @@ void launch_stage(int dtype, bool exact, bool symmetric, int ws,
                   LiftParams const &params, Stage const &st, cudaStream_t s) {
   int const sched =
       ws >= 0 && canonical_shifts(st.job, (ws & 1) != 0) ? ws : -1;
-  if (st.tma && sched >= 0) {
+  if (st.tma) {
     TWideParams p;
     std::memset(&p, 0, sizeof(p));
+    int tsched = sched;
+    if (sched < 0) {
+      tsched = kTableSched + (canonical_shifts(st.job, true) ? 1 : 0);
+      p.filters.npasses = params.npasses;
+      p.filters.c1_one_mask = params.c1_one_mask;
+      std::copy_n(params.offsets, kMaxPasses, p.filters.offsets);
+      std::copy_n(params.coeffs, kMaxPasses, p.filters.coeffs);
+    }
     int const code = twide_code(st, dtype);
     if (code != 0 && twide_enough(code, dtype, stage_points(st)) &&
         twide_job(st, dtype, p.job, p.map, p.total_tiles)) {
       check_stage_errors();
       p.error = stage_error_word();
-      return launch_twide(dtype, sched, code, p, s);
+      return launch_twide(dtype, exact, tsched, code, p, s);
     }
   }
   LiftParams p = params;

@@ -31,15 +31,25 @@ bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap &map,
 // start-up (mbarriers, the tensor map's first fetch).
 bool twide_enough(int code, int dtype, long long points);
 
-// sched = 2 * wavelet + (forward ? 1 : 0); code as from twide_code.
-void launch_twide(int dtype, int sched, int code, TWideParams const &p,
-                  cudaStream_t s);
+// Schedules of a caller's filters over the levels of dehierarchize_in and
+// (+ 1) hierarchize_in, after the wavelets' 0 .. 5.
+constexpr int kTableSched = 6;
+
+// sched = 2 * wavelet + (forward ? 1 : 0), or kTableSched (+ 1) for FP32 and
+// FP64 grids (then p.filters, and exact as from exact_scalers); code as from
+// twide_code.
+void launch_twide(int dtype, bool exact, int sched, int code,
+                  TWideParams const &p, cudaStream_t s);
 void launch_twide_f32(int sched, int code, TWideParams const &p,
                       cudaStream_t s);
 void launch_twide_f32c(int sched, int code, TWideParams const &p,
                        cudaStream_t s);
 void launch_twide_f64(int sched, int code, TWideParams const &p,
                       cudaStream_t s);
+void launch_twide_table_f32(bool exact, int sched, int code,
+                            TWideParams const &p, cudaStream_t s);
+void launch_twide_table_f64(bool exact, int sched, int code,
+                            TWideParams const &p, cudaStream_t s);
 
 // Launches one stage of a single grid: on the TMA wide kernel when it is
 // planned on it and qualifies, else on its own kernel. ws is the filters'

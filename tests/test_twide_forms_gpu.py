@@ -67,3 +67,43 @@ def test_more_tiles_than_resident_ctas(mode):
         torch.cuda.synchronize()
         exp = want(x, level, lmin, "biorthogonal", True, mode)
         assert np.array_equal(g.cpu().numpy(), exp), level
+
+
+FILTERS = {
+    # four passes, no coefficient a power of two
+    "cdf97": [(1, (-1.586134342, 1.0, -1.586134342)),
+              (0, (-0.05298011854, 1.0, -0.05298011854)),
+              (1, (0.8829110762, 1.0, 0.8829110762)),
+              (0, (0.4435068522, 1.0, 0.4435068522))],
+    # powers of two, asymmetric, a middle coefficient other than 1
+    "exact": [(0, (0.5, 2.0, -0.25)), (1, (0.0, 1.0, 0.125))],
+    "scaled": [(1, (0.3, 1.2, -0.7))],
+}
+
+
+@pytest.mark.parametrize("mode", ["f64", "f32"])
+@pytest.mark.parametrize("name", sorted(FILTERS))
+def test_callers_filters_over_ordered_levels(mode, name):
+    """transform_in over the level ranges of hierarchize_in and
+    dehierarchize_in (whole and partial) with a caller's filters, for every
+    form of the TMA wide kernel, against the oracle."""
+    import torch
+    import oracle as O
+    dtype = np.float64 if mode == "f64" else np.float32
+    rng = np.random.default_rng(29)
+    for level in ((3, 2, 4), (2, 4, 6), (4, 5, 3), (3, 6, 4), (2, 8, 5),
+                  (1, 9, 4), (1, 10, 3), (0, 11, 3), (6, 3), (5, 5), (4, 9),
+                  (2, 10), (1, 12), (4, 7, 1), (13,), (12,)):
+        dim = len(level) - 1 if len(level) < 3 else 1
+        top = level[dim]
+        for levels in (range(top, 0, -1), range(1, top + 1),
+                       range(top, max(0, top - 2), -1), [top],
+                       range(max(1, top - 2), top + 1)):
+            levels = list(levels)
+            x = rng.uniform(-1, 1, [1 << l for l in level]).astype(dtype)
+            g = torch.from_numpy(x).cuda()
+            pg.transform_in(g, dim, level, level, levels, FILTERS[name])
+            torch.cuda.synchronize()
+            exp = O.transform_in(x.copy(), level, level, dim, levels,
+                                 FILTERS[name])
+            assert np.array_equal(g.cpu().numpy(), exp), (level, levels)
