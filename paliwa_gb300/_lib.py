@@ -7,6 +7,7 @@ raises, so a GPU run can never pass on a silent substitute.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 from . import build as _build
@@ -159,16 +160,21 @@ def check(rc):
     raise _ERRORS.get(rc, PaliwaError)(msg)
 
 
+@functools.lru_cache(maxsize=None)
+def _array_type(ctype, n):
+    return ctype * n
+
+
 def i64(values):
     values = [int(v) for v in values]
-    return (ctypes.c_int64 * max(1, len(values)))(*values)
+    return _array_type(ctypes.c_int64, max(1, len(values)))(*values)
 
 
 def i32(values):
     values = [int(v) for v in values]
-    return (ctypes.c_int32 * max(1, len(values)))(*values)
+    return _array_type(ctypes.c_int32, max(1, len(values)))(*values)
 
 
 def f64(values):
     values = [float(v) for v in values]
-    return (ctypes.c_double * max(1, len(values)))(*values)
+    return _array_type(ctypes.c_double, max(1, len(values)))(*values)

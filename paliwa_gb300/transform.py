@@ -38,10 +38,17 @@ lifting_wavelet_reconstruct_offsets_and_coefficients = {
 }
 
 
+_WAVELET_IDS = {"hat": _lib.HAT, "biorthogonal": _lib.BIORTHOGONAL,
+                "fullweighting": _lib.FULLWEIGHTING}
+
+
 def wavelet_id(name):
     """Wavelet name -> library id; unknown names raise OutOfRange (a
     KeyError), as ``std::map::at`` throws std::out_of_range
     (paliwa_transform.hpp:370, 397)."""
+    known = _WAVELET_IDS.get(name) if isinstance(name, str) else None
+    if known is not None:
+        return known
     import ctypes
     out = ctypes.c_int(-1)
     _lib.check(_lib.load().paliwa_gb_wavelet_id(wavelet_name_bytes(name),
@@ -89,10 +96,16 @@ def _stream_handle(grid, stream):
 
 def _call(fn_name, grid, args, stream):
     import torch
-    lib = _lib.load()
-    with torch.cuda.device(grid.device):
-        s = _stream_handle(grid, stream)
-        _lib.check(getattr(lib, fn_name)(grid.data_ptr(), *args, s))
+    fn = getattr(_lib.load(), fn_name)
+    # The usual case needs no device switch (entering one costs more than the
+    # rest of the call's Python).
+    if grid.device.index == torch.cuda.current_device():
+        rc = fn(grid.data_ptr(), *args, _stream_handle(grid, stream))
+    else:
+        with torch.cuda.device(grid.device):
+            rc = fn(grid.data_ptr(), *args, _stream_handle(grid, stream))
+    if rc != _lib.OK:
+        _lib.check(rc)
 
 
 def hierarchize(grid, level, minimum_level, maximum_level,
