@@ -298,7 +298,8 @@ int paliwa_gb_batch_info(const paliwa_gb_batch *batch, int64_t *points,
  * point), 2048 + R the TMA wide kernel (+ 32: pencils of 8 to 32 chunks,
  * + 64: more, + 96: the last axis, + 160: its pencils of more than 32
  * chunks, + 128: inner extent 2; chunks of 32 doubles: 2048 + 224 with up to
- * 4 of them per pencil, + 225 with more, + 226 along the last axis);
+ * 4 of them per pencil, + 225 with more, + 226 along the last axis; its boxed
+ * form 2048 + 208, doubles + 227);
  * `kernels` may be null. Call with
  * capacity 0 to get *nlaunches first. */
 int paliwa_gb_batch_profile(paliwa_gb_batch *batch, int forward, void *stream,

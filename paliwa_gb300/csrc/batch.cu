@@ -389,7 +389,7 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
                 tuned || twide_enough(R - kTWide, b.dtype, points);
             for (Stage const *st : list) {
               TWideJob job;
-              CUtensorMap map;
+              CUtensorMap map[2];
               long long tiles = 0;
               if (!enough || !twide_job(*st, b.dtype, job, map, tiles)) {
                 rest[st->R].push_back(st);
@@ -397,7 +397,11 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
               }
               job.tile_begin = L.tiles;
               job.map = static_cast<int>(maps.size());
-              maps.push_back(map);
+              maps.push_back(map[0]);
+              if (st->box && job.win.seg_len > 0) {
+                job.win.halo_map = job.map + 1;
+                maps.push_back(map[1]);
+              }
               all_twide.push_back(job);
               twide_tiles.insert(twide_tiles.end(), tiles, L.njobs);
               L.tiles += tiles;

@@ -177,6 +177,33 @@ LiftJob make_job(AxisView const &v, std::vector<int> const &sh, size_t first,
 
 } // namespace
 
+namespace {
+
+// 32 or more chunks of the TMA wide kernel on more than 16 pages of 2 MB.
+bool spread_pages(AxisView const &v) {
+  int const log2chunks =
+      v.log2_n - (v.log2_es == 3 || (!v.wide_last && v.log2_n == 10) ? 5 : 4);
+  return log2chunks >= 5 && v.log2_n + v.log2_kstride + v.log2_es >= 26;
+}
+
+// Whole pencils that the TMA wide kernel runs in its boxed form: those spread
+// over pages, and FP32c pencils of 512 points in grids of 2^24 points and
+// more. Measured against the chunk-interleaved form (GB/s, 2^27 points,
+// forward CDF (2,2)): spread n = 512 4130 against 1240 (FP32c) and 5450
+// against 1240 (FP32); FP32c n = 512 otherwise 4070 against 3690, n = 256 4520
+// against 4470 and n = 128 4440 against 4620; FP32 n = 512 5400 against 5750.
+// Its CTAs take a whole SM, which costs a batch's concurrent launches more
+// than that (with FP32c and FP64 pencils of 512 points on it: 4D 20 - q 20.2
+// against 19.9 ms, FP64 4D 17 - q 3.43 against 3.18), hence the size.
+bool box_periodic(AxisView const &v) {
+  if (v.log2_inner + v.log2_es < 7 || v.log2_n < 7 || v.log2_n > 9)
+    return false;
+  return spread_pages(v) || (v.wide_last && v.log2_n == 9 &&
+                             v.columns << v.log2_n >= 1LL << 24);
+}
+
+} // namespace
+
 // Kernels that can run the periodic stages of view `v` (a bit per
 // KernelChoice), and the one chosen by default. Applicability: the wide and
 // tile kernels need a wavelet schedule (canonical level range) and a grid
@@ -254,21 +281,21 @@ KernelSet periodic_kernels(AxisView const &v, bool canon, bool ordered) {
   //  * strided FP64 pencils of 8 points and more (equal at 8, n = 512 1830
   //    against 1360);
   //  * strided float pencils of 8 points and more (FP32c n = 128 4670 against
-  //    2920, n = 2048 3430 against 2380; FP32 n = 512 5530 against 4850), but
-  //    FP32 up to 512 only (n = 1024, 16 columns: 3610 against 4650 on the
-  //    tile kernel). On 4-point chunks the two are within 1 % for single
+  //    2920, n = 2048 3430 against 2380; FP32 n = 512 5530 against 4850, n =
+  //    1024 5200 against 3840), but FP32 up to 1024 only (n = 2048, 16 columns:
+  //    3340 against 3910 on the tile kernel). On 4-point chunks the two are within 1 % for single
   //    grids, and the wide kernel is faster in batches (5.26 against
   //    4.39-4.55 TB/s).
   // Not where 32 or more chunks lie on more than 16 pages of 2 MB (pencils of
-  // 64 MB and more): a box visits the chunks row by row, so every box row
-  // then waits for its page, 8 clocks each (FP32c n = 512, 256 KB rows: 1240
-  // against 2600 GB/s, 64 KB rows 3720 against 2620; n = 1024 from 64 KB rows
-  // on 1650 against 2590; FP64 n = 1024 1250 against 1520).
+  // 64 MB and more) and the boxed form does not apply: a box visits the chunks
+  // row by row, so every box row then waits for its page, 8 clocks each (FP32c
+  // n = 512, 256 KB rows: 1240 against 2600 GB/s; n = 1024 from 64 KB rows on
+  // 1650 against 2590; FP64 n = 1024 1250 against 1520).
   if (k.has(kChooseTmaWide)) {
-    int const longest = v.log2_es == 3 ? 10 : v.wide_last ? 11 : 9;
-    int const log2chunks = v.log2_n - (v.log2_es == 3 ? 5 : 4);
-    bool const pages = log2chunks >= 5 &&
-                       v.log2_n + v.log2_kstride + v.log2_es >= 26;
+    int const longest = v.log2_es == 3 ? 10 : v.wide_last ? 11 : 10;
+    int const log2chunks =
+      v.log2_n - (v.log2_es == 3 || (!v.wide_last && v.log2_n == 10) ? 5 : 4);
+    bool const pages = spread_pages(v) && !box_periodic(v);
     if (last || pairs ||
         (v.log2_n >= 3 && v.log2_n <= longest && !pages))
       k.dflt = kChooseTmaWide;
@@ -314,6 +341,7 @@ void plan_periodic(AxisView const &v, std::vector<int> const &shifts, int ws,
                          canonical_shifts(st.job, false);
     KernelSet const ks = periodic_kernels(v, canon, ordered);
     st.tclass = tuning_class(v);
+    st.table = !canon;
     st.kernels = ks.mask;
     st.dflt = ks.dflt;
     int choice = ks.dflt;
@@ -333,6 +361,7 @@ void plan_periodic(AxisView const &v, std::vector<int> const &shifts, int ws,
       // Marked for the TMA wide kernel, and planned for the kernel it stands
       // in for, which runs the stages that do not qualify.
       st.tma = true;
+      st.box = box_periodic(v);
       choice = ks.fallback;
     }
     switch (choice) {
@@ -366,16 +395,32 @@ void plan_periodic(AxisView const &v, std::vector<int> const &shifts, int ws,
   }
 }
 
-// Fine levels of a long pencil on overlapping windows.
+// Whether the boxed form of the TMA wide kernel takes windows of view `v`
+// under these filters: rows of 128 bytes, 16-byte aligned grids, and a halo
+// that holds the reach of at least the finest level. Measured against the
+// staged kernel's windows (strided axis, GB/s): FP32 2^13 x 2^13 2770 against
+// 870, 2^15 x 2^10 2360 against 920; FP64 1490 against 800 and 1390 against
+// 890. Grids of fewer than 2^20 points (batches) keep the staged windows,
+// whose CTAs share the SMs with other launches (FP64 4D 17 - q, grids of 2^17
+// points: 3.18 against 3.23 ms).
+bool box_windows(AxisView const &v, size_t npasses) {
+  return v.base % 16 == 0 && v.shadow % 16 == 0 &&
+         v.log2_inner + v.log2_es >= 7 && npasses <= kBoxHalo &&
+         v.columns < (1LL << 29) && v.columns << v.log2_n >= 1LL << 20;
+}
+
+// Fine levels of a long pencil on overlapping windows: of 4096 points on the
+// staged kernel, or (box) of 512 on the TMA wide kernel's boxed form.
 void plan_windows(AxisView const &v, std::vector<int> const &shifts,
-                  std::vector<Filter> const &filters,
+                  std::vector<Filter> const &filters, bool box,
                   std::vector<Stage> &out) {
-  long long const window = 1LL << kWindowLog2;
+  int const log2_window = box ? kBoxWindowLog2 : kWindowLog2;
+  long long const window = 1LL << log2_window;
   AxisView wv = v;
-  wv.log2_n = kWindowLog2;
-  int const R = staged_chunk(wv);
+  wv.log2_n = log2_window;
+  int const R = box ? 16 : staged_chunk(wv);
   long long const C = static_cast<long long>(kRounds) *
-                      (kThreads >> (kWindowLog2 - (31 - __builtin_clz(R))));
+                      (kThreads >> (log2_window - (31 - __builtin_clz(R))));
   size_t first = 0;
   while (first < shifts.size()) {
     // Grow the run while the halo it needs fits the window: each step of
@@ -390,7 +435,7 @@ void plan_windows(AxisView const &v, std::vector<int> const &shifts,
       reach += add;
       ++count;
     }
-    long long const halo = ceil_div(reach, R) * R;
+    long long const halo = box ? kBoxHalo : ceil_div(reach, R) * R;
     long long const seg_len = window - 2 * halo;
     if (seg_len <= 0)
       throw StatusError(PALIWA_GB_INVALID_ARGUMENT,
@@ -424,7 +469,8 @@ void plan_windows(AxisView const &v, std::vector<int> const &shifts,
     st.job = make_job(v, shifts, first, count);
     st.job.halo_base = v.shadow;
     st.job.periodic = 0;
-    st.job.log2_window = kWindowLog2;
+    st.job.log2_window = log2_window;
+    st.tma = st.box = box;
     st.job.seg_len = static_cast<int>(seg_len);
     st.job.halo = static_cast<int>(halo);
     st.job.col_tiles = ceil_div(v.columns, C);
@@ -445,11 +491,24 @@ void plan_axis(AxisView const &view, std::vector<int> const &shifts,
     return;
   }
   // Long pencil: levels closer than 2^m run on windows with a halo of at most
-  // kHaloBudget points per side; the others run on the sub-lattice of every
-  // 2^m-th point, which is a periodic pencil 2^m times shorter.
+  // `budget` points per side; the others run on the sub-lattice of every
+  // 2^m-th point, which is a periodic pencil 2^m times shorter. Levels in
+  // order and rows of 128 bytes take the boxed form's windows, whose halo of
+  // 32 points of 512 is the same 14 % as 256 of 4096 and leaves 1/16 of the
+  // points (1/32 for one pass) to the sub-lattice.
   int const P = static_cast<int>(filters.size());
+  LiftJob const order = make_job(
+      view, shifts, 0, std::min(shifts.size(), static_cast<size_t>(kMaxLevels)));
+  bool const ordered = shifts.size() <= kMaxLevels &&
+                       (canonical_shifts(order, true) ||
+                        canonical_shifts(order, false));
+  // Not FP32c: it rounds to its storage between the two kinds of stages, so
+  // an earlier split would round more points twice.
+  bool const box =
+      ordered && !view.wide_last && box_windows(view, filters.size());
+  int const budget = box ? kBoxHalo : kHaloBudget;
   int m = 0;
-  while (static_cast<long long>(P) * ((2LL << m) - 1) <= kHaloBudget) ++m;
+  while (static_cast<long long>(P) * ((2LL << m) - 1) <= budget) ++m;
   if (m < 1) m = 1;
   size_t i = 0;
   while (i < shifts.size()) {
@@ -458,7 +517,7 @@ void plan_axis(AxisView const &view, std::vector<int> const &shifts,
     while (j < shifts.size() && (shifts[j] < m) == fine) ++j;
     std::vector<int> run(shifts.begin() + i, shifts.begin() + j);
     if (fine) {
-      plan_windows(view, run, filters, out);
+      plan_windows(view, run, filters, box, out);
     } else {
       AxisView sub = view;
       sub.log2_n = view.log2_n - m;

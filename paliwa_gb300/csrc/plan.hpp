@@ -87,12 +87,19 @@ struct Stage {
   // (otherwise launches of few points keep the stage's own kernel).
   bool tma = false;
   bool tuned = false;
+  // ... in its boxed form (twide_box.cuh): pencils whose rows lie on pages of
+  // their own, and windows of 2^kBoxWindowLog2 points.
+  bool box = false;
+  bool table = false;  // a caller's filters (no wavelet's levels)
 };
 
 constexpr int kWindowLog2 = 12;   // points per column per CTA round (4096)
 constexpr int kThreads = 256;
 constexpr int kRounds = kTileRounds;  // column rounds per tile
 constexpr int kHaloBudget = 256;  // halo per side of a window, in points
+// Windows of the TMA wide kernel's boxed form.
+constexpr int kBoxWindowLog2 = 9;
+constexpr int kBoxHalo = 32;
 
 int chunk_for(int log2_n);        // R for a periodic pencil of 2^log2_n
 

@@ -76,6 +76,10 @@ constexpr int kTWideLongContig = 160;
 constexpr int kTWide32Dense = 224;
 constexpr int kTWide32Chunked = 225;
 constexpr int kTWide32Pairs = 226;
+// The boxed form (twide_box.cuh): with the chunk size of floats, and with
+// 32-point chunks of doubles.
+constexpr int kTWideBox = 192;
+constexpr int kTWide32Box = 227;
 
 struct TWideJob {
   long long tile_begin;  // first tile of this job in the launch
@@ -83,15 +87,24 @@ struct TWideJob {
   int log2_n;            // pencil length
   int log2_inner;        // columns per outer index
   int nlevels;
-  int log2_bx;           // box: 2^log2_bx columns of one outer index
-  int log2_sx;           // box: 2^log2_sx outer indices
-  int nxb;               // boxes per tile
-  int chunked;           // 0: the dense layout, 1: the chunk-interleaved
-                         // layout (G >= 8), 2: the contiguous layout (the
-                         // last axis), 3: the pairs layout (strided,
-                         // inner extent 2)
-  int log2_rs;           // floats between a thread's rows in shared memory
-  int log2_xlo;          // chunk-interleaved layout: columns per group
+  union {
+    struct {
+      int log2_bx;     // box: 2^log2_bx columns of one outer index
+      int log2_sx;     // box: 2^log2_sx outer indices
+      int nxb;         // boxes per tile
+      int chunked;     // 0: the dense layout, 1: the chunk-interleaved layout
+                       // (G >= 8), 2: the contiguous layout (the last axis),
+                       // 3: the pairs layout (strided, inner extent 2)
+      int log2_rs;     // floats between a thread's rows in shared memory
+      int log2_xlo;    // chunk-interleaved layout: columns per group
+    };
+    // Boxed form: windows of segments of seg_len points (0: whole pencils of
+    // log2_n) with halo points on either side, of pencils of 2^log2_full
+    // points; the halo buffer's map; column tiles per segment.
+    struct {
+      int seg_len, halo, log2_full, halo_map, col_tiles;
+    } win;
+  };
 };
 
 struct TWideParams {
@@ -101,9 +114,10 @@ struct TWideParams {
   long long total_tiles;
   unsigned *error;          // set to 1 when a bounded wait gives up
   int ctas_per_sm;          // cap on the launch's CTAs per SM (0: none)
-  // jobs == nullptr: the launch's only job and its map.
+  // jobs == nullptr: the launch's only job and its maps
+  // (map[1]: a window's halo buffer).
   TWideJob job;
-  CUtensorMap map;
+  CUtensorMap map[2];
   FilterTable filters;  // read by TableSched launches
 };
 
@@ -306,7 +320,7 @@ __global__ void __launch_bounds__(twide_threads(R) + 32, R >= 16 ? 2 : 3)
   // The producer lane issues every copy; it keeps the last map it fenced.
   // A single job's map (0) lies in the parameters and needs no fence.
   TWideJob const *const jobs = p.jobs != nullptr ? p.jobs : &p.job;
-  CUtensorMap const *const maps = p.jobs != nullptr ? p.maps : &p.map;
+  CUtensorMap const *const maps = p.jobs != nullptr ? p.maps : p.map;
   int fenced = p.jobs != nullptr ? -1 : 0;
   auto issue_load = [&](long long k) {
     int const b = static_cast<int>(k % S);
@@ -607,7 +621,7 @@ __global__ void __launch_bounds__(kTWideThreads, 2)
   // bytes); it keeps the last map it fenced.
   // A single job's map (0) lies in the parameters and needs no fence.
   TWideJob const *const jobs = p.jobs != nullptr ? p.jobs : &p.job;
-  CUtensorMap const *const maps = p.jobs != nullptr ? p.maps : &p.map;
+  CUtensorMap const *const maps = p.jobs != nullptr ? p.maps : p.map;
   int fenced = p.jobs != nullptr ? -1 : 0;
   auto origin = [](TWideJob const &job, long long tile, int &q0, int &z0) {
     int const log2ct = LOG2NT + 1 - (job.log2_n - LOG2R);

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "launch.cuh"
+#include "twide_box.cuh"
 #include "twide_plan.hpp"
 
 namespace pgb {
@@ -11,14 +12,20 @@ template <class A, int R, class Sched, int FORM>
 void launch_twide_r(TWideParams const &p, cudaStream_t s) {
   static thread_local Occupancy occ;
   constexpr bool kLong = FORM == 2 || FORM == 5;
-  constexpr int kBlock = kLong ? kTWideThreads : twide_threads(R) + 32;
+  constexpr bool kBox = FORM == 6;
+  constexpr int kBlock = kLong  ? kTWideThreads
+                         : kBox ? box_threads(R) + 32
+                                : twide_threads(R) + 32;
   auto kernel = [] {
     if constexpr (kLong)
       return twide_long_kernel<A, Sched, FORM == 5>;
+    else if constexpr (kBox)
+      return twide_box_kernel<A, R, Sched>;
     else
       return twide_kernel<A, R, Sched, FORM>;
   }();
-  size_t const smem = twide_smem_bytes<R, kLong>();
+  size_t const smem =
+      kBox ? box_smem_bytes<R>() : twide_smem_bytes<R, kLong>();
   int const dev = current_device();
   if (dev < 0 || dev >= Occupancy::kMaxDevices)
     throw StatusError(2, "device ordinal beyond the launch cache");
@@ -60,6 +67,11 @@ void launch_twide_rows(int code, TWideParams const &p, cudaStream_t s) {
   case kTWidePairs + 16: return launch_twide_r<A, 16, Sched, 4>(p, s);
   case kTWideLong + 16: return launch_twide_r<A, 16, Sched, 2>(p, s);
   case kTWideLongContig + 16: return launch_twide_r<A, 16, Sched, 5>(p, s);
+  case kTWideBox + 16: return launch_twide_r<A, 16, Sched, 6>(p, s);
+  case kTWide32Chunked:
+    if constexpr (sizeof(typename A::V) <= 8)  // plain floats
+      return launch_twide_r<A, 32, Sched, 1>(p, s);
+    break;
   }
   throw StatusError(2, "twide launch with an unsupported form");
 }
@@ -78,6 +90,7 @@ void launch_twide_cols(int code, TWideParams const &p, cudaStream_t s) {
   case kTWide32Dense: return launch_twide_r<A, 32, Sched, 0>(p, s);
   case kTWide32Chunked: return launch_twide_r<A, 32, Sched, 1>(p, s);
   case kTWide32Pairs: return launch_twide_r<A, 32, Sched, 4>(p, s);
+  case kTWide32Box: return launch_twide_r<A, 32, Sched, 6>(p, s);
   }
   throw StatusError(2, "twide launch with an unsupported form");
 }

@@ -6,6 +6,7 @@
 #include <mutex>
 
 #include "paliwa_gb300.h"
+#include "twide_box.cuh"
 #include "twide_plan.hpp"
 
 namespace pgb {
@@ -32,11 +33,17 @@ namespace {
 // 32 points and chunks of 32 beyond: the FP64 pipe runs a coarse step of one
 // head per chunk as a whole warp instruction, so half the chunks are half
 // that waste (512 points: 140 instead of 160 DFMAs for every 128 needed).
-int twide_chunk(LiftJob const &job, int dtype) {
+int twide_chunk(LiftJob const &job, int dtype, bool table) {
   int const n = job.log2_n;
   bool const last = job.log2_inner == 0 && job.log2_kstride == 0;
   if (dtype == PALIWA_GB_F64) return n < 1 || n > 10 ? 0 : 1 << std::min(n, 5);
   if (n < 1 || n > (last ? 12 : 11)) return 0;
+  // Plain floats: strided pencils of 1024 points in chunks of 32, which
+  // exchange by shuffles (5200 GB/s against 3310-3870 in the long form and
+  // 3840-4650 on the tile kernel); with a caller's filters also those of 512
+  // (four passes: 3110 against 2830; CDF (2,2): 5470 against 5530).
+  if (dtype == PALIWA_GB_F32 && !last && (n == 10 || (n == 9 && table)))
+    return 32;
   if (n <= 4) return 1 << n;
   if (n <= 6 && !last) return 1 << (n - 2);
   return 16;
@@ -45,13 +52,15 @@ int twide_chunk(LiftJob const &job, int dtype) {
 } // namespace
 
 int twide_code(Stage const &st, int dtype) {
-  int const r = st.tma ? twide_chunk(st.job, dtype) : 0;
+  if (st.box)
+    return dtype == PALIWA_GB_F64 ? kTWide32Box : kTWideBox + 16;
+  int const r = st.tma ? twide_chunk(st.job, dtype, st.table) : 0;
   if (r == 0) return 0;
   int const log2G = st.job.log2_n - (31 - __builtin_clz(r));
   // Inner extent in floats (see twide_job).
   int const inner = st.job.log2_inner + (dtype == PALIWA_GB_F64 ? 1 : 0);
   if (r == 32)
-    return inner == 1 ? kTWide32Pairs
+    return dtype == PALIWA_GB_F64 && inner == 1 ? kTWide32Pairs
            : log2G >= 3 ? kTWide32Chunked : kTWide32Dense;
   bool const last = inner == 0 && st.job.log2_kstride == 0;
   return r + (last         ? (log2G > 5 ? kTWideLongContig : kTWideContig)
@@ -68,10 +77,72 @@ int twide_code(Stage const &st, int dtype) {
 // (FP32 n = 128 at 2^12 4.1 against 6.7).
 bool twide_enough(int code, int dtype, long long points) {
   bool const longer =
-      code == kTWide32Chunked || code == kTWideChunked + 16 ||
+      code == kTWideBox + 16 || code == kTWide32Box || code == kTWide32Chunked || code == kTWideChunked + 16 ||
       code == kTWideLong + 16 || code == kTWideLongContig + 16;
   return longer || points >= (dtype == PALIWA_GB_F64 ? 1LL << 12 : 1LL << 13);
 }
+
+namespace {
+
+// Boxed form: the 3D view [outer][n][inner] of the grid (and of the halo
+// buffer, in the same layout) in boxes of 128 bytes of columns by one chunk.
+bool twide_box_job(Stage const &st, int dtype, TWideJob &job,
+                   CUtensorMap map[2], long long &tiles) {
+  auto const encode = tensor_map_encoder();
+  LiftJob lj = st.job;
+  int const r = dtype == PALIWA_GB_F64 ? 32 : 16;
+  if (dtype == PALIWA_GB_F64) {  // a double column is two float columns
+    ++lj.log2_inner;
+    ++lj.log2_kstride;
+    ++lj.log2_astride;
+    lj.columns *= 2;
+  }
+  int const log2w = lj.periodic ? lj.log2_n : lj.log2_window;
+  int const log2boxes = 31 - __builtin_clz(
+                                 static_cast<unsigned>(kBoxRows / r));
+  int const log2G = log2w - (31 - __builtin_clz(static_cast<unsigned>(r)));
+  if (encode == nullptr || lj.log2_inner < 5 || log2w > 9 || log2G < 1 ||
+      log2G > log2boxes || (lj.base | lj.halo_base) % 16 != 0 ||
+      lj.log2_n > 30)
+    return false;
+  std::memset(&job, 0, sizeof(job));
+  job.log2_n = log2w;
+  job.log2_inner = lj.log2_inner;
+  job.nlevels = lj.nlevels;
+  job.win.halo_map = 1;
+  // Tiles of 2^(log2boxes - log2G) blocks of 32 floats.
+  int const log2ct = 5 + log2boxes - log2G;
+  long long const ct = (lj.columns + (1LL << log2ct) - 1) >> log2ct;
+  long long segments = 1;
+  if (!lj.periodic) {
+    if (lj.halo_base == 0 || lj.seg_len % r != 0 || lj.halo % r != 0)
+      return false;
+    job.win.seg_len = lj.seg_len;
+    job.win.halo = lj.halo;
+    job.win.log2_full = lj.log2_n;
+    segments = ((1LL << lj.log2_n) + lj.seg_len - 1) / lj.seg_len;
+  }
+  tiles = ct * segments;
+  if (tiles >= (1LL << 30)) return false;
+  job.win.col_tiles = static_cast<int>(ct);
+  cuuint64_t dims[3] = {static_cast<cuuint64_t>(1) << lj.log2_inner,
+                        static_cast<cuuint64_t>(1) << lj.log2_n,
+                        static_cast<cuuint64_t>(lj.columns >> lj.log2_inner)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(4) << lj.log2_kstride,
+                           static_cast<cuuint64_t>(4) << lj.log2_astride};
+  cuuint32_t box[3] = {32, static_cast<cuuint32_t>(r), 1};
+  cuuint32_t elem[3] = {1, 1, 1};
+  for (int i = 0; i < (lj.periodic ? 1 : 2); ++i)
+    if (encode(&map[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
+               reinterpret_cast<void *>(i == 0 ? lj.base : lj.halo_base),
+               dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return false;
+  return true;
+}
+
+} // namespace
 
 // Up to 4 chunks per pencil (dense): the 3D view [outer][n][inner] of the
 // stage's pencils with the axis' strides and boxes {Bx, n, Sx}. 8 chunks and
@@ -79,11 +150,12 @@ bool twide_enough(int code, int dtype, long long points) {
 // [chunk][X columns] and one box per tile, so that shared memory holds the
 // tile as [column group][row of chunk][chunk][X columns]. The last axis and
 // inner extents of 2 floats: rows of 128 bytes.
-bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap &map,
+bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap map[2],
                long long &tiles) {
   auto encode = tensor_map_encoder();
+  if (st.box) return twide_box_job(st, dtype, job, map, tiles);
   LiftJob lj = st.job;
-  int const r = twide_chunk(lj, dtype);
+  int const r = twide_chunk(lj, dtype, st.table);
   if (encode == nullptr || r == 0 || lj.periodic != 1 || lj.base % 16 != 0)
     return false;
   // A double column is two float columns: the grid is viewed as floats with
@@ -127,7 +199,7 @@ bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap &map,
     cuuint32_t box[2] = {32, 1u << (log2unit - 5)};
     cuuint32_t elem[2] = {1, 1};
     CUresult const res = encode(
-        &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+        &map[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
         reinterpret_cast<void *>(lj.base), dims, strides, box, elem,
         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -166,10 +238,13 @@ bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap &map,
     // where the pencils span 256 MB or more: every box row is then a page of
     // its own, at 8 clocks each (n = 128 4.75 against 3.25, n = 256 3.97
     // against 3.53 and less; below that span 4.77 against 4.84 and 3.97
-    // against 4.45).
+    // against 4.45). A caller's filters take 8 (four passes, n = 256 3.2
+    // against 2.9 TB/s).
     bool const spread =
         lj.log2_n + lj.log2_kstride + 2 >= 28 || dtype == PALIWA_GB_F32;
-    int const xmax = log2G > 5 ? 2 : log2G <= 4 && r == 16 && spread ? 4 : 3;
+    int const xmax = log2G > 5 ? 2
+                     : log2G <= 4 && dtype != PALIWA_GB_F64 && !st.table &&
+                             spread ? 4 : 3;
     int const xlo = std::max(2, std::min({xmax, log2ct, lj.log2_inner}));
     job.log2_xlo = xlo;
     job.log2_rs = log2G + xlo;
@@ -186,7 +261,7 @@ bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap &map,
                          1u << (job.log2_bx - xlo), 1u << job.log2_sx};
     cuuint32_t elem[5] = {1, 1, 1, 1, 1};
     CUresult const res = encode(
-        &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5,
+        &map[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5,
         reinterpret_cast<void *>(lj.base), dims, strides, box, elem,
         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -217,7 +292,7 @@ bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap &map,
   }
   cuuint32_t elem[3] = {1, 1, 1};
   CUresult const res = encode(
-      &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
+      &map[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
       reinterpret_cast<void *>(lj.base), dims, strides, box, elem,
       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

@@ -21,10 +21,11 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 // the other stages.
 int twide_code(Stage const &st, int dtype);
 
-// The stage's job, tensor map and tiles. False when it does not qualify
-// (alignment, 2^30 tiles or more, or the encoder refuses the map); the stage
+// The stage's job, tensor maps (map[1], the halo buffer's, for windows only)
+// and tiles; the job names them 0 and 1. False when it does not qualify
+// (alignment, 2^30 tiles or more, or the encoder refuses a map); the stage
 // then runs on its own kernel (Stage::R).
-bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap &map,
+bool twide_job(Stage const &st, int dtype, TWideJob &job, CUtensorMap map[2],
                long long &tiles);
 
 // Whether a launch of form `code` over `points` points in all is worth its

@@ -79,9 +79,11 @@ TWIDE_LONG = 64
 TWIDE_CONTIG = 96
 TWIDE_PAIRS = 128
 TWIDE_LONG_CONTIG = 160
-# Chunks of 32 points (FP64): their own codes per form.
+# Chunks of 32 points (FP64) have their own codes per form.
 TWIDE_32 = {224: "twide_kernel R=32", 225: "twide_kernel chunked R=32",
-            226: "twide_kernel inner 2 R=32"}
+            226: "twide_kernel inner 2 R=32",
+            # the boxed form, of floats and of doubles
+            208: "twide_kernel boxed R=16", 227: "twide_kernel boxed R=32"}
 
 
 def kernel_name(code):

@@ -107,3 +107,47 @@ def test_callers_filters_over_ordered_levels(mode, name):
             exp = O.transform_in(x.copy(), level, level, dim, levels,
                                  FILTERS[name])
             assert np.array_equal(g.cpu().numpy(), exp), (level, levels)
+
+
+@pytest.mark.parametrize("mode", ["f64", "f32"])
+@pytest.mark.parametrize("level,lmin", [
+    ((2, 13, 5), 0), ((2, 14, 4), 9), ((0, 15, 6), 3), ((1, 17, 4), 0),
+    ((3, 13, 3), 0), ((15, 5), 11), ((14, 4), 0)])
+def test_long_strided_pencils(mode, level, lmin):
+    """Pencils of more than 4096 points: windows in the boxed form (rows of
+    128 bytes and more; narrower ones on the staged kernel), with short last
+    segments and partial level ranges."""
+    import torch
+    dim = 0 if len(level) == 2 else 1
+    lo = tuple(lmin if d == dim else l for d, l in enumerate(level))
+    dtype = np.float64 if mode == "f64" else np.float32
+    rng = np.random.default_rng(sum(level))
+    x = rng.uniform(-1, 1, [1 << l for l in level]).astype(dtype)
+    for wavelet in WAVELETS:
+        for forward in (True, False):
+            g = torch.from_numpy(x).cuda()
+            f = pg.hierarchize if forward else pg.dehierarchize
+            f(g, level, lo, level, wavelet)
+            torch.cuda.synchronize()
+            exp = want(x, level, lo, wavelet, forward, mode)
+            assert np.array_equal(g.cpu().numpy(), exp), (wavelet, forward)
+
+
+@pytest.mark.parametrize("mode", ["f64", "f32", "f32c"])
+@pytest.mark.parametrize("level", [(9, 15), (9, 17)])
+def test_pencils_spread_over_pages(mode, level):
+    """512-point pencils of 64 MB and more: the boxed form for floats."""
+    import torch
+    dtype = np.float64 if mode == "f64" else np.float32
+    if mode == "f64" and sum(level) > 24:
+        pytest.skip("the doubles' form does not depend on the span")
+    rng = np.random.default_rng(7)
+    x = rng.uniform(-1, 1, [1 << l for l in level]).astype(dtype)
+    lo = (0, level[1])
+    for forward in (True, False):
+        g = torch.from_numpy(x).cuda()
+        f = pg.hierarchize if forward else pg.dehierarchize
+        f(g, level, lo, level, "biorthogonal", compensated=mode == "f32c")
+        torch.cuda.synchronize()
+        exp = want(x, level, lo, "biorthogonal", forward, mode)
+        assert np.array_equal(g.cpu().numpy(), exp), forward
