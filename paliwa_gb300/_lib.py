@@ -166,8 +166,11 @@ def _array_type(ctype, n):
 
 
 def i64(values):
-    values = [int(v) for v in values]
-    return _array_type(ctypes.c_int64, max(1, len(values)))(*values)
+    try:  # ints go in as they are
+        return _array_type(ctypes.c_int64, len(values) or 1)(*values)
+    except TypeError:
+        values = [int(v) for v in values]
+        return _array_type(ctypes.c_int64, len(values) or 1)(*values)
 
 
 def i32(values):

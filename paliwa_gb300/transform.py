@@ -90,6 +90,9 @@ def _check_grid(grid, level):
 def _stream_handle(grid, stream):
     import torch
     if stream is None:
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if raw is not None:  # the handle without a Stream object around it
+            return raw(grid.device.index)
         stream = torch.cuda.current_stream(grid.device)
     return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
