@@ -24,14 +24,8 @@
 #include "combine.cuh"
 #include "paliwa_gb300.h"
 #include "plan.hpp"
-#include "slab.cuh"
+#include "slab_plan.hpp"
 #include "twide_plan.hpp"
-
-namespace pgb {
-void launch_slab_f64(int sched, SlabParams const &p, cudaStream_t s);
-void launch_slab_f32(int sched, SlabParams const &p, cudaStream_t s);
-void launch_slab_f32c(int sched, SlabParams const &p, cudaStream_t s);
-} // namespace pgb
 
 using namespace pgb;
 
@@ -187,94 +181,6 @@ bool default_slabs(int dtype, long long points) {
   return true;
 }
 
-// The slab group of grid g: its trailing axes whose slab (the product of
-// their extents) fits one tile, when that group holds at least two axes
-// with levels to transform, the grid is a whole number of 1 KB boxes and
-// starts on a row of the tensor map. Returns the group's first axis, or
-// ndim for none.
-int slab_start(paliwa_gb_batch const &b, int g, int64_t const *levels,
-               int64_t const *lmin) {
-  size_t const es = dtype_size(b.dtype);
-  int const log2es = es == 8 ? 3 : 2;
-  int64_t const *lv = levels + static_cast<size_t>(g) * b.ndim;
-  int64_t total = 0;
-  for (int d = 0; d < b.ndim; ++d) total += lv[d];
-  if (total + log2es < 10) return b.ndim;  // under one 1 KB box
-  unsigned long long const addr =
-      reinterpret_cast<unsigned long long>(b.grids[g]);
-  if (addr < b.slab_base || (addr - b.slab_base) % 128 != 0) return b.ndim;
-  int m = b.ndim;
-  int64_t vol = 0;
-  while (m > 0 && vol + lv[m - 1] + log2es <= 15) vol += lv[--m];
-  int work = 0;
-  for (int d = m; d < b.ndim; ++d) work += lv[d] > lmin[d];
-  return work >= 2 ? m : b.ndim;
-}
-
-// The slab job of grid g for its axes m..ndim-1: per axis with levels to
-// transform, the pencil length, its element stride inside a tile (the
-// product of the later extents) and the chunk size: 32 points (at most the
-// pencil) for the contiguous last axis and for strides of 32 elements or
-// more, 8 or fewer for smaller strides when the pencil's chunks then fit
-// the CTA's 256 threads (distinct shared-memory banks under the swizzle).
-SlabJob slab_job(paliwa_gb_batch const &b, int g, int m,
-                 int64_t const *levels, int64_t const *lmin,
-                 void *const *grid_ptrs) {
-  size_t const es = dtype_size(b.dtype);
-  int const log2es = es == 8 ? 3 : 2;
-  int64_t const *lv = levels + static_cast<size_t>(g) * b.ndim;
-  SlabJob job;
-  std::memset(&job, 0, sizeof(job));
-  int64_t total = 0;
-  for (int d = 0; d < b.ndim; ++d) total += lv[d];
-  job.log2_tile = static_cast<int>(std::min<int64_t>(total, 15 - log2es));
-  job.row0 = static_cast<long long>(
-      (reinterpret_cast<unsigned long long>(grid_ptrs[g]) - b.slab_base) / 128);
-  int log2s = 0;
-  std::vector<SlabAxis> axes;
-  for (int d = b.ndim - 1; d >= m; --d) {
-    int const log2n = static_cast<int>(lv[d]);
-    int const nlev = static_cast<int>(lv[d] - lmin[d]);
-    if (nlev > 0) {
-      SlabAxis ax;
-      ax.log2n = static_cast<signed char>(log2n);
-      ax.log2s = static_cast<signed char>(log2s);
-      ax.nlevels = static_cast<signed char>(nlev);
-      int log2r = std::min(log2n, 5);
-      if (log2s >= 1 && log2s <= 4 && log2n + log2s - 3 <= 8)
-        log2r = std::min(log2n, 3);
-      ax.log2r = static_cast<signed char>(log2r);
-      axes.push_back(ax);
-    }
-    log2s += log2n;
-  }
-  std::reverse(axes.begin(), axes.end());
-  job.naxes = static_cast<int>(axes.size());
-  for (size_t i = 0; i < axes.size(); ++i) job.axis[i] = axes[i];
-  return job;
-}
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
-// against libcuda): a 2D view [rows][128 bytes] from `base`, 1 KB boxes
-// (8 rows), 128-byte swizzle.
-bool encode_slab_map(CUtensorMap *map, unsigned long long base,
-                     unsigned long long rows, size_t es) {
-  auto const encode = tensor_map_encoder();
-  if (encode == nullptr) return false;
-  if (rows == 0 || rows > (1ULL << 31)) return false;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(128 / es), rows};
-  cuuint64_t strides[1] = {128};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / es), 8};
-  cuuint32_t elem[2] = {1, 1};
-  CUresult const r = encode(
-      map, es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
-                   : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-      2, reinterpret_cast<void *>(base), dims, strides, box, elem,
-      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
-}
-
 // The tensor map over every grid of the batch (rows of 128 bytes from the
 // lowest grid address, rounded down to 128 bytes).
 void setup_slab_map(paliwa_gb_batch &b) {
@@ -314,7 +220,9 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
   std::vector<int> slab_from(b.ngrids, b.ndim);
   if (b.use_slabs && dr.slabs && b.slab_map_ok && ws >= 0)
     for (int g = 0; g < b.ngrids; ++g)
-      slab_from[g] = slab_start(b, g, levels, lmin);
+      slab_from[g] = slab_start(
+          b.dtype, b.ndim, levels + static_cast<size_t>(g) * b.ndim, lmin,
+          reinterpret_cast<unsigned long long>(b.grids[g]), b.slab_base);
   for (int grp = 0; grp < b.ngroups; ++grp) {
     std::vector<int> members;
     for (int g = 0; g < b.ngrids; ++g)
@@ -456,7 +364,10 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
     L.tile_first = slab_tiles.size();
     for (int g : members) {
       if (slab_from[g] >= b.ndim) continue;
-      SlabJob job = slab_job(b, g, slab_from[g], levels, lmin, grid_ptrs);
+      SlabJob job = slab_job(
+          b.dtype, b.ndim, slab_from[g],
+          levels + static_cast<size_t>(g) * b.ndim, lmin,
+          reinterpret_cast<unsigned long long>(grid_ptrs[g]), b.slab_base);
       job.tile_begin = L.tiles;
       int64_t total = 0;
       for (int k = 0; k < b.ndim; ++k) total += levels[g * b.ndim + k];
@@ -539,12 +450,7 @@ void launch_one(paliwa_gb_batch &b, Direction &dr, Launch const &L,
   p.njobs = L.njobs;
   p.total_tiles = L.tiles;
   p.error = b.slab_error;
-  switch (b.dtype) {
-  case PALIWA_GB_F64: return launch_slab_f64(L.sched, p, s);
-  case PALIWA_GB_F32: return launch_slab_f32(L.sched, p, s);
-  case PALIWA_GB_F32C: return launch_slab_f32c(L.sched, p, s);
-  }
-  throw StatusError(PALIWA_GB_INVALID_ARGUMENT, "unknown dtype");
+  launch_slab(b.dtype, L.sched, p, s);
 }
 
 void run_direction(paliwa_gb_batch &b, Direction &dr, cudaStream_t s) {

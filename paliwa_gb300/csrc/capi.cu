@@ -7,6 +7,7 @@
 
 #include "paliwa_gb300.h"
 #include "launch.cuh"
+#include "slab_plan.hpp"
 #include "twide_plan.hpp"
 
 namespace pgb {
@@ -665,10 +666,18 @@ int hierarchize_dims(void *grid, int dtype, int ndim, int64_t const *level,
     if (dim_begin < 0 || dim_end > ndim || dim_begin >= dim_end)
       throw StatusError(PALIWA_GB_INVALID_ARGUMENT, "bad dimension");
     auto const filters = wavelet_filters(wavelet, forward);
-    for (int d = dim_begin; d < dim_end; ++d)
+    cudaStream_t const s = static_cast<cudaStream_t>(stream);
+    // Every axis: the trailing ones may go in one launch of the slab kernel.
+    int const slab = dim_begin == 0 && dim_end == ndim
+                         ? single_slab_start(dtype, ndim, level, lmin, grid)
+                         : dim_end;
+    for (int d = dim_begin; d < dim_end; ++d) {
+      if (d == slab && launch_single_slab(dtype, ndim, slab, level, lmin, grid,
+                                          wavelet_schedule(filters), s))
+        break;
       transform_axis(grid, dtype, ndim, level, d,
-                     level_shifts(level[d], lmin[d], forward), filters,
-                     static_cast<cudaStream_t>(stream));
+                     level_shifts(level[d], lmin[d], forward), filters, s);
+    }
   });
 }
 

@@ -66,6 +66,7 @@ struct SlabParams {
   long long total_tiles;
   unsigned *error;          // set to 1 when a bounded wait gives up
   int ctas_per_sm;          // cap on the launch's CTAs per SM (0: none)
+  SlabJob job;              // jobs == nullptr: the launch's only job
 };
 
 // ---- PTX wrappers (sm_90+ bulk tensor copies and mbarriers)
@@ -364,10 +365,11 @@ __global__ void __launch_bounds__(kSlabThreads, 2)
   auto issue_load = [&](long long k) {
     int const b = static_cast<int>(k % kSlabStages);
     long long const tile = first + k * step;
-    int const j = p.tile_job[tile];
+    SlabJob const *const job_of =
+        p.jobs != nullptr ? p.jobs + p.tile_job[tile] : &p.job;
     if (lane < kJobWords)
       reinterpret_cast<unsigned *>(&sjob[b])[lane] =
-          reinterpret_cast<unsigned const *>(p.jobs + j)[lane];
+          reinterpret_cast<unsigned const *>(job_of)[lane];
     __syncwarp();
     SlabJob const &job = sjob[b];
     int const bytes = 1 << (job.log2_tile + LOG2ES);

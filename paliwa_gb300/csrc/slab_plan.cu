@@ -1,0 +1,149 @@
+// Host side of the slab kernel (slab.cuh): slab groups, jobs, tensor maps and
+// the single-grid launch.
+#include <algorithm>
+#include <cstring>
+#include <vector>
+
+#include "paliwa_gb300.h"
+#include "slab_plan.hpp"
+
+namespace pgb {
+
+// The slab group of a grid: its trailing axes whose slab (the product of
+// their extents) fits one tile, when that group holds at least two axes
+// with levels to transform, the grid is a whole number of 1 KB boxes and
+// starts on a row of the tensor map (rows of 128 bytes from map_base).
+// Returns the group's first axis, or ndim for none.
+int slab_start(int dtype, int ndim, int64_t const *lv, int64_t const *lmin,
+               unsigned long long addr, unsigned long long map_base) {
+  int const log2es = dtype_size(dtype) == 8 ? 3 : 2;
+  int64_t total = 0;
+  for (int d = 0; d < ndim; ++d) total += lv[d];
+  if (total + log2es < 10) return ndim;  // under one 1 KB box
+  if (addr < map_base || (addr - map_base) % 128 != 0) return ndim;
+  int m = ndim;
+  int64_t vol = 0;
+  while (m > 0 && vol + lv[m - 1] + log2es <= 15) vol += lv[--m];
+  int work = 0;
+  for (int d = m; d < ndim; ++d) work += lv[d] > lmin[d];
+  return work >= 2 && work <= kSlabMaxAxes ? m : ndim;
+}
+
+// The slab job of a grid for its axes m..ndim-1: per axis with levels to
+// transform, the pencil length, its element stride inside a tile (the
+// product of the later extents) and the chunk size: 32 points (at most the
+// pencil) for the contiguous last axis and for strides of 32 elements or
+// more, 8 or fewer for smaller strides when the pencil's chunks then fit
+// the CTA's 256 threads (distinct shared-memory banks under the swizzle).
+SlabJob slab_job(int dtype, int ndim, int m, int64_t const *lv,
+                 int64_t const *lmin, unsigned long long addr,
+                 unsigned long long map_base) {
+  int const log2es = dtype_size(dtype) == 8 ? 3 : 2;
+  SlabJob job;
+  std::memset(&job, 0, sizeof(job));
+  int64_t total = 0;
+  for (int d = 0; d < ndim; ++d) total += lv[d];
+  job.log2_tile = static_cast<int>(std::min<int64_t>(total, 15 - log2es));
+  job.row0 = static_cast<long long>((addr - map_base) / 128);
+  int log2s = 0;
+  std::vector<SlabAxis> axes;
+  for (int d = ndim - 1; d >= m; --d) {
+    int const log2n = static_cast<int>(lv[d]);
+    int const nlev = static_cast<int>(lv[d] - lmin[d]);
+    if (nlev > 0) {
+      SlabAxis ax;
+      ax.log2n = static_cast<signed char>(log2n);
+      ax.log2s = static_cast<signed char>(log2s);
+      ax.nlevels = static_cast<signed char>(nlev);
+      int log2r = std::min(log2n, 5);
+      if (log2s >= 1 && log2s <= 4 && log2n + log2s - 3 <= 8)
+        log2r = std::min(log2n, 3);
+      ax.log2r = static_cast<signed char>(log2r);
+      axes.push_back(ax);
+    }
+    log2s += log2n;
+  }
+  std::reverse(axes.begin(), axes.end());
+  job.naxes = static_cast<int>(axes.size());
+  for (size_t i = 0; i < axes.size(); ++i) job.axis[i] = axes[i];
+  return job;
+}
+
+// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
+// against libcuda): a 2D view [rows][128 bytes] from `base`, 1 KB boxes
+// (8 rows), 128-byte swizzle.
+bool encode_slab_map(CUtensorMap *map, unsigned long long base,
+                     unsigned long long rows, size_t es) {
+  auto const encode = tensor_map_encoder();
+  if (encode == nullptr) return false;
+  if (rows == 0 || rows > (1ULL << 31)) return false;
+  cuuint64_t dims[2] = {static_cast<cuuint64_t>(128 / es), rows};
+  cuuint64_t strides[1] = {128};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / es), 8};
+  cuuint32_t elem[2] = {1, 1};
+  CUresult const r = encode(
+      map, es == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64
+                   : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+      2, reinterpret_cast<void *>(base), dims, strides, box, elem,
+      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS;
+}
+
+void launch_slab(int dtype, int sched, SlabParams const &p, cudaStream_t s) {
+  switch (dtype) {
+  case PALIWA_GB_F64: return launch_slab_f64(sched, p, s);
+  case PALIWA_GB_F32: return launch_slab_f32(sched, p, s);
+  case PALIWA_GB_F32C: return launch_slab_f32c(sched, p, s);
+  }
+  throw StatusError(PALIWA_GB_INVALID_ARGUMENT, "unknown dtype");
+}
+
+// Measured, one call (us, hat / CDF (2,2)), slab against axis by axis:
+// launches are what small grids spend their time on (FP32 4^6 15 against 31,
+// FP32c 32^2 x 64 17 / 21 against 22 / 23, FP64 16^3 14 / 21 against 24 / 31).
+// Floats gain up to about 2^22 points (FP32c 1024 x 64 x 64 35 / 42 against 37
+// / 46; 4096 x 64 x 64 131 / 155 against 122 / 155). FP32 gains again where
+// the axes no longer run out of L2 (2^26 points: 341 / 363 against 370 / 377;
+// 2^24: 106 / 114 against 100 / 108). One SM's FP64 pipe holds doubles to
+// 2^13 points on three or more axes and 2^11 on two (64 x 64: 16 / 27 against
+// 17 / 21).
+int single_slab_start(int dtype, int ndim, int64_t const *level,
+                      int64_t const *lmin, void const *grid) {
+  auto const addr = reinterpret_cast<unsigned long long>(grid);
+  int64_t total = 0;
+  int axes = 0;
+  for (int d = 0; d < ndim; ++d) {
+    total += level[d];
+    axes += level[d] > lmin[d];
+  }
+  bool gain = false;
+  switch (dtype) {
+  case PALIWA_GB_F64: gain = total <= (axes >= 3 ? 13 : 11); break;
+  case PALIWA_GB_F32C: gain = total <= 22; break;
+  case PALIWA_GB_F32: gain = total <= 22 || total >= 26; break;
+  }
+  if (!gain || addr % 128 != 0 || tensor_map_encoder() == nullptr) return ndim;
+  return slab_start(dtype, ndim, level, lmin, addr, addr);
+}
+
+bool launch_single_slab(int dtype, int ndim, int m, int64_t const *level,
+                        int64_t const *lmin, void *grid, int sched,
+                        cudaStream_t s) {
+  auto const addr = reinterpret_cast<unsigned long long>(grid);
+  size_t const es = dtype_size(dtype);
+  int64_t total = 0;
+  for (int d = 0; d < ndim; ++d) total += level[d];
+  SlabParams p;
+  std::memset(&p, 0, sizeof(p));
+  if (!encode_slab_map(&p.map, addr, (es << total) / 128, es)) return false;
+  p.job = slab_job(dtype, ndim, m, level, lmin, addr, addr);
+  p.njobs = 1;
+  p.total_tiles = 1LL << (total - p.job.log2_tile);
+  check_stage_errors();
+  p.error = stage_error_word();
+  launch_slab(dtype, sched, p, s);
+  return true;
+}
+
+} // namespace pgb

@@ -322,6 +322,8 @@ namespace {
 // stream capture: the allocation is not part of the captured work).
 std::atomic<unsigned *> g_error_word{nullptr};
 
+} // namespace
+
 unsigned *stage_error_word() {
   unsigned *word = g_error_word.load(std::memory_order_acquire);
   if (word != nullptr) return word;
@@ -342,8 +344,6 @@ unsigned *stage_error_word() {
   g_error_word.store(word, std::memory_order_release);
   return word;
 }
-
-} // namespace
 
 void check_stage_errors() {
   unsigned volatile *const word = g_error_word.load(std::memory_order_acquire);

@@ -58,6 +58,9 @@ void launch_twide_table_f64(bool exact, int sched, int code,
 void launch_stage(int dtype, bool exact, bool symmetric, int ws,
                   LiftParams const &params, Stage const &st, cudaStream_t s);
 
+// The error word of single-grid launches (see check_stage_errors).
+unsigned *stage_error_word();
+
 // Throws PALIWA_GB_TIMEOUT (and clears the flag) when a bounded wait of a
 // single-grid launch gave up since the last call.
 void check_stage_errors();
