@@ -203,9 +203,9 @@ int paliwa_gb_dump_to_binary_file(const void *data, int64_t bytes,
  * where a library allocation can fail or fragment it, and time-step loops
  * that cannot pay for allocator calls or cudaFree's device synchronization.
  * Only grids with a pencil longer than 4096 points need scratch; this entry
- * point takes it from one 64 MiB array in device memory that every GPU
- * loading the library holds until the process exits, so such grids may be at
- * most 64 MiB (larger ones return PALIWA_GB_INVALID_ARGUMENT before any work
+ * point takes it from one 64 MiB array in device memory (and 8 MiB more for
+ * FP32c) that every GPU loading the library holds until the process exits, so
+ * such grids may be at most 64 MiB (larger ones return PALIWA_GB_INVALID_ARGUMENT before any work
  * is queued). The first call on each device looks up that array's address
  * (cudaGetSymbolAddress) with the device current; make it before any stream
  * capture. All calls share the array, which keeps the last call's contents

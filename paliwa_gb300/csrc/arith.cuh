@@ -314,6 +314,20 @@ struct RowF32C {
   }
 };
 
+// Two columns as double-float pairs in memory, unrounded (high parts, low
+// parts): what the windows and the coarse levels of a long pencil hand each
+// other.
+struct RowDF : RowF32C {
+  using Store = uint4;
+  using Elem = double;  // 8 bytes per column
+  static __device__ __forceinline__ V load(Store u) {
+    return {f2_bits(u.x, u.y), f2_bits(u.z, u.w)};
+  }
+  static __device__ __forceinline__ Store store(V v) {
+    return {f2_lo(v.h), f2_hi(v.h), f2_lo(v.l), f2_hi(v.l)};
+  }
+};
+
 // Plain<double, true> on two columns.
 struct F64Row2 {
   double x, y;

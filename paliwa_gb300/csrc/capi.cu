@@ -412,8 +412,9 @@ bool box_windows(AxisView const &v, size_t npasses) {
 
 // Fine levels of a long pencil on overlapping windows: of 4096 points on the
 // staged kernel, or (box) of 512 on the TMA wide kernel's boxed form.
+// With `heads` (FP32c), the windows hand their chunk heads on unrounded.
 void plan_windows(AxisView const &v, std::vector<int> const &shifts,
-                  std::vector<Filter> const &filters, bool box,
+                  std::vector<Filter> const &filters, bool box, bool heads,
                   std::vector<Stage> &out) {
   int const log2_window = box ? kBoxWindowLog2 : kWindowLog2;
   long long const window = 1LL << log2_window;
@@ -472,6 +473,7 @@ void plan_windows(AxisView const &v, std::vector<int> const &shifts,
     st.job.periodic = 0;
     st.job.log2_window = log2_window;
     st.tma = st.box = box;
+    st.heads = heads ? v.heads : 0;
     st.job.seg_len = static_cast<int>(seg_len);
     st.job.halo = static_cast<int>(halo);
     st.job.col_tiles = ceil_div(v.columns, C);
@@ -479,6 +481,33 @@ void plan_windows(AxisView const &v, std::vector<int> const &shifts,
     out.push_back(st);
     first += count;
   }
+}
+
+// The coarse levels (shifts in units of 16 points) of FP32c pencils whose
+// heads lie as double-float pairs in v.heads, and the copy of the heads to
+// the grid after them (forward) or from it before them.
+void plan_heads(AxisView const &v, std::vector<int> const &shifts,
+                bool forward, std::vector<Stage> &out) {
+  Stage copy;
+  copy.R = forward ? kHeadsOut : kHeadsIn;
+  copy.job = make_job(v, shifts, 0, 0);
+  copy.job.halo_base = v.heads;
+  Stage st;
+  AxisView h = v;
+  h.base = v.heads;
+  h.log2_n = v.log2_n - 4;
+  h.log2_kstride = v.log2_inner;
+  h.log2_astride = h.log2_n + v.log2_inner;
+  int const log2G = h.log2_n - 4;
+  st.R = kHeadsTile + (log2G <= 5 ? kTile : kTileLong) + 16;
+  st.job = make_job(h, shifts, 0, shifts.size());
+  st.job.periodic = 1;
+  st.job.log2_window = h.log2_n;
+  st.job.col_tiles = ceil_div(h.columns >> 1, kThreads >> log2G);
+  st.tiles = st.job.col_tiles;
+  if (forward) out.push_back(st);
+  out.push_back(copy);
+  if (!forward) out.push_back(st);
 }
 
 } // namespace
@@ -503,14 +532,21 @@ void plan_axis(AxisView const &view, std::vector<int> const &shifts,
   bool const ordered = shifts.size() <= kMaxLevels &&
                        (canonical_shifts(order, true) ||
                         canonical_shifts(order, false));
-  // Not FP32c: it rounds to its storage between the two kinds of stages, so
-  // an earlier split would round more points twice.
-  bool const box =
-      ordered && !view.wide_last && box_windows(view, filters.size());
+  // FP32c rounds to its storage between the two kinds of stages: it takes
+  // that split only where the windows hand the sub-lattice on unrounded, in a
+  // buffer of its own that the tile kernel transforms (512 to 4096 heads) and
+  // rounds where the other split does.
+  int const ws = wavelet_schedule(filters);
+  bool const heads = view.wide_last && view.heads != 0 && ws >= 0 && ordered &&
+                     canonical_shifts(order, (ws & 1) != 0) &&
+                     view.log2_n <= 16 && box_windows(view, filters.size());
+  bool const box = heads || (ordered && !view.wide_last &&
+                             box_windows(view, filters.size()));
   int const budget = box ? kBoxHalo : kHaloBudget;
   int m = 0;
   while (static_cast<long long>(P) * ((2LL << m) - 1) <= budget) ++m;
   if (m < 1) m = 1;
+  if (heads) m = 4;  // one head per chunk of 16 points
   size_t i = 0;
   while (i < shifts.size()) {
     bool const fine = shifts[i] < m;
@@ -518,7 +554,11 @@ void plan_axis(AxisView const &view, std::vector<int> const &shifts,
     while (j < shifts.size() && (shifts[j] < m) == fine) ++j;
     std::vector<int> run(shifts.begin() + i, shifts.begin() + j);
     if (fine) {
-      plan_windows(view, run, filters, box, out);
+      plan_windows(view, run, filters, box, heads && run.size() < shifts.size(),
+                   out);
+    } else if (heads) {
+      for (int &s : run) s -= m;
+      plan_heads(view, run, (ws & 1) != 0, out);
     } else {
       AxisView sub = view;
       sub.log2_n = view.log2_n - m;
@@ -626,11 +666,15 @@ void transform_axis(void *grid, int dtype, int ndim, int64_t const *level,
                             level, dim, dtype);
   void *shadow = nullptr;
   if (needs_shadow(view, shifts)) {
-    // Stream-ordered scratch for the windowed stages of long pencils.
+    // Stream-ordered scratch for the windowed stages of long pencils: the
+    // halo buffer and, for FP32c, the heads' buffer after it.
     size_t bytes = dtype_size(dtype);
     for (int d = 0; d < ndim; ++d) bytes <<= level[d];
-    cuda_check(cudaMallocAsync(&shadow, bytes, s), "cudaMallocAsync(shadow)");
+    size_t const heads = dtype == PALIWA_GB_F32C ? bytes / 8 : 0;
+    cuda_check(cudaMallocAsync(&shadow, bytes + heads, s),
+               "cudaMallocAsync(shadow)");
     view.shadow = reinterpret_cast<unsigned long long>(shadow);
+    if (heads != 0) view.heads = view.shadow + bytes;
   }
   try {
     std::vector<Stage> stages;

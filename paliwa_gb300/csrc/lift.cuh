@@ -376,6 +376,7 @@ struct FilterTable {
 // WaveletSched, and each pass takes its parity and coefficients from the
 // table (one uniform branch per pass).
 template <bool FWD> struct TableSched {
+  static constexpr bool kForward = FWD;
   static constexpr bool kTable = true;
 
   template <class A, int R, int K, class Ctx>

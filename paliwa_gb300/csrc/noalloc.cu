@@ -27,7 +27,9 @@ constexpr size_t kStaticScratchBytes = size_t(64) << 20;  // 64 MiB
 // Every GPU that loads the library holds this array until the process exits.
 // All calls share it and it keeps the last call's contents; the transform
 // writes every byte it later reads, so nothing needs clearing between calls.
-static __device__ __align__(256) unsigned char g_scratch[kStaticScratchBytes];
+// (An eighth more for the chunk heads of FP32c windows.)
+static __device__ __align__(256) unsigned char
+    g_scratch[kStaticScratchBytes + kStaticScratchBytes / 8];
 
 std::mutex g_scratch_mutex;
 std::array<void *, 256> g_scratch_address{};  // by device ordinal
@@ -110,6 +112,8 @@ extern "C" int paliwa_gb_transform_noalloc(void *grid, int dtype, int ndim,
                   "much scratch; the allocation-free transform holds at most "
                   "67108864 bytes (64 MiB)");
         view.shadow = reinterpret_cast<unsigned long long>(scratch_address());
+        if (dtype == PALIWA_GB_F32C)
+          view.heads = view.shadow + kStaticScratchBytes;
       }
       plan_axis(view, shifts, filters, plans[d]);
     }

@@ -42,6 +42,9 @@ struct AxisView {
   // Byte address of a buffer with the grid's size and layout that holds the
   // windowed stages' halos (pencils longer than one CTA holds; 0: none).
   unsigned long long shadow = 0;
+  // Byte address of a buffer of an eighth of the grid's size for the chunk
+  // heads of FP32c windows as double-float pairs (0: none).
+  unsigned long long heads = 0;
   long long columns = 1;        // outer * inner
   int log2_inner = 0;
   int log2_kstride = 0;  // element stride between consecutive pencil points
@@ -71,6 +74,12 @@ constexpr int kTile = 192;
 constexpr int kTileLong = 256;
 // Stage::R of a halo pass (halo_kernel) before a windowed stage.
 constexpr int kHalo = 512;
+// Stage::R of the copies between a grid's chunk heads and the buffer that
+// holds them as double-float pairs, and (plus kTile or kTileLong + 16) of the
+// coarse levels' stage on that buffer.
+constexpr int kHeadsIn = 4096;
+constexpr int kHeadsOut = 4097;
+constexpr int kHeadsTile = 8192;
 
 // One stage of an axis transform: a job for one kernel. The stages of one
 // axis must run in order; stages of different grids are independent.
@@ -91,6 +100,10 @@ struct Stage {
   // their own, and windows of 2^kBoxWindowLog2 points.
   bool box = false;
   bool table = false;  // a caller's filters (no wavelet's levels)
+  // Windows that hand their chunk heads on unrounded (in a buffer at
+  // `heads`), the stage of the coarse levels on that buffer, and its copies
+  // from and to the grid (R = kHeadsIn, kHeadsOut).
+  unsigned long long heads = 0;
 };
 
 constexpr int kWindowLog2 = 12;   // points per column per CTA round (4096)
@@ -156,6 +169,8 @@ LiftParams launch_params(std::vector<Filter> const &filters);
 // `jobs`, or the inline job of `params` when jobs == nullptr).
 // sched: 2 * wavelet + forward for the compile-time wavelet schedule (every
 // job's shifts must be canonical), or -1 for the runtime schedule.
+void launch_heads(int sched, int R, LiftParams params, long long total_tiles,
+                  cudaStream_t s);
 void launch_lift(int dtype, bool exact, bool symmetric, int sched, int R,
                  LiftParams params, LiftJob const *jobs, int njobs,
                  long long total_tiles, cudaStream_t stream);

@@ -80,6 +80,7 @@ constexpr int kTWide32Pairs = 226;
 // 32-point chunks of doubles.
 constexpr int kTWideBox = 192;
 constexpr int kTWide32Box = 227;
+constexpr int kTWideBoxHeads = 240;  // windows of FP32c grids with heads
 
 struct TWideJob {
   long long tile_begin;  // first tile of this job in the launch
@@ -119,6 +120,10 @@ struct TWideParams {
   TWideJob job;
   CUtensorMap map[2];
   FilterTable filters;  // read by TableSched launches
+  // Windows of FP32c pencils: the chunk heads as double-float pairs,
+  // [outer][n / 16][inner / 2] (see twide_box_kernel).
+  uint4 *heads;
+  long long head_columns;  // the pencils' columns
 };
 
 // The levels of one chunk under the launch's schedule.

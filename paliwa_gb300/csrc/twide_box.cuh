@@ -23,6 +23,13 @@
 // the grid) and not stored; the levels run as on a periodic pencil, which
 // reaches only points outside the segment's dependency cone.
 //
+// HEADS (FP32c windows): the chunk heads, every 16th point of the pencil, are
+// the points of the coarse levels' stage. A forward window also writes its
+// segment's heads to p.heads as unrounded double-float pairs, and an inverse
+// window takes its heads from there: rounding every 16th point to its storage
+// between the two stages would be eight times the rounding of the staged
+// kernel's split at every 128th.
+//
 // The CTA is warp-specialised as twide_kernel's, with one CTA of 512 (doubles
 // 256) transform threads per SM and three tiles in flight. Lane b of the
 // producer warp issues the tile's box b, load and store.
@@ -45,7 +52,7 @@ template <int R> constexpr size_t box_smem_bytes() {
   return size_t(kBoxStages) * (kBoxRows / R) * box_bytes_padded(R) + 1024;
 }
 
-template <class A, int R, class Sched>
+template <class A, int R, class Sched, bool HEADS>
 __global__ void __launch_bounds__(box_threads(R) + 32, 1)
     twide_box_kernel(__grid_constant__ const TWideParams p) {
   using V = typename A::V;
@@ -183,9 +190,44 @@ __global__ void __launch_bounds__(box_threads(R) + 32, 1)
     return;
   }
 
+  // HEADS: this thread's head in tile k (nullptr past the last column; own:
+  // of the tile's segment). A launch with heads has one job of 512-point
+  // windows (32 chunks, one block per tile): chunk = lane, column = warp.
+  auto head_of = [&](long long k, bool &own) -> uint4 * {
+    TWideJob const &job = p.job;
+    long long const tile = first + k * step;
+    int const seg = static_cast<int>(tile / job.win.col_tiles);
+    long long const ct =
+        tile - static_cast<long long>(seg) * job.win.col_tiles;
+    long long const col = (ct << 5) + 2 * (t >> 5);
+    long long const z = col >> job.log2_inner;
+    int const x = static_cast<int>(col & ((1LL << job.log2_inner) - 1));
+    int const w = lane << LOG2R;
+    int y = seg * job.win.seg_len - job.win.halo + w;
+    int const n = 1 << job.win.log2_full;
+    own = static_cast<unsigned>(w - job.win.halo) <
+              static_cast<unsigned>(job.win.seg_len) &&
+          y < n;
+    y &= n - 1;
+    if (col >= p.head_columns) return nullptr;
+    return p.heads +
+           ((((z << (job.win.log2_full - LOG2R)) + (y >> LOG2R))
+             << (job.log2_inner - 1)) +
+            (x >> 1));
+  };
+
   // Transform threads.
   for (long long k = 0; k < ntiles; ++k) {
     int const b = static_cast<int>(k % S);
+    uint4 *head = nullptr;
+    bool own = false;
+    uint4 head_in = {};
+    if constexpr (HEADS) {
+      head = head_of(k, own);
+      // (the load runs while the tile's boxes land)
+      if constexpr (!Sched::kForward)
+        if (head != nullptr) head_in = *head;
+    }
     bool const ok = mbar_wait_bounded(
         &full[b], static_cast<unsigned>((k / S) & 1), abort);
     // A warp leaves as a whole (its lanes exchange by shuffles).
@@ -217,9 +259,12 @@ __global__ void __launch_bounds__(box_threads(R) + 32, 1)
       for (int j = 0; j < R; ++j)
         v[j] = A::load(
             *reinterpret_cast<W const *>(mine + j * 128 + piece[j & 7]));
+      if constexpr (HEADS && !Sched::kForward) v[0] = RowDF::load(head_in);
       RoundCtx<A, NT, true> ctx(t, c, 1 << log2G, log2G, lane, 1, nullptr,
                                 nullptr, log2ls);
       twide_levels<Sched, A, R, NT>(v, ctx, job.nlevels, p);
+      if constexpr (HEADS && Sched::kForward)
+        if (own && head != nullptr) *head = RowDF::store(v[0]);
 #pragma unroll
       for (int j = 0; j < R; ++j)
         *reinterpret_cast<W *>(mine + j * 128 + piece[j & 7]) =

@@ -12,7 +12,7 @@ template <class A, int R, class Sched, int FORM>
 void launch_twide_r(TWideParams const &p, cudaStream_t s) {
   static thread_local Occupancy occ;
   constexpr bool kLong = FORM == 2 || FORM == 5;
-  constexpr bool kBox = FORM == 6;
+  constexpr bool kBox = FORM >= 6;  // 7: with heads
   constexpr int kBlock = kLong  ? kTWideThreads
                          : kBox ? box_threads(R) + 32
                                 : twide_threads(R) + 32;
@@ -20,7 +20,7 @@ void launch_twide_r(TWideParams const &p, cudaStream_t s) {
     if constexpr (kLong)
       return twide_long_kernel<A, Sched, FORM == 5>;
     else if constexpr (kBox)
-      return twide_box_kernel<A, R, Sched>;
+      return twide_box_kernel<A, R, Sched, FORM == 7>;
     else
       return twide_kernel<A, R, Sched, FORM>;
   }();
@@ -68,6 +68,10 @@ void launch_twide_rows(int code, TWideParams const &p, cudaStream_t s) {
   case kTWideLong + 16: return launch_twide_r<A, 16, Sched, 2>(p, s);
   case kTWideLongContig + 16: return launch_twide_r<A, 16, Sched, 5>(p, s);
   case kTWideBox + 16: return launch_twide_r<A, 16, Sched, 6>(p, s);
+  case kTWideBoxHeads + 16:
+    if constexpr (std::is_same<A, RowF32C>::value)
+      return launch_twide_r<A, 16, Sched, 7>(p, s);
+    break;
   case kTWide32Chunked:
     if constexpr (sizeof(typename A::V) <= 8)  // plain floats
       return launch_twide_r<A, 32, Sched, 1>(p, s);

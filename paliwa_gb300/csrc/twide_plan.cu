@@ -53,7 +53,9 @@ int twide_chunk(LiftJob const &job, int dtype, bool table) {
 
 int twide_code(Stage const &st, int dtype) {
   if (st.box)
-    return dtype == PALIWA_GB_F64 ? kTWide32Box : kTWideBox + 16;
+    return dtype == PALIWA_GB_F64 ? kTWide32Box
+           : st.heads != 0        ? kTWideBoxHeads + 16
+                                  : kTWideBox + 16;
   int const r = st.tma ? twide_chunk(st.job, dtype, st.table) : 0;
   if (r == 0) return 0;
   int const log2G = st.job.log2_n - (31 - __builtin_clz(r));
@@ -77,7 +79,7 @@ int twide_code(Stage const &st, int dtype) {
 // (FP32 n = 128 at 2^12 4.1 against 6.7).
 bool twide_enough(int code, int dtype, long long points) {
   bool const longer =
-      code == kTWideBox + 16 || code == kTWide32Box || code == kTWide32Chunked || code == kTWideChunked + 16 ||
+      code == kTWideBoxHeads + 16 || code == kTWideBox + 16 || code == kTWide32Box || code == kTWide32Chunked || code == kTWideChunked + 16 ||
       code == kTWideLong + 16 || code == kTWideLongContig + 16;
   return longer || points >= (dtype == PALIWA_GB_F64 ? 1LL << 12 : 1LL << 13);
 }
@@ -358,9 +360,16 @@ void launch_stage(int dtype, bool exact, bool symmetric, int ws,
                   LiftParams const &params, Stage const &st, cudaStream_t s) {
   int const sched =
       ws >= 0 && canonical_shifts(st.job, (ws & 1) != 0) ? ws : -1;
+  if (st.R >= kHeadsIn) {
+    LiftParams p = params;
+    p.job = st.job;
+    return launch_heads(sched, st.R, p, st.tiles, s);
+  }
   if (st.tma) {
     TWideParams p;
     std::memset(&p, 0, sizeof(p));
+    p.heads = reinterpret_cast<uint4 *>(st.heads);
+    p.head_columns = st.job.columns;
     int tsched = sched;
     if (sched < 0) {
       tsched = kTableSched + (canonical_shifts(st.job, true) ? 1 : 0);
@@ -376,6 +385,9 @@ void launch_stage(int dtype, bool exact, bool symmetric, int ws,
       p.error = stage_error_word();
       return launch_twide(dtype, exact, tsched, code, p, s);
     }
+    if (st.heads != 0)
+      throw StatusError(PALIWA_GB_CUDA_ERROR,
+                        "the tensor map of a windowed stage was refused");
   }
   LiftParams p = params;
   p.job = st.job;

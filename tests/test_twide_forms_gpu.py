@@ -151,3 +151,31 @@ def test_pencils_spread_over_pages(mode, level):
         torch.cuda.synchronize()
         exp = want(x, level, lo, "biorthogonal", forward, mode)
         assert np.array_equal(g.cpu().numpy(), exp), forward
+
+
+@pytest.mark.parametrize("level,lmin", [
+    ((13, 7), 0), ((15, 5), 3), ((16, 5), 11), ((14, 8), 10), ((2, 13, 6), 0),
+    ((13, 8), 12)])
+def test_long_compensated_pencils(level, lmin):
+    """FP32c pencils of 2^13 to 2^16 points in the boxed windows, whose heads
+    go to the coarse levels unrounded and are rounded where the staged
+    kernel's windows end: the bits of that plan (a batch's), forward and
+    inverse."""
+    import torch
+    from paliwa_gb300 import ct as pct
+    dim = 0 if len(level) == 2 else 1
+    lo = tuple(lmin if d == dim else l for d, l in enumerate(level))
+    rng = np.random.default_rng(sum(level))
+    x = rng.uniform(-1, 1, 1 << sum(level)).astype(np.float32)
+    for wavelet in WAVELETS:
+        for forward in (True, False):
+            g = torch.from_numpy(x).cuda()
+            f = pg.hierarchize if forward else pg.dehierarchize
+            f(g, level, lo, level, wavelet, compensated=True)
+            b = torch.from_numpy(x).cuda()
+            batch = pct.Batch([b], [level], lo, level, wavelet,
+                              compensated=True)
+            (batch.hierarchize if forward else batch.dehierarchize)()
+            torch.cuda.synchronize()
+            assert torch.equal(g, b), (wavelet, forward)
+            batch.close()
