@@ -302,7 +302,7 @@ KernelSet periodic_kernels(AxisView const &v, bool canon, bool ordered) {
       k.dflt = kChooseTmaWide;
     // A caller's filters otherwise run on the staged or direct kernel, which
     // read every step's distance, parity and coefficients (FP32 n = 512,
-    // 256 columns, four passes of CDF 9/7: 2830 against 1620 GB/s).
+    // 256 columns, four passes of CDF 9/7: 4030 against 1620 GB/s).
     if (!canon && !pages) k.dflt = kChooseTmaWide;
   }
   return k;

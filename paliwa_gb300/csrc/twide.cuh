@@ -175,19 +175,22 @@ __device__ __forceinline__ void fence_tensormap(void const *map) {
 // A tile is kUnits units of Ct * n * 4 = (2 NT / G) * (G R) * 4 bytes
 // (16 KB tiles for chunks of up to 8 points: per-tile synchronisation
 // dominated 8 KB ones); kStages tile buffers per CTA.
-template <int R> struct TWideShape {
+// 32-point chunks under a caller's filters take two buffers, for three CTAs
+// per SM (256 x 512 x 256 FP32, CDF 9/7: 4030 against 3120 GB/s); under a
+// wavelet's schedule three are faster (FP32 n = 1024 5180 against 4740).
+template <int R, bool TABLE = false> struct TWideShape {
   static constexpr int kUnits = R >= 8 ? 1 : 8 / R;
   static constexpr int kUnitBytes = 8 * twide_threads(R) * R;
   static constexpr int kTileBytes = kUnits * kUnitBytes;
-  static constexpr int kStages = R >= 16 ? 3 : 4;
+  static constexpr int kStages = R >= 32 && TABLE ? 2 : R >= 16 ? 3 : 4;
   static constexpr size_t kSmemBytes =
       size_t(kStages) * kTileBytes + 1024;  // + 1024-byte alignment slack
 };
 
 // The long form also holds the exchange buffers of its chunk heads (NT rows)
 // and fine steps (2 NT rows).
-template <int R, bool LONG> constexpr size_t twide_smem_bytes() {
-  return TWideShape<R>::kSmemBytes + (LONG ? 3 * kTWideThreads * 16 : 0);
+template <int R, bool LONG, bool TABLE> constexpr size_t twide_smem_bytes() {
+  return TWideShape<R, TABLE>::kSmemBytes + (LONG ? 3 * kTWideThreads * 16 : 0);
 }
 
 __device__ __forceinline__ void tma_load_5d(void *dst, void const *map,
@@ -260,7 +263,7 @@ __global__ void __launch_bounds__(twide_threads(R) + 32, R >= 16 ? 2 : 3)
   using W = typename A::Store;
   static_assert(sizeof(W) == 8, "rows of two float columns");
   constexpr int NT = twide_threads(R);
-  constexpr int S = TWideShape<R>::kStages;
+  constexpr int S = TWideShape<R, Sched::kTable>::kStages;
   constexpr int TILE = TWideShape<R>::kTileBytes;
   constexpr int U = TWideShape<R>::kUnits;
   constexpr int UNIT = TWideShape<R>::kUnitBytes;

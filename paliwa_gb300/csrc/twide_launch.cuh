@@ -25,7 +25,7 @@ void launch_twide_r(TWideParams const &p, cudaStream_t s) {
       return twide_kernel<A, R, Sched, FORM>;
   }();
   size_t const smem =
-      kBox ? box_smem_bytes<R>() : twide_smem_bytes<R, kLong>();
+      kBox ? box_smem_bytes<R>() : twide_smem_bytes<R, kLong, Sched::kTable>();
   int const dev = current_device();
   if (dev < 0 || dev >= Occupancy::kMaxDevices)
     throw StatusError(2, "device ordinal beyond the launch cache");

@@ -40,9 +40,10 @@ int twide_chunk(LiftJob const &job, int dtype, bool table) {
   if (n < 1 || n > (last ? 12 : 11)) return 0;
   // Plain floats: strided pencils of 1024 points in chunks of 32, which
   // exchange by shuffles (5200 GB/s against 3310-3870 in the long form and
-  // 3840-4650 on the tile kernel); with a caller's filters also those of 512
-  // (four passes: 3110 against 2830; CDF (2,2): 5470 against 5530).
-  if (dtype == PALIWA_GB_F32 && !last && (n == 10 || (n == 9 && table)))
+  // 3840-4650 on the tile kernel); with a caller's filters also those of 256
+  // and 512 (four passes, n = 512: 4030 against 2830; CDF (2,2): 5470 against
+  // 5530).
+  if (dtype == PALIWA_GB_F32 && !last && (n == 10 || (n >= 8 && n <= 9 && table)))
     return 32;
   if (n <= 4) return 1 << n;
   if (n <= 6 && !last) return 1 << (n - 2);
