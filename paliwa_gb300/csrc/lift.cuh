@@ -434,6 +434,15 @@ template <bool FWD> struct TableSched {
   }
 };
 
+// Policies whose loaded values have a zero low part (A::kLowZero).
+template <class A, class = void> struct LowZero {
+  static constexpr bool value = false;
+};
+template <class A>
+struct LowZero<A, typename std::enable_if<A::kLowZero>::type> {
+  static constexpr bool value = true;
+};
+
 // Schedule of hierarchize (FWD: levels fine to coarse, distances 1, 2, 4, ...)
 // and dehierarchize (coarse to fine) with a compile-time wavelet: the fine
 // levels are unrolled with compile-time distance, parity and coefficients.
@@ -444,35 +453,53 @@ template <int W, bool FWD> struct WaveletSched {
   static constexpr bool kTable = false;
   static constexpr bool kSplit = true;  // fine_only / coarse_only below
 
-  template <class A, int R, int NT, int K, class P, class Ctx>
+  // Pass I of P at level K. FRESH: the chunk's values are as loaded but for
+  // this call's levels. Then low parts are zero where no pass has written: at
+  // the finest level going forward, every point of the first pass and the
+  // written ones of the second; going back, at every level the odd points
+  // until the odd pass.
+  template <class A, int R, int NT, int K, int I, bool FRESH, class P,
+            class Ctx>
   static __device__ __forceinline__ void fine_pass(typename A::V (&v)[R],
                                                    Ctx &ctx) {
     using V = typename A::V;
     constexpr int S = 1 << K;
     constexpr Coeffs cf = P::coeffs();
+    constexpr bool Z = FRESH && LowZero<A>::value;
+    constexpr bool ZN =
+        Z && I == 0 && (FWD ? K == 0 : P::offset == 0);
+    constexpr bool ZM = Z && (FWD ? K == 0 : P::offset == 1);
+    auto update = [&](V lo, V me, V up) {
+      if constexpr (LowZero<A>::value)
+        return A::template update<P::c1one, ZN, ZM>(cf, lo, me, up);
+      else
+        return A::template update<P::c1one>(cf, lo, me, up);
+    };
     V const pub = P::offset == 1 ? v[0] : v[R - S];
     V const nb = ctx.fine_neighbor(P::offset, pub);
     if constexpr (P::offset == 1) {
 #pragma unroll
       for (int j = S; j < R; j += 2 * S) {
         V const up = (j + S < R) ? v[(j + S) % R] : nb;
-        v[j] = A::template update<P::c1one>(cf, v[j - S], v[j], up);
+        v[j] = update(v[j - S], v[j], up);
       }
     } else {
 #pragma unroll
       for (int j = 0; j < R; j += 2 * S) {
         V const lo = (j >= S) ? v[(j + R - S) % R] : nb;
-        v[j] = A::template update<P::c1one>(cf, lo, v[j], v[j + S]);
+        v[j] = update(lo, v[j], v[j + S]);
       }
     }
     ctx.fine_wrote_heads(P::offset);
   }
 
-  template <class A, int R, int NT, int K, class... P, class Ctx>
+  template <class A, int R, int NT, int K, bool FRESH = false, class P0,
+            class... P, class Ctx>
   static __device__ __forceinline__ void fine_level(typename A::V (&v)[R],
                                                     Ctx &ctx,
-                                                    PassList<P...>) {
-    (fine_pass<A, R, NT, K, P>(v, ctx), ...);
+                                                    PassList<P0, P...>) {
+    fine_pass<A, R, NT, K, 0, FRESH, P0>(v, ctx);
+    (fine_pass<A, R, NT, K, 1, FRESH, P>(v, ctx), ...);
   }
 
   template <class A, int R, int NT, class... P, class Ctx>
@@ -488,23 +515,23 @@ template <int W, bool FWD> struct WaveletSched {
      ...);
   }
 
-  template <class A, int R, int NT, int K, class Ctx>
+  template <class A, int R, int NT, int K, bool FRESH = false, class Ctx>
   static __device__ __forceinline__ void fine_up(typename A::V (&v)[R],
                                                  Ctx &ctx, int L) {
     if constexpr ((1 << K) < R) {
       if (K < L) {
-        fine_level<A, R, NT, K>(v, ctx, Passes{});
-        fine_up<A, R, NT, K + 1>(v, ctx, L);
+        fine_level<A, R, NT, K, FRESH>(v, ctx, Passes{});
+        fine_up<A, R, NT, K + 1, FRESH>(v, ctx, L);
       }
     }
   }
-  template <class A, int R, int NT, int K, class Ctx>
+  template <class A, int R, int NT, int K, bool FRESH = false, class Ctx>
   static __device__ __forceinline__ void fine_down(typename A::V (&v)[R],
                                                    Ctx &ctx,
                                                    int L) {
     if constexpr (K >= 0) {
-      if (K < L) fine_level<A, R, NT, K>(v, ctx, Passes{});
-      fine_down<A, R, NT, K - 1>(v, ctx, L);
+      if (K < L) fine_level<A, R, NT, K, FRESH>(v, ctx, Passes{});
+      fine_down<A, R, NT, K - 1, FRESH>(v, ctx, L);
     }
   }
 
@@ -624,7 +651,7 @@ template <int W, bool FWD> struct WaveletSched {
 #pragma unroll
     for (int k = 0; k < K; ++k) hv[k] = col[lane * K + k];
     RoundCtx<A, NT> hctx(lane, lane, 32, 5, lane, periodic, nullptr, nullptr);
-    run_levels<A, K, NT>(hv, hctx, Lc);
+    run_levels<A, K, NT, false>(hv, hctx, Lc);
 #pragma unroll
     for (int k = 0; k < K; ++k) col[lane * K + k] = hv[k];
   }
@@ -722,8 +749,9 @@ template <int W, bool FWD> struct WaveletSched {
     head = h1[0];
   }
 
-  // The L levels of a job (shifts 0 .. L-1 forward, L-1 .. 0 inverse).
-  template <class A, int R, int NT, class Ctx>
+  // The L levels of a job (shifts 0 .. L-1 forward, L-1 .. 0 inverse). FRESH:
+  // on values as loaded (but for coarser levels, going back).
+  template <class A, int R, int NT, bool FRESH = true, class Ctx>
   static __device__ __forceinline__ void run_levels(typename A::V (&v)[R],
                                                     Ctx &ctx,
                                                     int L) {
@@ -751,7 +779,7 @@ template <int W, bool FWD> struct WaveletSched {
       return;
     }
     if constexpr (FWD) {
-      fine_up<A, R, NT, 0>(v, ctx, L);
+      fine_up<A, R, NT, 0, FRESH>(v, ctx, L);
       if (L <= LOG2R || !coarse_heads<A, R, NT>(v[0], ctx, L - LOG2R))
         for (int sh = LOG2R; sh < L; ++sh)
           coarse_level<A, R, NT>(v, ctx, 1 << (sh - LOG2R), Passes{});
@@ -759,7 +787,7 @@ template <int W, bool FWD> struct WaveletSched {
       if (L <= LOG2R || !coarse_heads<A, R, NT>(v[0], ctx, L - LOG2R))
         for (int sh = L - 1; sh >= LOG2R; --sh)
           coarse_level<A, R, NT>(v, ctx, 1 << (sh - LOG2R), Passes{});
-      fine_down<A, R, NT, LOG2R - 1>(v, ctx, L);
+      fine_down<A, R, NT, LOG2R - 1, FRESH>(v, ctx, L);
     }
   }
 };
