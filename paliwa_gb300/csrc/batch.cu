@@ -684,7 +684,7 @@ void plan_combine(paliwa_gb_ct &ct, std::vector<CtSubspace> const &subs) {
   ct.params.order = ct.order_dev;
 }
 
-// The restrict's units of kCtUnit points (the grid of each) and every grid's
+// The restrict's units of ct_unit points (the grid of each) and every grid's
 // table of families: for the leading levels (s_1 .. s_{d-1}), 0 <= s <= l,
 // last dimension fastest, the first sparse point of (s_1 .. s_{d-1}, 0) and
 // the highest kept last level of the grid (a subspace's lower neighbours are
@@ -703,6 +703,7 @@ void plan_restrict(paliwa_gb_ct &ct, std::vector<CtSubspace> const &subs,
                        std::make_pair(ss.offset, -1)).first;
     it->second.second = std::max(it->second.second, s[nd - 1]);
   }
+  long long const unit = ct_unit(dtype_size(ct.dtype));
   std::vector<int> unit_grid;
   std::vector<long long> unit_first(ct.ngrids), first(ct.ngrids), table;
   for (int g = 0; g < ct.ngrids; ++g) {
@@ -711,7 +712,7 @@ void plan_restrict(paliwa_gb_ct &ct, std::vector<CtSubspace> const &subs,
     for (int d = 0; d < nd; ++d) total += lv[d];
     unit_first[g] = static_cast<long long>(unit_grid.size());
     unit_grid.insert(unit_grid.end(),
-                     ((1LL << total) + kCtUnit - 1) / kCtUnit, g);
+                     ((1LL << total) + unit - 1) / unit, g);
     first[g] = static_cast<long long>(table.size());
     std::fill(s.begin(), s.end(), 0);
     while (true) {

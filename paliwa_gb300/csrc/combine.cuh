@@ -67,7 +67,7 @@ struct CtParams {
   // Combine: its CTAs and the subspace ids they refer to.
   CtBlock const *blocks;
   int const *order;
-  // Restrict: the grid of every unit of kCtUnit points, each grid's first
+  // Restrict: the grid of every unit of ct_unit points, each grid's first
   // unit, and its families (see ct_restrict_kernel): families[
   // family_first[g] + index of (s_1 .. s_{d-1})].
   int const *unit_grid;
@@ -96,9 +96,17 @@ constexpr int kCtLog2Few = 3;
 inline int ct_max_subs(int log2p) {
   return log2p <= 1 ? 2 : log2p <= kCtLog2Few ? 4 : 8;
 }
-// Grid points per restrict CTA: kCtGroups groups of 4 per thread.
-constexpr int kCtGroups = 4;
-constexpr int kCtUnit = 4 * kCtGroups * kCtBlock;
+// Groups of 4 grid points per restrict thread (floats, doubles), and points
+// per CTA. Eight CTAs per SM (32 registers) hide the gathers: 4D |l|_1 = 19 -
+// q in floats 970 us, with the compiler's choice of six 1110, 2 groups 1176, 8
+// groups 1227; 17 - q in doubles 2 groups 289, 4 groups 372.
+__host__ __device__ constexpr int ct_groups(size_t element) {
+  return element == 8 ? 2 : 4;
+}
+__host__ __device__ constexpr int ct_unit(size_t element) {
+  return 4 * ct_groups(element) * kCtBlock;
+}
+constexpr int kCtRestrictCtas = 8;
 
 // A family is the subspaces (s_1 .. s_{d-1}, 0 .. top) of one leading level
 // vector; they lie one after another in the sparse grid. Packed as the first
@@ -319,8 +327,8 @@ __global__ void __launch_bounds__(kCtBlock)
 // Bound by memory: each grid is written once, in storage order, and the
 // sparse values are gathered. (Written from the sparse side, one thread per
 // sparse point over its grids, every store touched a 32-byte sector for 4
-// bytes: 4D |l|_1 = 19 - q 3.17 -> 1.11 ms, 20 - q 7.7 -> 2.6, 6D 16 - q
-// 2.65 -> 0.66.) Thread = 4 consecutive points 4 a .. 4 a + 3 of a last-axis row:
+// bytes: 4D |l|_1 = 19 - q 3.17 -> 0.97 ms, 20 - q 7.7 -> 2.3, 6D 16 - q
+// 2.65 -> 0.64.) Thread = 4 consecutive points 4 a .. 4 a + 3 of a last-axis row:
 // levels l, l - 1, l and, for 4 a, whatever its trailing zeros say, so a warp
 // gathers a few contiguous runs. The leading indices name the row's family,
 // whose first point and kept levels come from a table per grid. ND: the
@@ -394,8 +402,10 @@ template <typename I> struct CtRow {
 };
 
 template <typename S, int ND, typename I>
-__global__ void __launch_bounds__(kCtBlock)
+__global__ void __launch_bounds__(kCtBlock, kCtRestrictCtas)
     ct_restrict_kernel(CtParams const p) {
+  constexpr int GROUPS = ct_groups(sizeof(S));
+  constexpr int UNIT = ct_unit(sizeof(S));
   int const g = p.unit_grid[blockIdx.x];
   CtRows<ND, I> const rows(p, g);
   unsigned long long const base = p.grids[g].base;
@@ -407,13 +417,13 @@ __global__ void __launch_bounds__(kCtBlock)
   I const n = static_cast<I>(1) << total;
   int const l = rows.last();
   I const first =
-      static_cast<I>(blockIdx.x - p.unit_first[g]) * kCtUnit + 4 * threadIdx.x;
+      static_cast<I>(blockIdx.x - p.unit_first[g]) * UNIT + 4 * threadIdx.x;
   if (l >= 2) {
     bool const vec = (base & 15) == 0;
-    S v[kCtGroups][4];
-    unsigned keep[kCtGroups];
+    S v[GROUPS][4];
+    unsigned keep[GROUPS];
 #pragma unroll
-    for (int q = 0; q < kCtGroups; ++q) {
+    for (int q = 0; q < GROUPS; ++q) {
       I const f = first + q * 4 * kCtBlock;
       keep[q] = 0;
       if (f >= n) continue;
@@ -437,7 +447,7 @@ __global__ void __launch_bounds__(kCtBlock)
       }
     }
 #pragma unroll
-    for (int q = 0; q < kCtGroups; ++q) {
+    for (int q = 0; q < GROUPS; ++q) {
       S *const to = out + first + q * 4 * kCtBlock;
       if (keep[q] == 15u && vec) {
         constexpr int PER = 16 / sizeof(S);
@@ -456,7 +466,7 @@ __global__ void __launch_bounds__(kCtBlock)
     return;
   }
   // Rows of one or two points: each point has a row of its own.
-  for (int q = 0; q < kCtGroups; ++q)
+  for (int q = 0; q < GROUPS; ++q)
     for (int i = 0; i < 4; ++i) {
       I const f = first + q * 4 * kCtBlock + i;
       if (f >= n) continue;
