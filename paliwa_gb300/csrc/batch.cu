@@ -49,6 +49,7 @@ struct Launch {
   int njobs = 0;
   long long tiles = 0;
   long long points = 0;  // grid points stored by this launch
+  bool pairs = false;    // slab launches: some job is worth pairs
 };
 
 struct Direction {
@@ -375,6 +376,7 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
       slab_tiles.insert(slab_tiles.end(), tiles, L.njobs);
       L.tiles += tiles;
       L.points += 1LL << total;
+      L.pairs |= slab_pairs(job);
       all_slabs.push_back(job);
       ++L.njobs;
     }
@@ -450,6 +452,7 @@ void launch_one(paliwa_gb_batch &b, Direction &dr, Launch const &L,
   p.njobs = L.njobs;
   p.total_tiles = L.tiles;
   p.error = b.slab_error;
+  p.pairs = L.pairs;
   launch_slab(b.dtype, L.sched, p, s);
 }
 

@@ -25,7 +25,9 @@
 // G = n / R), so that consecutive threads take consecutive inner indices:
 // for s >= 32 a warp reads rows of 32 consecutive elements; for small s the
 // planner picks R (8 or less) so that the swizzle keeps the reads on
-// distinct banks; the contiguous last axis is read as 16-byte pieces. The G
+// distinct banks; the contiguous last axis is read as 16-byte pieces. Floats
+// along the other axes go in pairs of adjacent inner indices (one 8-byte row
+// per thread and point, f32x2 arithmetic; SlabAxis::pair). The G
 // chunks of a pencil exchange neighbours by warp shuffle when G s <= 32
 // (lanes s apart), else through shared memory with one barrier per pass.
 #pragma once
@@ -48,6 +50,7 @@ struct SlabAxis {
   signed char log2s;    // element stride of the pencil in the tile
   signed char nlevels;  // levels to run (shifts 0 .. nlevels - 1)
   signed char log2r;    // chunk size R = 2^log2r
+  signed char pair;     // a thread holds two adjacent inner indices (floats)
 };
 
 struct SlabJob {
@@ -66,6 +69,7 @@ struct SlabParams {
   long long total_tiles;
   unsigned *error;          // set to 1 when a bounded wait gives up
   int ctas_per_sm;          // cap on the launch's CTAs per SM (0: none)
+  int pairs;                // the kernel that honours SlabAxis::pair
   SlabJob job;              // jobs == nullptr: the launch's only job
 };
 
@@ -212,7 +216,8 @@ template <class A, int NT> struct SlabCtx {
 // axes whose chunks exchange by shuffle or not at all): the U chunks are
 // independent, so their level steps interleave and hide each other's
 // latencies (short pencils have few updates per chunk).
-template <class A, int R, int NT, class Sched, int U>
+// LAST: the contiguous last axis only.
+template <class A, int R, int NT, class Sched, int U, bool LAST>
 __device__ __forceinline__ void slab_items(unsigned char *tile, SlabAxis ax,
                                            int log2T, int t, int lane,
                                            typename A::V *heads,
@@ -221,7 +226,7 @@ __device__ __forceinline__ void slab_items(unsigned char *tile, SlabAxis ax,
   using S = typename A::Store;
   constexpr int ES = sizeof(S);
   constexpr int LOG2R = Log2<R>::value;
-  int const log2n = ax.log2n, log2s = ax.log2s;
+  int const log2n = ax.log2n, log2s = LAST ? 0 : ax.log2s;
   int const log2G = log2n - LOG2R;
   int const items = 1 << (log2T - LOG2R);
   bool const vec = log2s == 0 && R * ES >= 16;  // contiguous 16-byte pieces
@@ -258,7 +263,7 @@ __device__ __forceinline__ void slab_items(unsigned char *tile, SlabAxis ax,
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < R; ++j) v[u][j] = A::load(S(0));
+        for (int j = 0; j < R; ++j) v[u][j] = A::load(S{});
       }
     }
 #pragma unroll
@@ -291,16 +296,36 @@ __device__ __forceinline__ void slab_items(unsigned char *tile, SlabAxis ax,
   }
 }
 
+// Rows of two adjacent floats, with the same operations per column.
+template <class A> struct SlabPair {
+  using type = void;
+};
+template <> struct SlabPair<Plain<float, true>> {
+  using type = RowF32x2<true>;
+};
+template <> struct SlabPair<CompensatedSym> {
+  using type = RowF32C;
+};
+// The largest value an exchange buffer holds.
+template <class A, bool PAIRS> constexpr size_t slab_value_bytes() {
+  if constexpr (PAIRS)
+    return sizeof(typename SlabPair<A>::type::V);
+  else
+    return sizeof(typename A::V);
+}
+
 // One axis of a tile held in shared memory: every pencil, every level.
 // Chunks of up to 8 points run 2 or 4 per thread at once where the axis has
 // enough of them.
-template <class A, int R, int NT, class Sched>
+template <class A, int R, int NT, class Sched, bool LAST>
 __device__ __forceinline__ void slab_axis(unsigned char *tile, SlabAxis ax,
                                           int log2T, int t, int lane,
                                           typename A::V *heads,
                                           typename A::V *xch) {
   constexpr int LOG2R = Log2<R>::value;
-  constexpr int UMAX = R <= 4 ? 4 : (R <= 8 ? 2 : 1);
+  // (half as many of double-float pairs, which would spill)
+  constexpr int UMAX =
+      (R <= 4 ? 4 : (R <= 8 ? 2 : 1)) / (sizeof(typename A::V) >= 16 ? 2 : 1);
   int const log2G = ax.log2n - LOG2R;
   int const items = 1 << (log2T - LOG2R);
   // A pencil held by one thread (G == 1) exchanges nothing; otherwise its
@@ -308,26 +333,53 @@ __device__ __forceinline__ void slab_axis(unsigned char *tile, SlabAxis ax,
   bool const in_warp = log2G == 0 || log2G + ax.log2s <= 5;
   if constexpr (UMAX > 1) {
     if (in_warp && items >= UMAX * NT) {
-      slab_items<A, R, NT, Sched, UMAX>(tile, ax, log2T, t, lane, heads, xch,
-                                        true);
+      slab_items<A, R, NT, Sched, UMAX, LAST>(tile, ax, log2T, t, lane, heads,
+                                              xch, true);
       return;
     }
   }
-  slab_items<A, R, NT, Sched, 1>(tile, ax, log2T, t, lane, heads, xch,
-                                 in_warp);
+  slab_items<A, R, NT, Sched, 1, LAST>(tile, ax, log2T, t, lane, heads, xch,
+                                       in_warp);
+}
+
+// ... in pairs where the planner says so: the tile is then an array of pairs.
+template <class A, int R, int NT, class Sched, bool PAIRS>
+__device__ __forceinline__ void slab_axis_any(unsigned char *tile, SlabAxis ax,
+                                              int log2T, int t, int lane,
+                                              unsigned char *xbuf) {
+  using P = typename SlabPair<A>::type;
+  if constexpr (PAIRS) {
+    // (32-point chunks of double-float pairs would not fit the registers)
+    if constexpr (R * sizeof(typename P::V) <= 256) {
+      if (ax.pair) {
+        --ax.log2s;
+        auto *const heads = reinterpret_cast<typename P::V *>(xbuf);
+        slab_axis<P, R, NT, Sched, false>(tile, ax, log2T - 1, t, lane, heads,
+                                          heads + NT);
+        return;
+      }
+    }
+  }
+  auto *const heads = reinterpret_cast<typename A::V *>(xbuf);
+  // (FP32 in pairs has only the contiguous axis left to do here; without this
+  // 32 x 16 x 16 axes of 2^28 points measure 682 us instead of 647)
+  constexpr bool kLast =
+      PAIRS && std::is_same<A, Plain<float, true>>::value;
+  slab_axis<A, R, NT, Sched, kLast>(tile, ax, log2T, t, lane, heads,
+                                    heads + NT);
 }
 
 // Dynamic shared memory: the tile buffers (1 KB aligned for the swizzle,
 // plus 1 KB of alignment slack) and the chunk heads and exchange buffers.
-template <class A> constexpr size_t slab_smem_bytes() {
+template <class A, bool PAIRS> constexpr size_t slab_smem_bytes() {
   return size_t(kSlabStages) * kSlabTileBytes + kSlabBoxBytes +
-         3 * kSlabThreads * sizeof(typename A::V);
+         3 * kSlabThreads * slab_value_bytes<A, PAIRS>();
 }
 
-template <class A, class Sched>
+// PAIRS: some axis of the launch runs in pairs.
+template <class A, class Sched, bool PAIRS>
 __global__ void __launch_bounds__(kSlabThreads, 2)
     slab_kernel(__grid_constant__ const SlabParams p) {
-  using V = typename A::V;
   using S = typename A::Store;
   constexpr int NT = kSlabThreads;
   constexpr int ES = sizeof(S);
@@ -337,9 +389,7 @@ __global__ void __launch_bounds__(kSlabThreads, 2)
   unsigned char *const tiles =
       smem_raw + ((kSlabBoxBytes - (base_addr & (kSlabBoxBytes - 1))) &
                   (kSlabBoxBytes - 1));
-  V *const heads =
-      reinterpret_cast<V *>(tiles + kSlabStages * kSlabTileBytes);
-  V *const xch = heads + NT;
+  unsigned char *const xbuf = tiles + kSlabStages * kSlabTileBytes;
   __shared__ uint64_t full[kSlabStages];
   __shared__ SlabJob sjob[kSlabStages];
 
@@ -422,11 +472,26 @@ __global__ void __launch_bounds__(kSlabThreads, 2)
     for (int a = 0; a < job.naxes; ++a) {
       SlabAxis const ax = job.axis[a];
       switch (ax.log2r) {
-      case 1: slab_axis<A, 2, NT, Sched>(tile, ax, job.log2_tile, t, lane, heads, xch); break;
-      case 2: slab_axis<A, 4, NT, Sched>(tile, ax, job.log2_tile, t, lane, heads, xch); break;
-      case 3: slab_axis<A, 8, NT, Sched>(tile, ax, job.log2_tile, t, lane, heads, xch); break;
-      case 4: slab_axis<A, 16, NT, Sched>(tile, ax, job.log2_tile, t, lane, heads, xch); break;
-      case 5: slab_axis<A, 32, NT, Sched>(tile, ax, job.log2_tile, t, lane, heads, xch); break;
+      case 1:
+        slab_axis_any<A, 2, NT, Sched, PAIRS>(tile, ax, job.log2_tile, t,
+                                                 lane, xbuf);
+        break;
+      case 2:
+        slab_axis_any<A, 4, NT, Sched, PAIRS>(tile, ax, job.log2_tile, t,
+                                                 lane, xbuf);
+        break;
+      case 3:
+        slab_axis_any<A, 8, NT, Sched, PAIRS>(tile, ax, job.log2_tile, t,
+                                                 lane, xbuf);
+        break;
+      case 4:
+        slab_axis_any<A, 16, NT, Sched, PAIRS>(tile, ax, job.log2_tile, t,
+                                                 lane, xbuf);
+        break;
+      case 5:
+        slab_axis_any<A, 32, NT, Sched, PAIRS>(tile, ax, job.log2_tile, t,
+                                                 lane, xbuf);
+        break;
       default: break;
       }
       __syncthreads();  // the next axis reads what this one wrote

@@ -7,11 +7,11 @@
 
 namespace pgb {
 
-template <class A, class Sched>
-void launch_slab_r(SlabParams const &p, cudaStream_t s) {
+template <class A, class Sched, bool PAIRS>
+void launch_slab_k(SlabParams const &p, cudaStream_t s) {
   static thread_local Occupancy occ;
-  auto kernel = slab_kernel<A, Sched>;
-  size_t const smem = slab_smem_bytes<A>();
+  auto kernel = slab_kernel<A, Sched, PAIRS>;
+  size_t const smem = slab_smem_bytes<A, PAIRS>();
   int const dev = current_device();
   if (dev < 0 || dev >= Occupancy::kMaxDevices)
     throw StatusError(2, "device ordinal beyond the launch cache");
@@ -34,6 +34,13 @@ void launch_slab_r(SlabParams const &p, cudaStream_t s) {
   long long const blocks = std::min(p.total_tiles, resident);
   kernel<<<static_cast<unsigned>(blocks), kSlabThreads, smem, s>>>(p);
   cuda_check(cudaGetLastError(), "slab kernel launch");
+}
+
+template <class A, class Sched>
+void launch_slab_r(SlabParams const &p, cudaStream_t s) {
+  if constexpr (!std::is_void<typename SlabPair<A>::type>::value)
+    if (p.pairs) return launch_slab_k<A, Sched, true>(p, s);
+  launch_slab_k<A, Sched, false>(p, s);
 }
 
 // sched = 2 * wavelet + (forward ? 1 : 0).

@@ -11,6 +11,7 @@ int slab_start(int dtype, int ndim, int64_t const *level, int64_t const *lmin,
 SlabJob slab_job(int dtype, int ndim, int m, int64_t const *level,
                  int64_t const *lmin, unsigned long long addr,
                  unsigned long long map_base);
+bool slab_pairs(SlabJob const &job);
 bool encode_slab_map(CUtensorMap *map, unsigned long long base,
                      unsigned long long rows, size_t es);
 

@@ -152,3 +152,34 @@ def test_single_grids_with_slab_launches(mode, level, lmin):
                         1e-6 * np.max(np.abs(want))
                     continue
                 assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("dtype_name", ["f32", "f32c"])
+@pytest.mark.parametrize("level", [
+    (5, 6), (6, 6), (11, 1), (6, 5, 1), (1, 1, 10), (4, 8, 1), (5, 7, 2),
+    (12, 1, 2), (3, 3, 2, 2, 2), (1, 0, 12), (7, 6, 0), (9, 2, 4)])
+def test_pairs_of_floats_equal_the_per_axis_plan(dtype_name, level):
+    """Axes worked in pairs of adjacent inner indices: tiles of 2^11 points
+    (no pairs) and from 2^12, inner extents from one pair up, pencils of one
+    chunk, of chunks in one warp and of chunks that meet at barriers; bit for
+    bit the axis-by-axis plan, which holds no pairs in a slab."""
+    import torch
+    lmin = (0,) * len(level)
+    for w, wavelet in enumerate(WAVELETS):
+        _, out = run_pair([level], lmin, level, wavelet, torch.float32,
+                          dtype_name == "f32c", w)
+        (f1, b1, _, kernels), (f2, b2, _, _) = out
+        assert 1024 in kernels
+        assert torch.equal(f1, f2) and torch.equal(b1, b2)
+
+
+def test_pairs_only_where_tiles_are_large_enough():
+    """A launch of small and large tiles: the small grids go through the
+    kernel that works in pairs as well, with the same bits."""
+    import torch
+    levels = [(3, 2, 2), (6, 6, 3), (2, 5, 4), (5, 5, 5)]
+    for compensated in (False, True):
+        _, out = run_pair(levels, (0,) * 3, (6,) * 3, "biorthogonal",
+                          torch.float32, compensated, 5)
+        (f1, b1, _, _), (f2, b2, _, _) = out
+        assert torch.equal(f1, f2) and torch.equal(b1, b2)
