@@ -235,8 +235,13 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
       size_t shadow_off = b.group_shadow[grp];
       for (size_t i = 0; i < members.size(); ++i) {
         int const g = members[i];
-        if (d >= slab_from[g]) continue;  // in the grid's slab launch
         int64_t const *lv = levels + static_cast<size_t>(g) * b.ndim;
+        // In the grid's slab launch; a single axis there (slab_start) still
+        // has its class, and a kernel that is chosen for it (tuning) runs it.
+        int work = 0;
+        for (int k = 0; k < b.ndim; ++k) work += lv[k] > lmin[k];
+        bool const in_slab = d >= slab_from[g];
+        if (in_slab && (work > 1 || lv[d] == lmin[d])) continue;
         AxisView view =
             axis_view(reinterpret_cast<unsigned long long>(grid_ptrs[g]),
                       b.ndim, lv, d, b.dtype);
@@ -260,6 +265,15 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
             ci.dflt = st.dflt;
           }
           ci.points += st.job.columns << st.job.log2_n;
+        }
+        if (in_slab) {
+          bool chosen = false;
+          for (Stage const &st : stages[i])
+            chosen |= st.kernels != 0 && dr.tuning.choice.count(st.tclass) != 0;
+          if (chosen)
+            slab_from[g] = b.ndim;
+          else
+            stages[i].clear();
         }
         depth = std::max(depth, stages[i].size());
       }

@@ -11,9 +11,12 @@ namespace pgb {
 
 // The slab group of a grid: its trailing axes whose slab (the product of
 // their extents) fits one tile, when that group holds at least two axes
-// with levels to transform, the grid is a whole number of 1 KB boxes and
-// starts on a row of the tensor map (rows of 128 bytes from map_base).
-// Returns the group's first axis, or ndim for none.
+// with levels to transform, or one in a grid that is a single tile: a batch
+// then needs no launch of its own for it (there and back, us: FP64 6D |l|_1 =
+// 9 - q 59 -> 23, FP32 3D 75 -> 63). The grid is a whole number of 1 KB boxes
+// and starts on a row of the tensor map (rows of 128 bytes from map_base).
+// FP32c pencils of more than 4096 points are windows that round in between
+// (plan_axis), and stay so. Returns the group's first axis, or ndim for none.
 int slab_start(int dtype, int ndim, int64_t const *lv, int64_t const *lmin,
                unsigned long long addr, unsigned long long map_base) {
   int const log2es = dtype_size(dtype) == 8 ? 3 : 2;
@@ -25,8 +28,11 @@ int slab_start(int dtype, int ndim, int64_t const *lv, int64_t const *lmin,
   int64_t vol = 0;
   while (m > 0 && vol + lv[m - 1] + log2es <= 15) vol += lv[--m];
   int work = 0;
-  for (int d = m; d < ndim; ++d) work += lv[d] > lmin[d];
-  return work >= 2 && work <= kSlabMaxAxes ? m : ndim;
+  for (int d = m; d < ndim; ++d) {
+    work += lv[d] > lmin[d];
+    if (dtype == PALIWA_GB_F32C && lv[d] > 12) return ndim;
+  }
+  return work >= (m == 0 ? 1 : 2) && work <= kSlabMaxAxes ? m : ndim;
 }
 
 // The slab job of a grid for its axes m..ndim-1: per axis with levels to
@@ -152,7 +158,7 @@ int single_slab_start(int dtype, int ndim, int64_t const *level,
   case PALIWA_GB_F32C: gain = total <= 22; break;
   case PALIWA_GB_F32: gain = total <= 22 || total >= 26; break;
   }
-  if (!gain || addr % 128 != 0 || tensor_map_encoder() == nullptr) return ndim;
+  if (!gain || axes < 2 || addr % 128 != 0 || tensor_map_encoder() == nullptr) return ndim;
   return slab_start(dtype, ndim, level, lmin, addr, addr);
 }
 

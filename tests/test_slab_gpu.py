@@ -183,3 +183,52 @@ def test_pairs_only_where_tiles_are_large_enough():
                           torch.float32, compensated, 5)
         (f1, b1, _, _), (f2, b2, _, _) = out
         assert torch.equal(f1, f2) and torch.equal(b1, b2)
+
+
+@pytest.mark.parametrize("dtype_name", ["f64", "f32", "f32c"])
+def test_one_axis_of_a_single_tile_in_the_slab_launch(dtype_name):
+    """Grids of one tile with one axis to transform go in the slab launch of
+    the others, leading, middle and last axis alike, up to a whole tile; a
+    kernel chosen for their tuning class takes them out again. The bits are
+    the axis-by-axis plan's."""
+    import torch
+    top = 12 if dtype_name == "f64" else 13
+    levels = [(top, 0, 0), (0, top, 0), (0, 0, top), (9, 0, 1), (1, 8, 1),
+              (0, 2, 8), (4, 3, 3)]
+    lmin = [0, 0, 0]
+    dtype = torch.float64 if dtype_name == "f64" else torch.float32
+    for w, wavelet in enumerate(WAVELETS):
+        _, out = run_pair(levels, lmin, (top,) * 3, wavelet, dtype,
+                          dtype_name == "f32c", w)
+        (f1, b1, _, kernels), (f2, b2, _, _) = out
+        # (long FP32c pencils are windows that round in between)
+        assert 1024 in kernels
+        assert set(kernels) == {1024} or dtype_name == "f32c"
+        assert torch.equal(f1, f2) and torch.equal(b1, b2)
+    buf, views = pct.packed_grids(levels, dtype)
+    buf.copy_(torch.from_numpy(
+        np.random.default_rng(7).uniform(-1, 1, buf.numel())))
+    start = buf.clone()
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    bt = pct.Batch(views, levels, lmin, (top,) * 3, "hat",
+                   compensated=dtype_name == "f32c")
+    bt.hierarchize(s)
+    s.synchronize()
+    want = buf.clone()
+    code, _, names, chosen = next(
+        (r for r in bt.tuning(True) if len(r[2]) > 1), (None,) * 4)
+    if code is None:  # one kernel applies to every class
+        assert dtype_name != "f64"
+        bt.close()
+        return
+    bt.set_tuning({code: next(n for n in names if n != chosen)}, True)
+    _, _, kernels = bt.profile(forward=True, stream=s)
+    assert set(kernels) != {1024}
+    s.synchronize()
+    buf.copy_(start)
+    torch.cuda.synchronize()
+    bt.hierarchize(s)
+    s.synchronize()
+    assert torch.equal(buf, want)
+    bt.close()
