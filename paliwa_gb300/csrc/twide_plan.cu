@@ -80,8 +80,10 @@ int twide_code(Stage const &st, int dtype) {
 // (FP32 n = 128 at 2^12 4.1 against 6.7).
 bool twide_enough(int code, int dtype, long long points) {
   bool const longer =
-      code == kTWideBoxHeads + 16 || code == kTWideBox + 16 || code == kTWide32Box || code == kTWide32Chunked || code == kTWideChunked + 16 ||
-      code == kTWideLong + 16 || code == kTWideLongContig + 16;
+      code == kTWideBoxHeads + 16 || code == kTWideBox + 16 ||
+      code == kTWide32Box || code == kTWide32Chunked ||
+      code == kTWideChunked + 16 || code == kTWideLong + 16 ||
+      code == kTWideLongContig + 16;
   return longer || points >= (dtype == PALIWA_GB_F64 ? 1LL << 12 : 1LL << 13);
 }
 
