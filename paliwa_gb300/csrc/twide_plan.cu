@@ -388,7 +388,7 @@ void launch_stage(int dtype, bool exact, bool symmetric, int ws,
       p.error = stage_error_word();
       return launch_twide(dtype, exact, tsched, code, p, s);
     }
-    if (st.heads != 0)
+    if (st.heads != 0)  // (plan_axis has seen its maps accepted)
       throw StatusError(PALIWA_GB_CUDA_ERROR,
                         "the tensor map of a windowed stage was refused");
   }
