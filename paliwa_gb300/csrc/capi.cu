@@ -510,7 +510,44 @@ void plan_heads(AxisView const &v, std::vector<int> const &shifts,
   if (!forward) out.push_back(st);
 }
 
+// The levels of hierarchize_in or dehierarchize_in.
+bool ordered_levels(AxisView const &view, std::vector<int> const &shifts) {
+  if (shifts.size() > kMaxLevels) return false;
+  LiftJob const order = make_job(view, shifts, 0, shifts.size());
+  return canonical_shifts(order, true) || canonical_shifts(order, false);
+}
+
+// FP32c pencils that the boxed form's windows take. It rounds to its storage
+// between windows and sub-lattice, so it takes that split only where the
+// windows hand the sub-lattice on unrounded, in a buffer of its own that the
+// tile kernel transforms (512 to 4096 heads) and rounds where the other split
+// does.
+bool head_windows(AxisView const &view, std::vector<int> const &shifts,
+                  std::vector<Filter> const &filters) {
+  int const ws = wavelet_schedule(filters);
+  return view.wide_last && ws >= 0 && ordered_levels(view, shifts) &&
+         canonical_shifts(make_job(view, shifts, 0, shifts.size()),
+                          (ws & 1) != 0) &&
+         view.log2_n > kWindowLog2 && view.log2_n <= 16 &&
+         box_windows(view, filters.size());
+}
+
+// Levels that windows leave to the sub-lattice of the heads, one per chunk of
+// 16 points.
+constexpr int kHeadShift = 4;
+
+bool coarse_levels(std::vector<int> const &shifts) {
+  return std::any_of(shifts.begin(), shifts.end(),
+                     [](int s) { return s >= kHeadShift; });
+}
+
 } // namespace
+
+bool uses_heads(AxisView const &view, std::vector<int> const &shifts,
+                std::vector<Filter> const &filters) {
+  return tensor_map_encoder() != nullptr && coarse_levels(shifts) &&
+         head_windows(view, shifts, filters);
+}
 
 void plan_axis(AxisView const &view, std::vector<int> const &shifts,
                std::vector<Filter> const &filters, std::vector<Stage> &out,
@@ -527,26 +564,16 @@ void plan_axis(AxisView const &view, std::vector<int> const &shifts,
   // 32 points of 512 is the same 14 % as 256 of 4096 and leaves 1/16 of the
   // points (1/32 for one pass) to the sub-lattice.
   int const P = static_cast<int>(filters.size());
-  LiftJob const order = make_job(
-      view, shifts, 0, std::min(shifts.size(), static_cast<size_t>(kMaxLevels)));
-  bool const ordered = shifts.size() <= kMaxLevels &&
-                       (canonical_shifts(order, true) ||
-                        canonical_shifts(order, false));
-  // FP32c rounds to its storage between the two kinds of stages: it takes
-  // that split only where the windows hand the sub-lattice on unrounded, in a
-  // buffer of its own that the tile kernel transforms (512 to 4096 heads) and
-  // rounds where the other split does.
   int const ws = wavelet_schedule(filters);
-  bool const heads = view.wide_last && view.heads != 0 && ws >= 0 && ordered &&
-                     canonical_shifts(order, (ws & 1) != 0) &&
-                     view.log2_n <= 16 && box_windows(view, filters.size());
-  bool const box = heads || (ordered && !view.wide_last &&
+  bool const heads = head_windows(view, shifts, filters) &&
+                     (view.heads != 0 || !coarse_levels(shifts));
+  bool const box = heads || (!view.wide_last && ordered_levels(view, shifts) &&
                              box_windows(view, filters.size()));
   int const budget = box ? kBoxHalo : kHaloBudget;
   int m = 0;
   while (static_cast<long long>(P) * ((2LL << m) - 1) <= budget) ++m;
   if (m < 1) m = 1;
-  if (heads) m = 4;  // one head per chunk of 16 points
+  if (heads) m = kHeadShift;
   size_t const planned = out.size();
   size_t i = 0;
   while (i < shifts.size()) {
@@ -685,12 +712,18 @@ void transform_axis(void *grid, int dtype, int ndim, int64_t const *level,
   void *shadow = nullptr;
   if (needs_shadow(view, shifts)) {
     // Stream-ordered scratch for the windowed stages of long pencils: the
-    // halo buffer and, for FP32c, the heads' buffer after it.
+    // halo buffer and, where the plan has a use for it and memory allows, the
+    // heads' buffer after it.
     size_t bytes = dtype_size(dtype);
     for (int d = 0; d < ndim; ++d) bytes <<= level[d];
-    size_t const heads = dtype == PALIWA_GB_F32C ? bytes / 8 : 0;
-    cuda_check(cudaMallocAsync(&shadow, bytes + heads, s),
-               "cudaMallocAsync(shadow)");
+    size_t heads = uses_heads(view, shifts, filters) ? bytes / 8 : 0;
+    cudaError_t e = cudaMallocAsync(&shadow, bytes + heads, s);
+    if (e == cudaErrorMemoryAllocation && heads != 0) {
+      cudaGetLastError();
+      heads = 0;
+      e = cudaMallocAsync(&shadow, bytes, s);
+    }
+    cuda_check(e, "cudaMallocAsync(shadow)");
     view.shadow = reinterpret_cast<unsigned long long>(shadow);
     if (heads != 0) view.heads = view.shadow + bytes;
   }

@@ -112,7 +112,7 @@ extern "C" int paliwa_gb_transform_noalloc(void *grid, int dtype, int ndim,
                   "much scratch; the allocation-free transform holds at most "
                   "67108864 bytes (64 MiB)");
         view.shadow = reinterpret_cast<unsigned long long>(scratch_address());
-        if (dtype == PALIWA_GB_F32C)
+        if (uses_heads(view, shifts, filters))
           view.heads = view.shadow + kStaticScratchBytes;
       }
       plan_axis(view, shifts, filters, plans[d]);

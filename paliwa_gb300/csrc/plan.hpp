@@ -43,7 +43,7 @@ struct AxisView {
   // windowed stages' halos (pencils longer than one CTA holds; 0: none).
   unsigned long long shadow = 0;
   // Byte address of a buffer of an eighth of the grid's size for the chunk
-  // heads of FP32c windows as double-float pairs (0: none).
+  // heads of FP32c windows as double-float pairs (0: none; uses_heads).
   unsigned long long heads = 0;
   long long columns = 1;        // outer * inner
   int log2_inner = 0;
@@ -161,6 +161,10 @@ long long stage_points(Stage const &st);
 inline bool needs_shadow(AxisView const &view, std::vector<int> const &shifts) {
   return !shifts.empty() && view.log2_n > kWindowLog2;
 }
+
+// True when planning `view` along `shifts` makes use of the field `heads`.
+bool uses_heads(AxisView const &view, std::vector<int> const &shifts,
+                std::vector<Filter> const &filters);
 
 // Kernel-level parameters shared by every job of a launch.
 LiftParams launch_params(std::vector<Filter> const &filters);
