@@ -67,9 +67,13 @@ const char *paliwa_gb_last_error(void);
 int paliwa_gb_version(void);
 
 /* Waits for the work queued on `stream` (the fence() of an execution-space
- * instance, paliwa/paliwa_utils.hpp:27-32). PALIWA_GB_TIMEOUT if a bounded
- * wait of a single-grid transform's tile copies gave up since the last
- * report (the next transform call reports it too). */
+ * instance, paliwa/paliwa_utils.hpp:27-32). A single-grid transform returns
+ * once its work is queued; this call confirms its result: PALIWA_GB_TIMEOUT if
+ * a bounded wait of the tile copies of such a transform on `stream`, or of a
+ * captured one on any stream, gave up since the last report (its grid then
+ * holds no result). Otherwise the next single-grid transform on the stream
+ * reports it, before it queues anything. (Streams are told apart by their
+ * handles, up to 1023 of them per device.) */
 int paliwa_gb_synchronize(void *stream);
 
 /* Wavelet name -> id. Unknown names return PALIWA_GB_OUT_OF_RANGE, as
@@ -205,9 +209,11 @@ int paliwa_gb_dump_to_binary_file(const void *data, int64_t bytes,
  * Only grids with a pencil longer than 4096 points need scratch; this entry
  * point takes it from one 64 MiB array in device memory (and 8 MiB more for
  * FP32c) that every GPU loading the library holds until the process exits, so
- * such grids may be at most 64 MiB (larger ones return PALIWA_GB_INVALID_ARGUMENT before any work
- * is queued). The first call on each device looks up that array's address
- * (cudaGetSymbolAddress) with the device current; make it before any stream
+ * such grids may be at most 64 MiB (larger ones return
+ * PALIWA_GB_INVALID_ARGUMENT before any work is queued). The first call on each
+ * device looks up that array's address (cudaGetSymbolAddress) with the device
+ * current, and takes a page of pinned host memory for the error words of the
+ * bounded waits unless another single-grid call has; make it before any stream
  * capture. All calls share the array, which keeps the last call's contents
  * (the transform writes every byte it reads back, so nothing is cleared):
  * calls whose work overlaps on the GPU (different streams) race on it and

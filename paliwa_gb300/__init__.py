@@ -19,7 +19,7 @@ from .transform import (dehierarchize, dehierarchize_in, hierarchize,
                         hierarchize_in,
                         lifting_wavelet_filter_offsets_and_coefficients,
                         lifting_wavelet_reconstruct_offsets_and_coefficients,
-                        transform_bounds, transform_in, transform_in_window,
+                        synchronize, transform_bounds, transform_in, transform_in_window,
                         transform_outputs,
                         wavelet_id)
 
@@ -32,6 +32,7 @@ __all__ = [
     "strided_hierarchical_domain_from_level", "dehierarchize",
     "dehierarchize_in", "hierarchize", "hierarchize_in",
     "lifting_wavelet_filter_offsets_and_coefficients",
-    "lifting_wavelet_reconstruct_offsets_and_coefficients", "transform_bounds",
+    "lifting_wavelet_reconstruct_offsets_and_coefficients", "synchronize",
+    "transform_bounds",
     "transform_in", "transform_in_window", "transform_outputs", "wavelet_id",
 ]

@@ -705,7 +705,8 @@ void check_shape(void *grid, int dtype, int ndim, int64_t const *level,
 
 void transform_axis(void *grid, int dtype, int ndim, int64_t const *level,
                     int dim, std::vector<int> const &shifts,
-                    std::vector<Filter> const &filters, cudaStream_t s) {
+                    std::vector<Filter> const &filters, unsigned *error,
+                    cudaStream_t s) {
   LiftParams const params = launch_params(filters);
   AxisView view = axis_view(reinterpret_cast<unsigned long long>(grid), ndim,
                             level, dim, dtype);
@@ -716,7 +717,9 @@ void transform_axis(void *grid, int dtype, int ndim, int64_t const *level,
     // heads' buffer after it.
     size_t bytes = dtype_size(dtype);
     for (int d = 0; d < ndim; ++d) bytes <<= level[d];
-    size_t heads = uses_heads(view, shifts, filters) ? bytes / 8 : 0;
+    size_t heads = error != nullptr && uses_heads(view, shifts, filters)
+                       ? bytes / 8
+                       : 0;
     cudaError_t e = cudaMallocAsync(&shadow, bytes + heads, s);
     if (e == cudaErrorMemoryAllocation && heads != 0) {
       cudaGetLastError();
@@ -734,7 +737,7 @@ void transform_axis(void *grid, int dtype, int ndim, int64_t const *level,
     bool const sym = symmetric_filters(filters);
     int const ws = wavelet_schedule(filters);
     for (auto const &st : stages)
-      launch_stage(dtype, exact, sym, ws, params, st, s);
+      launch_stage(dtype, exact, sym, ws, params, st, error, s);
   } catch (...) {
     if (shadow) cudaFreeAsync(shadow, s);
     throw;
@@ -762,16 +765,18 @@ int hierarchize_dims(void *grid, int dtype, int ndim, int64_t const *level,
       throw StatusError(PALIWA_GB_INVALID_ARGUMENT, "bad dimension");
     auto const filters = wavelet_filters(wavelet, forward);
     cudaStream_t const s = static_cast<cudaStream_t>(stream);
+    unsigned *const error = begin_stages(s);
     // Every axis: the trailing ones may go in one launch of the slab kernel.
-    int const slab = dim_begin == 0 && dim_end == ndim
+    int const slab = dim_begin == 0 && dim_end == ndim && error != nullptr
                          ? single_slab_start(dtype, ndim, level, lmin, grid)
                          : dim_end;
     for (int d = dim_begin; d < dim_end; ++d) {
       if (d == slab && launch_single_slab(dtype, ndim, slab, level, lmin, grid,
-                                          wavelet_schedule(filters), s))
+                                          wavelet_schedule(filters), error, s))
         break;
       transform_axis(grid, dtype, ndim, level, d,
-                     level_shifts(level[d], lmin[d], forward), filters, s);
+                     level_shifts(level[d], lmin[d], forward), filters, error,
+                     s);
     }
   });
 }
@@ -786,9 +791,9 @@ int paliwa_gb_version(void) { return 100; }
 
 int paliwa_gb_synchronize(void *stream) {
   return guarded([&] {
-    cuda_check(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)),
-               "cudaStreamSynchronize");
-    check_stage_errors();
+    cudaStream_t const s = static_cast<cudaStream_t>(stream);
+    cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+    check_stage_errors(s);
   });
 }
 
@@ -843,8 +848,9 @@ int paliwa_gb_transform_in(void *grid, int dtype, int ndim,
                           "transform level out of range");
       shifts.push_back(static_cast<int>(level[dim] - levels[i]));
     }
+    cudaStream_t const s = static_cast<cudaStream_t>(stream);
     transform_axis(grid, dtype, ndim, level, dim, shifts, filters,
-                   static_cast<cudaStream_t>(stream));
+                   begin_stages(s), s);
   });
 }
 

@@ -8,7 +8,9 @@
 // scratch only for grids with a pencil longer than 4096 points (the halo
 // buffer of its windowed stages, the grid's size) and takes it from the
 // stream-ordered allocator. This variant takes it from one file-scope device
-// array instead and allocates nothing.
+// array instead and allocates nothing on the device. (The first single-grid
+// call on a device, this one or another, takes one page of pinned host memory
+// for the error words of the bounded waits.)
 #include <array>
 #include <cstdint>
 #include <mutex>
@@ -96,6 +98,7 @@ extern "C" int paliwa_gb_transform_noalloc(void *grid, int dtype, int ndim,
     bool const exact = exact_scalers(filters);
     bool const sym = symmetric_filters(filters);
     int const ws = wavelet_schedule(filters);
+    unsigned *const error = begin_stages(s);
     // Plan every axis first, so that a grid whose scratch does not fit is
     // rejected before any work is queued.
     std::vector<std::vector<Stage>> plans(ndim);
@@ -112,13 +115,13 @@ extern "C" int paliwa_gb_transform_noalloc(void *grid, int dtype, int ndim,
                   "much scratch; the allocation-free transform holds at most "
                   "67108864 bytes (64 MiB)");
         view.shadow = reinterpret_cast<unsigned long long>(scratch_address());
-        if (uses_heads(view, shifts, filters))
+        if (error != nullptr && uses_heads(view, shifts, filters))
           view.heads = view.shadow + kStaticScratchBytes;
       }
       plan_axis(view, shifts, filters, plans[d]);
     }
     for (auto const &stages : plans)
       for (auto const &st : stages)
-        launch_stage(dtype, exact, sym, ws, params, st, s);
+        launch_stage(dtype, exact, sym, ws, params, st, error, s);
   });
 }

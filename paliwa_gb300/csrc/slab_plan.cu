@@ -164,7 +164,7 @@ int single_slab_start(int dtype, int ndim, int64_t const *level,
 
 bool launch_single_slab(int dtype, int ndim, int m, int64_t const *level,
                         int64_t const *lmin, void *grid, int sched,
-                        cudaStream_t s) {
+                        unsigned *error, cudaStream_t s) {
   auto const addr = reinterpret_cast<unsigned long long>(grid);
   size_t const es = dtype_size(dtype);
   int64_t total = 0;
@@ -176,8 +176,7 @@ bool launch_single_slab(int dtype, int ndim, int m, int64_t const *level,
   p.njobs = 1;
   p.pairs = slab_pairs(p.job);
   p.total_tiles = 1LL << (total - p.job.log2_tile);
-  check_stage_errors();
-  p.error = stage_error_word();
+  p.error = error;
   launch_slab(dtype, sched, p, s);
   return true;
 }

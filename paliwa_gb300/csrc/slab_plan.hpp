@@ -22,12 +22,12 @@ void launch_slab_f32(int sched, SlabParams const &p, cudaStream_t s);
 void launch_slab_f32c(int sched, SlabParams const &p, cudaStream_t s);
 
 // First axis of the trailing axes that a single grid's transform runs as one
-// slab launch (ndim: none), and that launch (false: the tensor map was
-// refused and nothing was launched).
+// slab launch (ndim: none), and that launch (error: from begin_stages; false:
+// the tensor map was refused and nothing was launched).
 int single_slab_start(int dtype, int ndim, int64_t const *level,
                       int64_t const *lmin, void const *grid);
 bool launch_single_slab(int dtype, int ndim, int m, int64_t const *level,
                         int64_t const *lmin, void *grid, int sched,
-                        cudaStream_t s);
+                        unsigned *error, cudaStream_t s);
 
 } // namespace pgb

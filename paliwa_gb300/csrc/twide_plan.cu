@@ -5,6 +5,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "launch.cuh"
 #include "paliwa_gb300.h"
 #include "twide_box.cuh"
 #include "twide_plan.hpp"
@@ -321,46 +322,104 @@ void launch_twide(int dtype, bool exact, int sched, int code,
 
 namespace {
 
-// The error word of the single-grid launches' bounded waits: one mapped,
-// portable host word, so that the host reads it without a copy and every
-// device can set it. Allocated by the first such launch (also inside a
-// stream capture: the allocation is not part of the captured work).
-std::atomic<unsigned *> g_error_word{nullptr};
+// Error words of the single-grid launches' bounded waits, per device: one per
+// stream handle, given out in order of use (once all are, further streams
+// share them), and one for captured launches, whose replays may run on any
+// stream. They lie in mapped host memory (one page), which the host reads
+// without a copy. (By the handle, not the id: cudaStreamGetId ends a capture.)
+constexpr unsigned kStreamWords = 1023;
+std::atomic<unsigned *> g_error_words[Occupancy::kMaxDevices];
+std::atomic<uintptr_t> g_word_streams[Occupancy::kMaxDevices][kStreamWords];
 
-} // namespace
-
-unsigned *stage_error_word() {
-  unsigned *word = g_error_word.load(std::memory_order_acquire);
-  if (word != nullptr) return word;
+// Allocated by a device's first single-grid call (also inside a stream
+// capture: the allocation is not part of the captured work); nullptr where
+// that fails.
+unsigned *error_words(int dev) {
+  if (dev < 0 || dev >= Occupancy::kMaxDevices) return nullptr;
+  unsigned *words = g_error_words[dev].load(std::memory_order_acquire);
+  if (words != nullptr) return words;
   static std::mutex mutex;
   std::lock_guard<std::mutex> lock(mutex);
-  word = g_error_word.load(std::memory_order_acquire);
-  if (word != nullptr) return word;
+  words = g_error_words[dev].load(std::memory_order_acquire);
+  if (words != nullptr) return words;
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   cuda_check(cudaThreadExchangeStreamCaptureMode(&mode),
              "cudaThreadExchangeStreamCaptureMode");
   void *p = nullptr;
-  cudaError_t const e = cudaHostAlloc(
-      &p, sizeof(unsigned), cudaHostAllocPortable | cudaHostAllocMapped);
+  size_t const bytes = (kStreamWords + 1) * sizeof(unsigned);
+  cudaError_t const e =
+      cudaHostAlloc(&p, bytes, cudaHostAllocPortable | cudaHostAllocMapped);
   cudaThreadExchangeStreamCaptureMode(&mode);
-  cuda_check(e, "cudaHostAlloc(error word)");
-  word = static_cast<unsigned *>(p);
-  *static_cast<unsigned volatile *>(word) = 0;
-  g_error_word.store(word, std::memory_order_release);
-  return word;
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  std::memset(p, 0, bytes);
+  words = static_cast<unsigned *>(p);
+  g_error_words[dev].store(words, std::memory_order_release);
+  return words;
 }
 
-void check_stage_errors() {
-  unsigned volatile *const word = g_error_word.load(std::memory_order_acquire);
-  if (word == nullptr || *word == 0) return;
-  *word = 0;
-  throw StatusError(PALIWA_GB_TIMEOUT,
-                    "a bounded wait of an earlier transform's tile copies "
-                    "gave up");
+unsigned stream_slot(int dev, cudaStream_t s) {
+  uintptr_t const key =
+      s == nullptr ? reinterpret_cast<uintptr_t>(cudaStreamLegacy)
+                   : reinterpret_cast<uintptr_t>(s);
+  unsigned const first = static_cast<unsigned>((key >> 4) % kStreamWords);
+  for (unsigned i = 0, k = first; i < kStreamWords; ++i) {
+    auto &slot = g_word_streams[dev][k];
+    uintptr_t cur = slot.load(std::memory_order_relaxed);
+    if (cur == key ||
+        (cur == 0 && (slot.compare_exchange_strong(cur, key) || cur == key)))
+      return k;
+    k = k + 1 == kStreamWords ? 0 : k + 1;
+  }
+  return first;
+}
+
+// Whether the word was set; clears it. (A report that comes in between is
+// either part of this one or stays.)
+bool take_error(unsigned *word) {
+  return __atomic_load_n(word, __ATOMIC_RELAXED) != 0 &&
+         __atomic_exchange_n(word, 0u, __ATOMIC_ACQ_REL) != 0;
+}
+
+} // namespace
+
+unsigned *stage_error_word(cudaStream_t s) {
+  if (tensor_map_encoder() == nullptr) return nullptr;
+  int const dev = current_device();
+  unsigned *const words = error_words(dev);
+  if (words == nullptr) return nullptr;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) cudaGetLastError();
+  return words + (capture != cudaStreamCaptureStatusNone
+                      ? kStreamWords
+                      : stream_slot(dev, s));
+}
+
+void check_stage_errors(cudaStream_t s) {
+  int const dev = current_device();
+  if (dev < 0 || dev >= Occupancy::kMaxDevices) return;
+  unsigned *const words = g_error_words[dev].load(std::memory_order_acquire);
+  if (words == nullptr) return;
+  bool const own = take_error(words + stream_slot(dev, s));
+  bool const captured = take_error(words + kStreamWords);
+  if (own || captured)
+    throw StatusError(PALIWA_GB_TIMEOUT,
+                      own ? "a bounded wait of an earlier transform's tile "
+                            "copies on this stream gave up"
+                          : "a bounded wait of a captured transform's tile "
+                            "copies gave up");
+}
+
+unsigned *begin_stages(cudaStream_t s) {
+  check_stage_errors(s);
+  return stage_error_word(s);
 }
 
 void launch_stage(int dtype, bool exact, bool symmetric, int ws,
-                  LiftParams const &params, Stage const &st, cudaStream_t s) {
+                  LiftParams const &params, Stage const &st, unsigned *error,
+                  cudaStream_t s) {
   int const sched =
       ws >= 0 && canonical_shifts(st.job, (ws & 1) != 0) ? ws : -1;
   if (st.R >= kHeadsIn) {
@@ -368,7 +427,7 @@ void launch_stage(int dtype, bool exact, bool symmetric, int ws,
     p.job = st.job;
     return launch_heads(sched, st.R, p, st.tiles, s);
   }
-  if (st.tma) {
+  if (st.tma && error != nullptr) {
     TWideParams p;
     std::memset(&p, 0, sizeof(p));
     p.heads = reinterpret_cast<uint4 *>(st.heads);
@@ -384,14 +443,13 @@ void launch_stage(int dtype, bool exact, bool symmetric, int ws,
     int const code = twide_code(st, dtype);
     if (code != 0 && twide_enough(code, dtype, stage_points(st)) &&
         twide_job(st, dtype, p.job, p.map, p.total_tiles)) {
-      check_stage_errors();
-      p.error = stage_error_word();
+      p.error = error;
       return launch_twide(dtype, exact, tsched, code, p, s);
     }
-    if (st.heads != 0)  // (plan_axis has seen its maps accepted)
-      throw StatusError(PALIWA_GB_CUDA_ERROR,
-                        "the tensor map of a windowed stage was refused");
   }
+  if (st.heads != 0)  // (planned with an error word and its maps accepted)
+    throw StatusError(PALIWA_GB_CUDA_ERROR,
+                      "the tensor map of a windowed stage was refused");
   LiftParams p = params;
   p.job = st.job;
   launch_lift(dtype, exact, symmetric, sched, st.R, p, nullptr, 1, st.tiles,

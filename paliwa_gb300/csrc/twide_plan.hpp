@@ -52,17 +52,23 @@ void launch_twide_table_f32(bool exact, int sched, int code,
 void launch_twide_table_f64(bool exact, int sched, int code,
                             TWideParams const &p, cudaStream_t s);
 
+// Before a single-grid call on stream s queues anything: throws
+// PALIWA_GB_TIMEOUT as check_stage_errors does (the call's grid is untouched),
+// and returns the word that the call's bounded waits report to; nullptr where
+// there is none, or no encoder: the call then runs without TMA launches.
+unsigned *begin_stages(cudaStream_t s);
+unsigned *stage_error_word(cudaStream_t s);
+
+// Throws PALIWA_GB_TIMEOUT when a bounded wait of a single-grid launch gave
+// up since the last report: one on stream s, or one that was captured (on any
+// stream of the device). Clears the report.
+void check_stage_errors(cudaStream_t s);
+
 // Launches one stage of a single grid: on the TMA wide kernel when it is
-// planned on it and qualifies, else on its own kernel. ws is the filters'
-// wavelet schedule (or -1).
+// planned on it, qualifies and error (from begin_stages) is there, else on its
+// own kernel. ws is the filters' wavelet schedule (or -1).
 void launch_stage(int dtype, bool exact, bool symmetric, int ws,
-                  LiftParams const &params, Stage const &st, cudaStream_t s);
-
-// The error word of single-grid launches (see check_stage_errors).
-unsigned *stage_error_word();
-
-// Throws PALIWA_GB_TIMEOUT (and clears the flag) when a bounded wait of a
-// single-grid launch gave up since the last call.
-void check_stage_errors();
+                  LiftParams const &params, Stage const &st, unsigned *error,
+                  cudaStream_t s);
 
 } // namespace pgb

@@ -111,6 +111,21 @@ def _call(fn_name, grid, args, stream):
         _lib.check(rc)
 
 
+def synchronize(stream=None, device=None):
+    """Waits for the work queued on ``stream`` (default: the current stream of
+    ``device``) and confirms the single-grid transforms on it: raises
+    DeviceTimeout if a bounded wait inside one of them, or inside a captured
+    one, gave up (its grid then holds no result). Otherwise the next transform
+    on the stream raises that, with its grid untouched."""
+    import torch
+    if stream is None:
+        stream = torch.cuda.current_stream(device)
+    with torch.cuda.device(getattr(stream, "device", device)):
+        _lib.check(_lib.load().paliwa_gb_synchronize(
+            stream.cuda_stream if hasattr(stream, "cuda_stream")
+            else int(stream)))
+
+
 def hierarchize(grid, level, minimum_level, maximum_level,
                 wavelet_name="hat", stream=None, compensated=False):
     """Forward transform over every dimension, dimension 0 first."""
