@@ -269,10 +269,30 @@ void launch_out_list(OutPass const &p, OutList const &q, size_t smem,
   cuda_check(cudaGetLastError(), "out_list_kernel launch");
 }
 
-// One launch for the whole list when the touched stretch of the axis fits
-// shared memory with 4 columns or more (up to 32: whole 128-byte lines of
-// floats; fewer when that leaves under two CTAs per SM), else one launch per
-// pass.
+// Whether one launch for the list is worth it. It saves launches and passes
+// over memory, but a CTA runs its columns' passes one after another, where a
+// launch per pass spreads each over the chip: one column of 4609 floats, two
+// passes, took 47 us against 4.1. Both sides' times in us, fitted to 668 calls
+// of 2 to 18 passes on 1 to 2^19 columns (a thread's chain of steps, and what
+// the columns take together; FP64 by its pipe), the list's rather long: one of
+// them is then more than 2 % slower than a launch per pass (6 %), and all gain
+// 1.77x, where the better side of each would give 1.82x.
+bool out_list_pays(bool f64, long long columns, int log2cols, size_t npasses,
+                   long long extent, long long updates) {
+  double const rows = 256 >> log2cols;  // of a CTA's threads along the axis
+  double const mega = columns * 1e-6;
+  double const list = 2.6 + 0.2 * npasses +
+                      ((f64 ? 0.2 : 0.15) * updates + 0.45 * extent) / rows +
+                      mega * (100 + (f64 ? 2.4 : 0.8) * updates +
+                              (f64 ? 2.1 : 0.6) * extent);
+  double const passes = 0.2 + 1.9 * npasses + mega * (f64 ? 9 : 7.3) * updates;
+  return list < 0.85 * passes;
+}
+
+// One launch for the whole list when that pays and the touched stretch of the
+// axis fits shared memory with 4 columns or more (up to 32: whole 128-byte
+// lines of floats; fewer when that leaves under two CTAs per SM), else one
+// launch per pass.
 void launch_out_call(int dtype, bool exact, OutCall const &call,
                      long long columns, long long window_extent,
                      cudaStream_t s) {
@@ -293,9 +313,10 @@ void launch_out_call(int dtype, bool exact, OutCall const &call,
   auto index = [&](long long u) {
     return ((u - p.wfront) & (p.period - 1)) >> p.log2_spacing;
   };
-  long long lo = window_extent, hi = -1;
+  long long lo = window_extent, hi = -1, updates = 0;
   for (size_t i = 0; i < n; ++i) {
     OutPass const &r = call.passes[i];
+    updates += r.count;
     long long const last = r.first + (r.count - 1) * r.step;
     long long const a = index(r.first - r.s), b = index(r.first);
     long long const c = index(last), d = index(last + r.s);
@@ -326,7 +347,9 @@ void launch_out_call(int dtype, bool exact, OutCall const &call,
   while (log2cols > 2 && (smem_of(log2cols) > kOutSmem ||
                           (columns >> log2cols) < 2 * 152))
     --log2cols;
-  if (smem_of(log2cols) > kOutSmem) return one_by_one();
+  if (smem_of(log2cols) > kOutSmem ||
+      !out_list_pays(es == 8, columns, log2cols, n, extent, updates))
+    return one_by_one();
   q.k0 = static_cast<int>(lo);
   q.extent = static_cast<int>(extent);
   q.log2cols = log2cols;

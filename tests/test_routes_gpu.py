@@ -1,0 +1,57 @@
+"""Calls for which one launch is the slower way: the launches of a call, as
+the kernel nodes of its capture."""
+import ctypes
+
+import pytest
+
+import paliwa_gb300 as pg
+
+pytestmark = pytest.mark.gpu
+
+
+def launches(call):
+    """Kernel nodes that call(stream) adds to a capture."""
+    import torch
+    cu = ctypes.CDLL("libcuda.so.1")
+    s = torch.cuda.Stream()
+    call(s)  # what a first call sets up is not part of it
+    torch.cuda.synchronize()
+    graph, n = ctypes.c_void_p(), ctypes.c_size_t()
+    h = ctypes.c_void_p(s.cuda_stream)
+    # CU_STREAM_CAPTURE_MODE_RELAXED
+    assert cu.cuStreamBeginCapture_v2(h, 2) == 0
+    call(s)
+    assert cu.cuStreamEndCapture(h, ctypes.byref(graph)) == 0
+    assert cu.cuGraphGetNodes(graph, None, ctypes.byref(n)) == 0
+    nodes = (ctypes.c_void_p * n.value)()
+    assert cu.cuGraphGetNodes(graph, nodes, ctypes.byref(n)) == 0
+    kernels = 0
+    for node in nodes:
+        kind = ctypes.c_int()
+        assert cu.cuGraphNodeGetType(ctypes.c_void_p(node),
+                                     ctypes.byref(kind)) == 0
+        kernels += kind.value == 0  # CU_GRAPH_NODE_TYPE_KERNEL
+    assert cu.cuGraphDestroy(graph) == 0
+    return kernels
+
+
+@pytest.mark.parametrize("level, dim, first, count, levels, want", [
+    # few columns: a launch per pass
+    ((13,), 0, 100, 4609, (13,), 2),
+    ((2, 13), 1, 0, 4096, (13, 12), 4),
+    # columns for every SM, a short stretch: one launch
+    ((8, 8, 7), 0, 16, 160, (8, 7, 6, 5), 1),
+    ((6, 6, 8), 2, 16, 160, (8, 7, 6, 5), 1),
+])
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_pass_list_launches(dtype, level, dim, first, count, levels, want):
+    import torch
+    shape = [1 << l for l in level]
+    shape[dim] = count
+    front = [0] * len(level)
+    front[dim] = first
+    x = torch.zeros(shape, dtype=getattr(torch, dtype), device="cuda")
+    filters = pg.lifting_wavelet_filter_offsets_and_coefficients[
+        "biorthogonal"]
+    assert launches(lambda s: pg.transform_in_window(
+        x, dim, level, level, levels, filters, front, stream=s)) == want
