@@ -136,13 +136,18 @@ void launch_slab(int dtype, int sched, SlabParams const &p, cudaStream_t s) {
 
 // Measured, one call (us, hat / CDF (2,2)), slab against axis by axis:
 // launches are what small grids spend their time on (FP32 4^6 15 against 31,
-// FP32c 32^2 x 64 17 / 21 against 22 / 23, FP64 16^3 14 / 21 against 24 / 31).
-// Floats gain up to about 2^22 points (FP32c 1024 x 64 x 64 35 / 42 against 37
-// / 46; 4096 x 64 x 64 131 / 155 against 122 / 155). FP32 gains again where
-// the axes no longer run out of L2 (2^26 points: 341 / 363 against 370 / 377;
-// 2^24: 106 / 114 against 100 / 108). One SM's FP64 pipe holds doubles to
-// 2^13 points on three or more axes and 2^11 on two (64 x 64: 16 / 27 against
-// 17 / 21).
+// 128 x 128 x 64 14 / 15 against 19 / 19; FP32c 32^2 x 64 15 / 17 against 19 /
+// 20). Floats gain up to about 2^22 points (FP32c 1024 x 64 x 64 34 / 42
+// against 36 / 46; 4096 x 64 x 64 130 / 159 against 120 / 152). FP32 gains
+// again where the axes no longer run out of L2 (2^26 points: 331 / 361 against
+// 362 / 371; 2^24: 106 / 114 against 99 / 108, on four axes 75 / 85 against 70
+// / 78). Doubles: one SM's FP64 pipe holds them to 2^13 points on three or
+// more axes and 2^11 on two; and a chunk is one thread's chain of updates,
+// which the wide kernel cuts into more (on the device, 32 x 32 12 / 22 against
+// 7 / 9, 8 x 64 8 / 14 against 6 / 8): no axis in chunks of 32, and two axes in
+// chunks of 16 only up to 2^8 points (32 x 16 7 / 10 against 6 / 9; 8 x 16, as
+// calls in a row, 8 / 10 against 11 / 12). Over 613 random FP64 grids that is
+// 1.25x axis by axis, where the better side of each would give 1.27x.
 int single_slab_start(int dtype, int ndim, int64_t const *level,
                       int64_t const *lmin, void const *grid) {
   auto const addr = reinterpret_cast<unsigned long long>(grid);
@@ -158,8 +163,17 @@ int single_slab_start(int dtype, int ndim, int64_t const *level,
   case PALIWA_GB_F32C: gain = total <= 22; break;
   case PALIWA_GB_F32: gain = total <= 22 || total >= 26; break;
   }
-  if (!gain || axes < 2 || addr % 128 != 0 || tensor_map_encoder() == nullptr) return ndim;
-  return slab_start(dtype, ndim, level, lmin, addr, addr);
+  if (!gain || axes < 2 || addr % 128 != 0 || tensor_map_encoder() == nullptr)
+    return ndim;
+  int const m = slab_start(dtype, ndim, level, lmin, addr, addr);
+  if (dtype == PALIWA_GB_F64 && m < ndim) {
+    SlabJob const job = slab_job(dtype, ndim, m, level, lmin, addr, addr);
+    int log2r = 0;
+    for (int a = 0; a < job.naxes; ++a)
+      log2r = std::max(log2r, static_cast<int>(job.axis[a].log2r));
+    if (log2r > 4 || (log2r == 4 && job.naxes < 3 && total > 8)) return ndim;
+  }
+  return m;
 }
 
 bool launch_single_slab(int dtype, int ndim, int m, int64_t const *level,

@@ -55,3 +55,20 @@ def test_pass_list_launches(dtype, level, dim, first, count, levels, want):
         "biorthogonal"]
     assert launches(lambda s: pg.transform_in_window(
         x, dim, level, level, levels, filters, front, stream=s)) == want
+
+
+@pytest.mark.parametrize("level, want", [
+    # a chunk of 32 points along some axis, or of 16 along one of two
+    ((5, 5), 2), ((3, 6), 2), ((6, 5), 2), ((5, 4), 2), ((3, 3, 5), 3),
+    # shorter chunks, more axes or tiny grids
+    ((6, 3), 1), ((4, 4), 1), ((4, 4, 3), 1), ((2, 2, 2, 4), 1),
+])
+@pytest.mark.parametrize("forward", [True, False])
+def test_small_double_grids_launches(level, want, forward):
+    import torch
+    x = torch.zeros([1 << l for l in level], dtype=torch.float64,
+                    device="cuda")
+    zero = (0,) * len(level)
+    fn = pg.hierarchize if forward else pg.dehierarchize
+    assert launches(lambda s: fn(x, level, zero, level, "biorthogonal",
+                                 stream=s)) == want
