@@ -88,6 +88,18 @@ bool twide_enough(int code, int dtype, long long points) {
   return longer || points >= (dtype == PALIWA_GB_F64 ? 1LL << 12 : 1LL << 13);
 }
 
+// A caller's filters on pencils of 2 points, and of 4 floats, have less work
+// for the same start-up (us, four passes / one, against the direct kernel:
+// FP32 n = 2 at 2^18 points 5.6 / 4.4 against 3.5 / 2.7, at 2^20 6.8 / 5.3
+// against 8.2 / 6.0; n = 4 5.2 / 3.7 against 4.5 / 3.0 and 6.5 / 5.1 against
+// 8.0 / 5.6; FP64 n = 2 at 2^16 9.0 / 5.2 against 7.2 / 3.6, at 2^18 8.7 / 5.0
+// against 11.4 / 4.6; FP64 n = 4 gains from 2^12 on).
+static bool table_enough(Stage const &st, int dtype) {
+  int const log2_n = st.job.log2_n;
+  return !st.table || log2_n > 2 || (log2_n == 2 && dtype == PALIWA_GB_F64) ||
+         stage_points(st) >= (dtype == PALIWA_GB_F64 ? 1LL << 18 : 1LL << 19);
+}
+
 namespace {
 
 // Boxed form: the 3D view [outer][n][inner] of the grid (and of the halo
@@ -442,6 +454,7 @@ void launch_stage(int dtype, bool exact, bool symmetric, int ws,
     }
     int const code = twide_code(st, dtype);
     if (code != 0 && twide_enough(code, dtype, stage_points(st)) &&
+        table_enough(st, dtype) &&
         twide_job(st, dtype, p.job, p.map, p.total_tiles)) {
       p.error = error;
       return launch_twide(dtype, exact, tsched, code, p, s);

@@ -1,5 +1,5 @@
-"""Calls for which one launch is the slower way: the launches of a call, as
-the kernel nodes of its capture."""
+"""Calls for which a newer route is the slower way: the kernels of a call, as
+the nodes of its capture."""
 import ctypes
 
 import pytest
@@ -9,8 +9,8 @@ import paliwa_gb300 as pg
 pytestmark = pytest.mark.gpu
 
 
-def launches(call):
-    """Kernel nodes that call(stream) adds to a capture."""
+def kernels(call):
+    """Names of the kernel nodes that call(stream) adds to a capture."""
     import torch
     cu = ctypes.CDLL("libcuda.so.1")
     s = torch.cuda.Stream()
@@ -25,14 +25,29 @@ def launches(call):
     assert cu.cuGraphGetNodes(graph, None, ctypes.byref(n)) == 0
     nodes = (ctypes.c_void_p * n.value)()
     assert cu.cuGraphGetNodes(graph, nodes, ctypes.byref(n)) == 0
-    kernels = 0
-    for node in nodes:
+    names = []
+    for node in map(ctypes.c_void_p, nodes):
         kind = ctypes.c_int()
-        assert cu.cuGraphNodeGetType(ctypes.c_void_p(node),
-                                     ctypes.byref(kind)) == 0
-        kernels += kind.value == 0  # CU_GRAPH_NODE_TYPE_KERNEL
+        assert cu.cuGraphNodeGetType(node, ctypes.byref(kind)) == 0
+        if kind.value != 0:  # CU_GRAPH_NODE_TYPE_KERNEL
+            continue
+        # CUDA_KERNEL_NODE_PARAMS_v2: func first, kern after extents,
+        # shared memory and two pointers
+        params, name = (ctypes.c_uint64 * 16)(), ctypes.c_char_p()
+        assert cu.cuGraphKernelNodeGetParams_v2(node, params) == 0
+        if params[0]:
+            assert cu.cuFuncGetName(ctypes.byref(name),
+                                    ctypes.c_void_p(params[0])) == 0
+        else:
+            assert cu.cuKernelGetName(ctypes.byref(name),
+                                      ctypes.c_void_p(params[7])) == 0
+        names.append(name.value.decode())
     assert cu.cuGraphDestroy(graph) == 0
-    return kernels
+    return names
+
+
+def launches(call):
+    return len(kernels(call))
 
 
 @pytest.mark.parametrize("level, dim, first, count, levels, want", [
@@ -72,3 +87,24 @@ def test_small_double_grids_launches(level, want, forward):
     fn = pg.hierarchize if forward else pg.dehierarchize
     assert launches(lambda s: fn(x, level, zero, level, "biorthogonal",
                                  stream=s)) == want
+
+
+@pytest.mark.parametrize("dtype, level, dim, tma", [
+    # few points in pencils of 2, or of 4 floats: no TMA launch
+    ("float32", (8, 1, 5), 1, False), ("float32", (8, 2, 5), 1, False),
+    ("float32", (12, 2), 1, False), ("float32", (13, 2, 3), 1, False),
+    ("float64", (8, 1, 5), 1, False), ("float64", (8, 1, 1), 1, False),
+    # longer pencils, or many points
+    ("float32", (8, 3, 5), 1, True), ("float32", (12, 2, 6), 1, True),
+    ("float32", (12, 1, 7), 1, True), ("float64", (8, 2, 5), 1, True),
+    ("float64", (12, 1, 7), 1, True),
+])
+def test_callers_filters_on_short_pencils(dtype, level, dim, tma):
+    import torch
+    x = torch.zeros([1 << l for l in level], dtype=getattr(torch, dtype),
+                    device="cuda")
+    filters = [(1, (-0.4, 1.0, -0.6)), (0, (0.3, 1.0, 0.2))]
+    names = kernels(lambda s: pg.transform_in(
+        x, dim, level, level, range(level[dim], 0, -1), filters, stream=s))
+    assert len(names) == 1
+    assert ("twide" in names[0]) == tma, names
