@@ -291,65 +291,52 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
             }
             by_r[code].push_back(&st);
           }
-        for (auto const &[R, list] : by_r) {
-          if (R > kTWide) {
-            Launch L;
-            L.group = grp;
-            L.R = R;
-            L.sched = ws;
-            L.job_first = all_twide.size();
-            L.tile_first = twide_tiles.size();
-            // Stages that do not qualify, by their own kernel; all of them
-            // when they are too few points together.
-            std::map<int, std::vector<Stage const *>> rest;
-            long long points = 0;
-            bool tuned = false;
-            for (Stage const *st : list) {
-              points += stage_points(*st);
-              tuned |= st->tuned;
-            }
-            bool const enough =
-                tuned || twide_enough(R - kTWide, b.dtype, points);
-            for (Stage const *st : list) {
-              TWideJob job;
-              CUtensorMap map[2];
-              long long tiles = 0;
-              if (!enough || !twide_job(*st, b.dtype, job, map, tiles)) {
-                rest[st->R].push_back(st);
-                continue;
-              }
-              job.tile_begin = L.tiles;
-              job.map = static_cast<int>(maps.size());
-              maps.push_back(map[0]);
-              if (st->box && job.win.seg_len > 0) {
-                job.win.halo_map = job.map + 1;
-                maps.push_back(map[1]);
-              }
-              all_twide.push_back(job);
-              twide_tiles.insert(twide_tiles.end(), tiles, L.njobs);
-              L.tiles += tiles;
-              L.points += stage_points(*st);
-              ++L.njobs;
-            }
-            if (L.njobs > 0) dr.launches.push_back(L);
-            for (auto const &[rR, rlist] : rest) {
-              Launch W;
-              W.group = grp;
-              W.R = rR;
-              W.sched = ws;
-              W.job_first = all_jobs.size();
-              W.njobs = static_cast<int>(rlist.size());
-              for (Stage const *st : rlist) {
-                LiftJob job = st->job;
-                job.tile_begin = W.tiles;
-                W.tiles += st->tiles;
-                W.points += stage_points(*st);
-                all_jobs.push_back(job);
-              }
-              dr.launches.push_back(W);
-            }
-            continue;
+        // TMA wide launches: stages that do not qualify, and all of a form
+        // that are too few points together, join the launches of their own
+        // kernels (3D |l|_1 = 4 - q with lmin 0, FP64: 37 launches, 43 where
+        // they had launches to themselves).
+        std::vector<Launch> wide;
+        for (auto it = by_r.upper_bound(kTWide); it != by_r.end();
+             it = by_r.erase(it)) {
+          auto const &[R, list] = *it;
+          Launch L;
+          L.group = grp;
+          L.R = R;
+          L.sched = ws;
+          L.job_first = all_twide.size();
+          L.tile_first = twide_tiles.size();
+          long long points = 0;
+          bool tuned = false;
+          for (Stage const *st : list) {
+            points += stage_points(*st);
+            tuned |= st->tuned;
           }
+          bool const enough =
+              tuned || twide_enough(R - kTWide, b.dtype, points);
+          for (Stage const *st : list) {
+            TWideJob job;
+            CUtensorMap map[2];
+            long long tiles = 0;
+            if (!enough || !twide_job(*st, b.dtype, job, map, tiles)) {
+              by_r[st->R].push_back(st);
+              continue;
+            }
+            job.tile_begin = L.tiles;
+            job.map = static_cast<int>(maps.size());
+            maps.push_back(map[0]);
+            if (st->box && job.win.seg_len > 0) {
+              job.win.halo_map = job.map + 1;
+              maps.push_back(map[1]);
+            }
+            all_twide.push_back(job);
+            twide_tiles.insert(twide_tiles.end(), tiles, L.njobs);
+            L.tiles += tiles;
+            L.points += stage_points(*st);
+            ++L.njobs;
+          }
+          if (L.njobs > 0) wide.push_back(L);
+        }
+        for (auto const &[R, list] : by_r) {
           Launch L;
           L.group = grp;
           L.R = R;
@@ -368,6 +355,7 @@ void plan_direction(paliwa_gb_batch &b, Direction &dr, bool forward,
           }
           if (L.R != 0 && L.tiles > 0) dr.launches.push_back(L);
         }
+        dr.launches.insert(dr.launches.end(), wide.begin(), wide.end());
       }
     }
     // The group's slab launch, after every per-axis stage of its grids.

@@ -108,3 +108,25 @@ def test_callers_filters_on_short_pencils(dtype, level, dim, tma):
         x, dim, level, level, range(level[dim], 0, -1), filters, stream=s))
     assert len(names) == 1
     assert ("twide" in names[0]) == tma, names
+
+
+def test_small_stages_of_a_batch_share_launches(oracle_mod):
+    """Stages too small for two forms of the TMA wide kernel that fall back to
+    one kernel run in one launch of it."""
+    import numpy as np
+    import torch
+    from paliwa_gb300 import ct
+    levels, lmin = [(3, 2), (5, 2)], (0, 2)
+    rng = np.random.default_rng(1)
+    hosts = [rng.uniform(-1, 1, [1 << l for l in lv]) for lv in levels]
+    grids = [torch.from_numpy(h).cuda() for h in hosts]
+    batch = ct.Batch(grids, levels, lmin, (5, 2), "biorthogonal", groups=1,
+                     slabs=False)
+    assert len(batch.profile(True)[2]) == 1
+    for g, h in zip(grids, hosts):
+        g.copy_(torch.from_numpy(h))
+    batch.hierarchize()
+    torch.cuda.synchronize()
+    for g, h, lv in zip(grids, hosts, levels):
+        want = oracle_mod.hierarchize(h.copy(), lv, lmin, lv, "biorthogonal")
+        assert np.array_equal(g.cpu().numpy(), want)
