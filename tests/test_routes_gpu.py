@@ -130,3 +130,18 @@ def test_small_stages_of_a_batch_share_launches(oracle_mod):
     for g, h, lv in zip(grids, hosts, levels):
         want = oracle_mod.hierarchize(h.copy(), lv, lmin, lv, "biorthogonal")
         assert np.array_equal(g.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_one_axis_grids_in_slab_launches(dtype):
+    """A slab launch where it saves launches (code 1024), not for a lone grid
+    with one axis."""
+    import torch
+    from paliwa_gb300 import ct
+    levels = [(9,), (8,), (10,)]
+    grids = [torch.zeros(1 << lv[0], dtype=getattr(torch, dtype),
+                         device="cuda") for lv in levels]
+    kinds = [ct.Batch(grids[:n], levels[:n], (0,), (10,), "biorthogonal",
+                      groups=1).profile(True)[2] for n in (1, 3)]
+    assert len(kinds[0]) == 1 and kinds[0] != [1024]
+    assert kinds[1] == [1024]
