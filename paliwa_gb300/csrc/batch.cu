@@ -609,7 +609,8 @@ struct paliwa_gb_ct {
   long long *unit_first_dev = nullptr;
   long long *families_dev = nullptr;
   long long *family_first_dev = nullptr;
-  // FP32 grids: the sparse values as floats during a restrict.
+  // FP32 grids, kCtNarrow points and more: the sparse values as floats during
+  // a restrict.
   float *values_dev = nullptr;
   long long ncombine = 0;   // combine CTAs
   long long nrestrict = 0;  // restrict CTAs
@@ -753,7 +754,7 @@ void plan_restrict(paliwa_gb_ct &ct, std::vector<CtSubspace> const &subs,
   ct.params.unit_first = ct.unit_first_dev;
   ct.params.families = ct.families_dev;
   ct.params.family_first = ct.family_first_dev;
-  if (ct.dtype != PALIWA_GB_F64 && ct.npoints > 0)
+  if (ct.dtype != PALIWA_GB_F64 && ct.npoints >= kCtNarrow)
     cuda_check(cudaMalloc(&ct.values_dev, ct.npoints * sizeof(float)),
                "cudaMalloc(restrict values)");
 }
@@ -932,32 +933,35 @@ void ct_combine(paliwa_gb_ct const &ct, double *sparse, cudaStream_t s) {
                    : launch_combine<float, false>(ct, p, s);
 }
 
-// Two to six dimensions have kernels of their own while 32-bit indices hold
+// One to six dimensions have kernels of their own while 32-bit indices hold
 // every grid and the sparse grid (with a unit to spare past a grid's end);
 // anything else takes the general one.
-template <typename S>
+template <typename S, typename V>
 void launch_restrict(paliwa_gb_ct const &ct, CtParams const &p,
                      cudaStream_t s) {
   unsigned const blocks = static_cast<unsigned>(ct.nrestrict);
   bool const small = !ct.big && ct.npoints < (1LL << 31);
   switch (small ? ct.ndim : 0) {
+  case 1:
+    ct_restrict_kernel<S, 1, unsigned, V><<<blocks, kCtBlock, 0, s>>>(p);
+    break;
   case 2:
-    ct_restrict_kernel<S, 2, unsigned><<<blocks, kCtBlock, 0, s>>>(p);
+    ct_restrict_kernel<S, 2, unsigned, V><<<blocks, kCtBlock, 0, s>>>(p);
     break;
   case 3:
-    ct_restrict_kernel<S, 3, unsigned><<<blocks, kCtBlock, 0, s>>>(p);
+    ct_restrict_kernel<S, 3, unsigned, V><<<blocks, kCtBlock, 0, s>>>(p);
     break;
   case 4:
-    ct_restrict_kernel<S, 4, unsigned><<<blocks, kCtBlock, 0, s>>>(p);
+    ct_restrict_kernel<S, 4, unsigned, V><<<blocks, kCtBlock, 0, s>>>(p);
     break;
   case 5:
-    ct_restrict_kernel<S, 5, unsigned><<<blocks, kCtBlock, 0, s>>>(p);
+    ct_restrict_kernel<S, 5, unsigned, V><<<blocks, kCtBlock, 0, s>>>(p);
     break;
   case 6:
-    ct_restrict_kernel<S, 6, unsigned><<<blocks, kCtBlock, 0, s>>>(p);
+    ct_restrict_kernel<S, 6, unsigned, V><<<blocks, kCtBlock, 0, s>>>(p);
     break;
   default:
-    ct_restrict_kernel<S, kMaxDims, unsigned long long>
+    ct_restrict_kernel<S, kMaxDims, unsigned long long, V>
         <<<blocks, kCtBlock, 0, s>>>(p);
   }
   cuda_check(cudaGetLastError(), "ct_restrict_kernel launch");
@@ -969,13 +973,16 @@ void ct_restrict(paliwa_gb_ct const &ct, double const *sparse,
   CtParams p = ct.params;
   if (ct.dtype == PALIWA_GB_F64) {
     p.values = sparse;
-    launch_restrict<double>(ct, p, s);
+    launch_restrict<double, double>(ct, p, s);
+  } else if (ct.npoints < kCtNarrow) {
+    p.values = sparse;
+    launch_restrict<float, double>(ct, p, s);
   } else {
     long long const nb = (ct.npoints + kCtBlock - 1) / kCtBlock;
     ct_narrow_kernel<<<static_cast<unsigned>(std::min(nb, 16LL * 152)),
                        kCtBlock, 0, s>>>(sparse, ct.values_dev, ct.npoints);
     p.values = ct.values_dev;
-    launch_restrict<float>(ct, p, s);
+    launch_restrict<float, float>(ct, p, s);
   }
 }
 

@@ -74,7 +74,7 @@ struct CtParams {
   long long const *unit_first;
   long long const *families;
   long long const *family_first;
-  void const *values;  // the sparse values in the grids' type
+  void const *values;  // the sparse values, in the grids' type or as doubles
 };
 
 // Points (threads) per CTA of the combine and scatter kernels.
@@ -312,7 +312,12 @@ __global__ void __launch_bounds__(kCtBlock, kCtCtas)
 }
 
 // The sparse values in the grids' type, converted once per point: a
-// conversion per grid value would take the FP64 pipe as long as the combine.
+// conversion per grid value would take the FP64 pipe as long as the combine
+// (and gather twice the bytes: 4D |l|_1 = 19 - q with lmin 2 365 us, 499
+// converting as it gathers). Sparse grids of fewer points are converted as
+// they are gathered: this launch would be what they wait for (up to 2^17
+// points 1.3-2.2 us faster without, never slower; from 2^18 on either side).
+constexpr long long kCtNarrow = 1LL << 17;
 __global__ void __launch_bounds__(kCtBlock)
     ct_narrow_kernel(double const *in, float *out, long long n) {
   long long const step = static_cast<long long>(gridDim.x) * kCtBlock;
@@ -401,7 +406,7 @@ template <typename I> struct CtRow {
   }
 };
 
-template <typename S, int ND, typename I>
+template <typename S, int ND, typename I, typename V>
 __global__ void __launch_bounds__(kCtBlock, kCtRestrictCtas)
     ct_restrict_kernel(CtParams const p) {
   constexpr int GROUPS = ct_groups(sizeof(S));
@@ -410,7 +415,8 @@ __global__ void __launch_bounds__(kCtBlock, kCtRestrictCtas)
   CtRows<ND, I> const rows(p, g);
   unsigned long long const base = p.grids[g].base;
   S *const out = reinterpret_cast<S *>(base);
-  S const *const val = reinterpret_cast<S const *>(p.values);
+  V const *const values = reinterpret_cast<V const *>(p.values);
+  auto val = [&](I at) { return static_cast<S>(values[at]); };
   int total = 0;
 #pragma unroll
   for (int d = 0; d < ND; ++d) total += rows.lv[d];
@@ -432,17 +438,17 @@ __global__ void __launch_bounds__(kCtBlock, kCtRestrictCtas)
       int s;
       I const at0 = r.of(k, l, s);
       if (s <= r.top) {
-        v[q][0] = val[at0];
+        v[q][0] = val(at0);
         keep[q] = 1;
       }
       if (l - 1 <= r.top) {
-        v[q][2] = val[r.at(l - 1, k >> 2)];
+        v[q][2] = val(r.at(l - 1, k >> 2));
         keep[q] |= 4;
       }
       if (l <= r.top) {
         I const at1 = r.at(l, k >> 1);
-        v[q][1] = val[at1];
-        v[q][3] = val[at1 + 1];
+        v[q][1] = val(at1);
+        v[q][3] = val(at1 + 1);
         keep[q] |= 10;
       }
     }
@@ -465,16 +471,27 @@ __global__ void __launch_bounds__(kCtBlock, kCtRestrictCtas)
     }
     return;
   }
-  // Rows of one or two points: each point has a row of its own.
-  for (int q = 0; q < GROUPS; ++q)
+  // Rows of one or two points: each point has a row of its own. (Four points'
+  // loads at once: one after another 2D grids of 2^17 points in such rows took
+  // 8.3 us, 6.4 so.)
+  for (int q = 0; q < GROUPS; ++q) {
+    S v[4];
+    unsigned keep = 0;
+#pragma unroll
     for (int i = 0; i < 4; ++i) {
       I const f = first + q * 4 * kCtBlock + i;
       if (f >= n) continue;
       CtRow<I> const r(rows, f >> l);
       int s;
       I const at = r.of(static_cast<unsigned>(f) & ((1u << l) - 1), l, s);
-      if (s <= r.top) out[f] = val[at];
+      if (s > r.top) continue;
+      v[i] = val(at);
+      keep |= 1u << i;
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if ((keep >> i) & 1u) out[first + q * 4 * kCtBlock + i] = v[i];
+  }
 }
 
 // Scatter: full[p] += sparse[p] on the full grid at the maximum level.
