@@ -615,6 +615,7 @@ struct paliwa_gb_ct {
   long long ncombine = 0;   // combine CTAs
   long long nrestrict = 0;  // restrict CTAs
   bool big = false;         // a grid of 2^31 points or more
+  bool direct = false;      // combine by ct_combine_direct_kernel
   CtParams params{};
 };
 
@@ -873,6 +874,10 @@ void build_ct(paliwa_gb_ct &ct, int64_t const *levels,
   for (int d = 0; d < nd && d < kMaxDims; ++d)
     ct.params.max_level[d] = static_cast<signed char>(lmax[d]);
   ct.params.block_sub = ct.block_sub_dev;
+  int longest = 0;
+  for (auto const &ss : subs)
+    longest = std::max(longest, ss.grid_end - ss.grid_begin);
+  ct.direct = ct_direct(dtype_size(ct.dtype), ct.npoints, longest);
   plan_combine(ct, subs);
   plan_restrict(ct, subs, levels);
   // Products c * v are exact in FP64 when c has at most 53 - 24 = 29
@@ -922,10 +927,29 @@ void launch_combine(paliwa_gb_ct const &ct, CtParams const &p,
   cuda_check(cudaGetLastError(), "ct_combine_kernel launch");
 }
 
+void launch_combine_direct(paliwa_gb_ct const &ct, CtParams const &p,
+                           cudaStream_t s) {
+  unsigned const blocks =
+      static_cast<unsigned>((ct.npoints + kCtBlock - 1) / kCtBlock);
+  if (ct.dtype == PALIWA_GB_F64) {
+    if (p.exact_products)
+      ct_combine_direct_kernel<double, true><<<blocks, kCtBlock, 0, s>>>(p);
+    else
+      ct_combine_direct_kernel<double, false><<<blocks, kCtBlock, 0, s>>>(p);
+  } else {
+    if (p.exact_products)
+      ct_combine_direct_kernel<float, true><<<blocks, kCtBlock, 0, s>>>(p);
+    else
+      ct_combine_direct_kernel<float, false><<<blocks, kCtBlock, 0, s>>>(p);
+  }
+  cuda_check(cudaGetLastError(), "ct_combine_direct_kernel launch");
+}
+
 void ct_combine(paliwa_gb_ct const &ct, double *sparse, cudaStream_t s) {
   if (ct.npoints == 0) return;
   CtParams p = ct.params;
   p.sparse = sparse;
+  if (ct.direct) return launch_combine_direct(ct, p, s);
   if (ct.dtype == PALIWA_GB_F64)
     return p.exact_products ? launch_combine<double, true>(ct, p, s)
                             : launch_combine<double, false>(ct, p, s);

@@ -53,3 +53,18 @@ def run(levels, dtype):
 def test_restrict_converts_in_a_launch_of_its_own_from_2_17_points(
         dtype, levels, launches):
     assert len(run(levels, dtype)[1]) == launches
+
+
+@pytest.mark.parametrize("dtype, levels, direct", [
+    ("float64", [(9, 9), (9, 9), (10, 8)], True),      # 2^18 in 3 grids
+    ("float64", [(8, 8), (9, 7), (7, 9)], False),      # 2^15
+    ("float64", [(9, 9)] * 20, False),                 # 20 grids
+    ("float32", [(9, 9), (9, 9), (10, 8)], False),
+    ("float32", [(10, 10), (10, 10), (11, 9)], True),  # 2^20
+    ("float64", [(18,), (18,)], True),
+    ("float64", [(5, 2, 4, 6), (5, 2, 4, 6), (4, 2, 5, 6)], True),
+])
+def test_combine_of_few_grids_walks_the_lists(dtype, levels, direct):
+    names = run(levels, dtype)[0]
+    assert len(names) == 1
+    assert ("ct_combine_direct" in names[0]) == direct, names
