@@ -269,25 +269,45 @@ void launch_out_list(OutPass const &p, OutList const &q, size_t smem,
   cuda_check(cudaGetLastError(), "out_list_kernel launch");
 }
 
-// Whether one launch for the list is worth it. It saves launches and passes
-// over memory, but a CTA runs its columns' passes one after another, where a
-// launch per pass spreads each over the chip: one column of 4609 floats, two
-// passes, took 47 us against 4.1. Both sides' times in us, fitted to 668 calls
-// of 2 to 18 passes on 1 to 2^19 columns (a thread's chain of steps, and what
-// the columns take together; FP64 by its pipe), the list's rather long: one of
-// them is then more than 2 % slower than a launch per pass (6 %), and all gain
-// 1.77x, where the better side of each would give 1.82x.
-bool out_list_pays(bool f64, long long columns, int log2cols, size_t npasses,
-                   long long extent, long long updates) {
-  double const rows = 256 >> log2cols;  // of a CTA's threads along the axis
-  double const mega = columns * 1e-6;
-  double const list = 2.6 + 0.2 * npasses +
-                      ((f64 ? 0.2 : 0.15) * updates + 0.45 * extent) / rows +
-                      mega * (100 + (f64 ? 2.4 : 0.8) * updates +
-                              (f64 ? 2.1 : 0.6) * extent);
-  double const passes = 0.2 + 1.9 * npasses + mega * (f64 ? 9 : 7.3) * updates;
-  return list < 0.85 * passes;
-}
+// Whether one launch for the list is worth it. It saves launches, passes over
+// memory and index arithmetic (a division per dimension and point), but a CTA
+// runs its columns' passes one after another, where a launch per pass spreads
+// each over the chip: one column of 4609 floats, two passes, took 47 us
+// against 4.1, 32768 columns of 256 doubles, twelve passes, 228 against 250.
+//
+// Both sides' times in us, fitted to 2600 random calls of one to six
+// dimensions: a thread's chain of updates and copies (longer where CTAs wait
+// for a place), the columns' work together and their offsets; and per pass a
+// launch and its points. On 1400 others the choice is within 0.5 % of the
+// better side's mean time; 1.0 % of them are more than 5 % slower than a
+// launch per pass and 1.7 % than the list, mostly calls of 4 to 6 us. (Always
+// the list: 16 % slower than a launch per pass, up to 9.7x; never: 81 % slower
+// than the list, up to 5.7x.)
+struct OutCost {
+  bool f64, along;
+  int ndim, log2cols;
+  size_t npasses, smem;
+  long long columns, extent, updates;
+
+  bool list_pays() const {
+    double const rows = 256 >> log2cols;  // of a CTA's threads along the axis
+    double const u = updates / rows, io = extent / rows;
+    double const resident =
+        std::min<size_t>(8, std::max<size_t>(1, (227 << 10) / (smem + 1024)));
+    double const ctas = static_cast<double>((columns >> log2cols) + 1);
+    double const wait =
+        std::max(0.0, ctas / (resident * device_sm_count()) - 1);
+    double const mega = columns * 1e-6;
+    double const list = 2.7 + 0.2 * npasses +
+                        u * ((f64 ? 0.2 : 0.09) + 0.055 * wait) +
+                        io * (0.36 + 0.63 * wait) +
+                        mega * (updates * (f64 ? 3 : 1) + (along ? 105 : 55));
+    double const passes =
+        npasses * (1.45 + 0.2 * ndim) +
+        mega * updates * (f64 ? 5.8 + 1.45 * ndim : 4.3 + 1.6 * ndim);
+    return list < passes;
+  }
+};
 
 // One launch for the whole list when that pays and the touched stretch of the
 // axis fits shared memory with 4 columns or more (up to 32: whole 128-byte
@@ -345,23 +365,22 @@ void launch_out_call(int dtype, bool exact, OutCall const &call,
   };
   if (extent > (1 << 20) || columns > (1LL << 32)) return one_by_one();
   while (log2cols > 2 && (smem_of(log2cols) > kOutSmem ||
-                          (columns >> log2cols) < 2 * 152))
+                          (columns >> log2cols) < 2 * device_sm_count()))
     --log2cols;
-  if (smem_of(log2cols) > kOutSmem ||
-      !out_list_pays(es == 8, columns, log2cols, n, extent, updates))
-    return one_by_one();
+  OutCost const cost{es == 8, along,   p.ndim, log2cols,
+                     n,       smem_of(log2cols), columns, extent, updates};
+  if (cost.smem > kOutSmem || !cost.list_pays()) return one_by_one();
   q.k0 = static_cast<int>(lo);
   q.extent = static_cast<int>(extent);
   q.log2cols = log2cols;
   q.pitch = along ? static_cast<int>(extent | 1) : 1 << log2cols;
-  size_t const smem = smem_of(log2cols);
   auto go = [&](auto value, auto ex) {
     using T = decltype(value);
     constexpr bool E = decltype(ex)::value;
     if (along)
-      launch_out_list<T, E, true>(p, q, smem, s);
+      launch_out_list<T, E, true>(p, q, cost.smem, s);
     else
-      launch_out_list<T, E, false>(p, q, smem, s);
+      launch_out_list<T, E, false>(p, q, cost.smem, s);
   };
   if (dtype == PALIWA_GB_F64)
     exact ? go(double{}, std::true_type{}) : go(double{}, std::false_type{});
