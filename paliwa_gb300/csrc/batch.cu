@@ -1003,7 +1003,7 @@ void ct_restrict(paliwa_gb_ct const &ct, double const *sparse,
     launch_restrict<float, double>(ct, p, s);
   } else {
     long long const nb = (ct.npoints + kCtBlock - 1) / kCtBlock;
-    ct_narrow_kernel<<<static_cast<unsigned>(std::min(nb, 16LL * 152)),
+    ct_narrow_kernel<<<static_cast<unsigned>(std::min(nb, 16LL * device_sms())),
                        kCtBlock, 0, s>>>(sparse, ct.values_dev, ct.npoints);
     p.values = ct.values_dev;
     launch_restrict<float, float>(ct, p, s);

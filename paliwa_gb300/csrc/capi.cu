@@ -284,9 +284,9 @@ KernelSet periodic_kernels(AxisView const &v, bool canon, bool ordered) {
   //  * strided float pencils of 8 points and more (FP32c n = 128 4670 against
   //    2920, n = 2048 3430 against 2380; FP32 n = 512 5530 against 4850, n =
   //    1024 5200 against 3840), but FP32 up to 1024 only (n = 2048, 16 columns:
-  //    3340 against 3910 on the tile kernel). On 4-point chunks the two are within 1 % for single
-  //    grids, and the wide kernel is faster in batches (5.26 against
-  //    4.39-4.55 TB/s).
+  //    3340 against 3910 on the tile kernel). On 4-point chunks the two are
+  //    within 1 % for single grids, and the wide kernel is faster in batches
+  //    (5.26 against 4.39-4.55 TB/s).
   // Not where 32 or more chunks lie on more than 16 pages of 2 MB (pencils of
   // 64 MB and more) and the boxed form does not apply: a box visits the chunks
   // row by row, so every box row then waits for its page, 8 clocks each (FP32c
@@ -294,8 +294,6 @@ KernelSet periodic_kernels(AxisView const &v, bool canon, bool ordered) {
   // 1650 against 2590; FP64 n = 1024 1250 against 1520).
   if (k.has(kChooseTmaWide)) {
     int const longest = v.log2_es == 3 ? 10 : v.wide_last ? 11 : 10;
-    int const log2chunks =
-      v.log2_n - (v.log2_es == 3 || (!v.wide_last && v.log2_n == 10) ? 5 : 4);
     bool const pages = spread_pages(v) && !box_periodic(v);
     if (last || pairs ||
         (v.log2_n >= 3 && v.log2_n <= longest && !pages))

@@ -11,9 +11,6 @@
 
 namespace pgb {
 
-int device_sms();
-int current_device();
-
 // Occupancy of one kernel instantiation, per device: the dynamic shared
 // memory opt-in (cudaFuncSetAttribute) and the occupancy query apply to the
 // device that is current when they are made, so a host thread that drives

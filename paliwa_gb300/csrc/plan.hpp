@@ -125,8 +125,7 @@ enum KernelChoice {
   kChooseWide = 2,
   kChooseTile = 3,
   kChooseStaged32 = 4,  // staged, 32 points per thread
-  // the wide kernel's transform with TMA copies (batches of FP32c grids;
-  // elsewhere the wide kernel)
+  // the wide kernel's transform with TMA copies
   kChooseTmaWide = 5,
   kChooseCount = 6
 };
@@ -134,8 +133,8 @@ struct KernelSet {
   unsigned mask = 0;  // a bit per applicable KernelChoice
   int dflt = kChooseStaged;
   // The kernel that a stage choosing kChooseTmaWide is planned for (the
-  // wide kernel, else the default without the TMA wide kernel): it runs the
-  // stage outside batches and where the tensor map cannot be made.
+  // default without the TMA wide kernel): it runs the stage in launches of few
+  // points, with TMA launches off and where the tensor map cannot be made.
   int fallback = kChooseStaged;
   bool has(int c) const { return (mask >> c) & 1u; }
 };
@@ -169,12 +168,14 @@ bool uses_heads(AxisView const &view, std::vector<int> const &shifts,
 // Kernel-level parameters shared by every job of a launch.
 LiftParams launch_params(std::vector<Filter> const &filters);
 
+// One of the stages of chunk heads (R as in kHeadsIn, kHeadsOut and
+// kHeadsTile) on the inline job of `params`.
+void launch_heads(int sched, int R, LiftParams params, long long total_tiles,
+                  cudaStream_t s);
 // Launch the lifting kernel for `dtype` over `njobs` jobs (device array
 // `jobs`, or the inline job of `params` when jobs == nullptr).
 // sched: 2 * wavelet + forward for the compile-time wavelet schedule (every
 // job's shifts must be canonical), or -1 for the runtime schedule.
-void launch_heads(int sched, int R, LiftParams params, long long total_tiles,
-                  cudaStream_t s);
 void launch_lift(int dtype, bool exact, bool symmetric, int sched, int R,
                  LiftParams params, LiftJob const *jobs, int njobs,
                  long long total_tiles, cudaStream_t stream);
@@ -184,6 +185,8 @@ int wavelet_schedule(std::vector<Filter> const &filters);
 bool canonical_shifts(LiftJob const &job, bool forward);
 
 void cuda_check(cudaError_t e, char const *what);
+int current_device();
+int device_sms();
 size_t dtype_size(int dtype);
 
 // Shifts (log2 distances) of hierarchize_in (forward: levels level..lmin+1)

@@ -14,7 +14,7 @@
 //    min(inner, Ct, 256), Sx = Ct / inner when inner < Ct), in shared
 //    memory as [box][outer][row][column];
 //  * chunk-interleaved (8 to 128 chunks of 16 points): a 5D map {X columns,
-//    G chunks, R rows of a chunk, column groups, outer index} (X = 4 or 8)
+//    G chunks, R rows of a chunk, column groups, outer index} (X = 4 to 16)
 //    and one box per tile, in shared memory as [column group][row of
 //    chunk][chunk][X columns], so that the chunks a warp reads together lie
 //    in consecutive X-column groups (with the dense layout they would read
@@ -44,8 +44,9 @@
 // barrier more than on anything else). twide_long_kernel (pencils of more
 // than 32 chunks) has no producer warp; see there.
 //
-// The maps live in global memory, written by the host before the launch;
-// they cover only this GPU's grid memory (no multicast).
+// A batch's maps live in global memory, written by the host before the launch,
+// a single grid's in the launch parameters; they cover only this GPU's grid
+// memory (no multicast).
 #pragma once
 
 #include <cstdint>
@@ -57,7 +58,7 @@
 namespace pgb {
 
 constexpr int kTWideThreads = 256;  // transform threads
-// Chunks of 32 points (FP64) take 128, for tiles of the same 32 KB; the
+// Chunks of 32 points take 128, for tiles of the same 32 KB; the
 // producer warp comes on top.
 __host__ __device__ constexpr int twide_threads(int r) {
   return r >= 32 ? kTWideThreads / 2 : kTWideThreads;
@@ -71,8 +72,8 @@ constexpr int kTWideLong = 64;
 constexpr int kTWideContig = 96;
 constexpr int kTWidePairs = 128;
 constexpr int kTWideLongContig = 160;
-// Launch codes of the forms with 32-point chunks (FP64): dense, chunked and
-// pairs.
+// Launch codes of the forms with 32-point chunks: dense, chunked (floats too)
+// and pairs.
 constexpr int kTWide32Dense = 224;
 constexpr int kTWide32Chunked = 225;
 constexpr int kTWide32Pairs = 226;
@@ -155,7 +156,7 @@ __device__ __forceinline__ void tma_store_3d(void const *map, int x, int y,
       : "memory");
 }
 // Chunk-interleaved layout, [column group][row of chunk][chunk][X columns]
-// (X = 2^log2_xlo, 4 or 8): the float index of row 0 of chunk c of column
+// (X = 2^log2_xlo, 4 to 16): the float index of row 0 of chunk c of column
 // pair g (rows follow X G floats apart).
 template <int LOG2R>
 __device__ __forceinline__ int chunk_index(TWideJob const &job, int g, int c,
