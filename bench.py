@@ -739,7 +739,8 @@ def run_gpu(args, w, world, rank, local):
 def measure_link(host_in, host_out, dev_buf):
     """GB/s of the host link in this run: the whole pinned input copied to
     the device, the device buffer copied to the pinned output, and both at
-    once on two streams (each direction's rate), best of two, CUDA events."""
+    once on two streams (each direction's rate), best of eight (the link
+    stalls for tens of milliseconds about every half second), CUDA events."""
     import torch
     nbytes = dev_buf.numel() * dev_buf.element_size()
     s_in, s_out = torch.cuda.Stream(), torch.cuda.Stream()
@@ -766,7 +767,7 @@ def measure_link(host_in, host_out, dev_buf):
     out = {}
     for key, h2d, d2h in (("h2d_gbs", True, False), ("d2h_gbs", False, True),
                           ("concurrent_gbs_each", True, True)):
-        ms = min(once(h2d, d2h) for _ in range(2))
+        ms = min(once(h2d, d2h) for _ in range(8))
         out[key] = nbytes / (ms / 1e3) / 1e9
     return out
 

@@ -360,6 +360,12 @@ void paliwa_gb_batch_destroy(paliwa_gb_batch *batch);
  * lexicographically, each stored densely over the extents of
  * paliwa::strided_hierarchical_domain_from_level(s, maximum_level)
  * (paliwa/paliwa_domains.hpp:51-83), concatenated.
+ *
+ * Besides its tables (the grid lists of every subspace and, per grid, 8 bytes
+ * for every combination of its leading dimensions' levels) an object for F32
+ * or F32C grids with 2^17 sparse points or more holds the sparse values as
+ * floats, which a restrict fills: restricts of one object are to be ordered by
+ * the caller (they write the same grids).
  */
 typedef struct paliwa_gb_ct paliwa_gb_ct;
 

@@ -165,15 +165,16 @@ struct paliwa_gb_batch {
 namespace {
 
 // Whether a new batch plans slabs. They save launches, which is what small
-// batches spend their time on (FP32c 6D |l|_1 = 12 - q, 2.6 M points: 134
-// against 247 us there and back; FP64 165 against 300), but their axes are
-// bound by barriers and latencies at about half the TMA wide kernel's rate
-// for double and double-float arithmetic: FP32c from about 2^25 points on
-// (6D 14 - q, 30 M points: 592 against 744 us; 4D 16 - q, 48 M: 1059 against
-// 1068; 5D 16 - q, 139 M: 2288 against 2051; 4D 20 - q: 23.1 against 19.9 ms)
-// and FP64 from about 2^22 (4D 14 - q, 7.4 M: 602 against 518) are faster
-// axis by axis. Plain FP32 is bound by memory either way and takes slabs
-// throughout (5D 16 - q 1532 against 1685; 4D 18 - q 3105 against 3102).
+// batches spend their time on (us, there and back, CDF (2,2): FP32c 6D |l|_1 =
+// 12 - q, 2.6 M points, 67 against 240, 4D 15 - q, 19 M, 485 against 512; FP64
+// 6D 12 - q 137 against 387, 4D 13 - q, 2.8 M, 320 against 335), but their
+// axes are bound by barriers and latencies at about half the TMA wide kernel's
+// rate for double and double-float arithmetic: FP64 from about 2^22 points on
+// (4D 14 - q, 7.4 M: 597 against 518) and FP32c somewhere from 2^25 on (6D 14
+// - q, 30 M: 515 against 742; 4D 16 - q, 48 M: 1040 against 1052; 5D 16 - q,
+// 139 M: 2109 against 2006) are faster axis by axis. Plain FP32 is bound by
+// memory either way and takes slabs throughout (5D 16 - q 1425 against 1697;
+// 4D 18 - q 3108 against 3109).
 bool default_slabs(int dtype, long long points) {
   switch (dtype) {
   case PALIWA_GB_F64: return points <= 1LL << 22;
